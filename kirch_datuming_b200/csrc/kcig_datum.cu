@@ -12,7 +12,7 @@
 //     source side    Uout[iw] = Ks[iw] . Utmp[iw], Ks[is][ic]  (ns x ns)
 // (k_cgemm, batched over a chunk of frequencies, skipping the K tiles outside
 // the aperture band).  The operators of a chunk are built on the device
-// (k_dat_op): per term the weight of :508-523 (aperture taper, distance,
+// (k_dat_op_fft; k_dat_op for filters beyond 63 samples): per term the weight of :508-523 (aperture taper, distance,
 // tau) precomputed on the host in the reference's arithmetic, times the
 // anti-aliasing weight (:197-226) and the filter H(tau, w) (:98-182), which is
 // evaluated in FP64 with exact phase reduction (the reference's FP32 phase
@@ -189,6 +189,225 @@ __global__ void __launch_bounds__(128) k_dat_op(const DatOpArgs a)
         const double mr = (double)ec * lr + (double)es * li, mi = (double)ec * li - (double)es * lr;
         const double hr = mr * sr - mi * si, hi = mr * si + mi * sr;
         o[(size_t)c * a.ne] = make_float2((float)(wa * hr), (float)(wa * hi));
+    }
+}
+
+// ---- the same operators by short FFTs ---------------------------------------
+// A term's factor is a real FIR filter of K + 1 samples placed at n = m - 1 ..
+// m - 1 + K (the K filter samples, and the split of tau between samples m - 1
+// and m as a two-sample filter over them):
+//     H(iw) = sum_n G[n] W_N^(iw n),  W_N = exp(-2 pi i / nfft).
+// For the frequencies iw = a + M b (M = nfft / Q, b = 0 .. Q - 1) of one
+// residue a, W_N^(iw n) = W_N^(a n) W_Q^(b n): a Q-point FFT over n mod Q of
+// G[n] W_N^(a n) gives all of them, and since G is real the half above
+// nfft / 2 is the conjugate of residue M - a.  Residues a = 0 .. M / 2 give
+// every frequency; the spectra's rows are kept in that order (dat_row), so a
+// chunk of rows is a group of residues.  About 30 FP64 operations per (term,
+// frequency) for Q = 64 in place of Horner's five per filter sample and the
+// phase's own sine and cosine: 17.1 -> 6.7 ms for 400 x 400 terms, 8193
+// frequencies and 51 filter samples (10.5 GB of operators written).
+//
+// A block of 256 threads takes 256 / T entries, T = Q / 8 sub-threads per
+// entry with eight points each: an 8-point DFT in registers, the twiddles, an
+// exchange through shared memory, a T-point DFT.
+// Lanes are entries, so every table read is a broadcast, the exchange has no
+// bank conflicts and a row is stored as 256 consecutive bytes per warp.
+struct C64 {
+    double x, y;
+};
+__device__ __forceinline__ C64 operator+(C64 a, C64 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ C64 operator-(C64 a, C64 b) { return {a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ C64 operator*(C64 a, C64 b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+__device__ __forceinline__ C64 mul_mi(C64 a) { return {a.y, -a.x}; }  // -i a
+
+__device__ __forceinline__ void dft2(C64 *v)
+{
+    const C64 t = v[0];
+    v[0] = t + v[1];
+    v[1] = t - v[1];
+}
+__device__ __forceinline__ void dft4(C64 *v)
+{
+    const C64 a = v[0] + v[2], b = v[0] - v[2], c = v[1] + v[3], d = mul_mi(v[1] - v[3]);
+    v[0] = a + c;
+    v[1] = b + d;
+    v[2] = a - c;
+    v[3] = b - d;
+}
+__device__ __forceinline__ void dft8(C64 *v)
+{
+    constexpr double r = 0.70710678118654752440;
+    C64 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    dft4(e);
+    dft4(o);
+    const C64 o1 = {(o[1].x + o[1].y) * r, (o[1].y - o[1].x) * r};   // W_8 o1
+    const C64 o2 = mul_mi(o[2]);
+    const C64 o3 = {(o[3].y - o[3].x) * r, -(o[3].x + o[3].y) * r};  // W_8^3 o3
+    v[0] = e[0] + o[0];
+    v[4] = e[0] - o[0];
+    v[1] = e[1] + o1;
+    v[5] = e[1] - o1;
+    v[2] = e[2] + o2;
+    v[6] = e[2] - o2;
+    v[3] = e[3] + o3;
+    v[7] = e[3] - o3;
+}
+
+// row of frequency w in the residue order (Q = 0: the natural order)
+__device__ __forceinline__ int dat_row(int w, int Q, int M)
+{
+    if (Q == 0) return w;
+    int a = w & (M - 1), b = w >> (__ffs(M) - 1);  // M is a power of two
+    if (a == 0) return b;
+    if (2 * a > M) {
+        a = M - a;
+        b += Q / 2;
+    }
+    return Q / 2 + 1 + (a - 1) * Q + b;
+}
+
+// W_N^(a q) for the residues a = 0 .. M / 2 and q = 0 .. 2 Q - 1
+__global__ void k_dat_twiddles(C64 *tw, int Q, int M)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (M / 2 + 1) * 2 * Q) return;
+    const long long n = (long long)(i / (2 * Q)) * (i % (2 * Q)) % ((long long)M * Q);
+    double s, c;
+    sincospi(2.0 * (double)n / (double)((long long)M * Q), &s, &c);
+    tw[i] = {c, -s};
+}
+
+struct DatFftArgs {
+    const DatEntry *ent;
+    const C64 *tw;   // [M / 2 + 1][2 Q]
+    float2 *out;     // [rows of residues a0 .. a0 + na - 1][ne]
+    int ne, a0, na, M, K, nfft;
+    float dt, antialias;
+};
+constexpr int kOpGroup = 4;  // residues of one block: the filters are formed once for them
+
+template <int Q>
+__host__ __device__ constexpr int dat_op_smem()
+{
+    // exchange (or the filter roots), twiddles of the group, W_Q, entry phases, row frequencies
+    return 8 * 256 * 16 + kOpGroup * 2 * Q * 16 + Q * 16 + kOpGroup * (2048 / Q) * 16 + (kOpGroup * Q + 4) * 4;
+}
+
+template <int Q>
+__global__ void __launch_bounds__(256, 2) k_dat_op_fft(const DatFftArgs a)
+{
+    constexpr int T = Q / 8, EB = 256 / T, G = kOpGroup;
+    extern __shared__ __align__(16) unsigned char osm[];
+    C64 *xch = reinterpret_cast<C64 *>(osm);              // [Q][EB]
+    double *root = reinterpret_cast<double *>(osm);       // [Q][EB], before the exchange is used
+    C64 *tw = xch + 8 * 256;                              // [G][2 Q]
+    C64 *wq = tw + G * 2 * Q;                             // [Q]
+    C64 *ph = wq + Q;                                     // [G][EB]
+    float *fq = reinterpret_cast<float *>(ph + G * EB);   // rows of the group
+    const int en = threadIdx.x % EB, j = threadIdx.x / EB, e = blockIdx.x * EB + en;
+    const int M = a.M, K = a.K;
+    const int g0 = a.a0 + blockIdx.y * G, g1 = min(a.a0 + a.na, g0 + G);
+    // rows of residue r start at r ? Q / 2 + 1 + (r - 1) Q : 0
+    auto row_of = [](int r) { return r ? Q / 2 + 1 + (r - 1) * Q : 0; };
+    const int row0 = row_of(g0), nrow = (g1 == M / 2 + 1 ? M / 2 * Q + 1 : row_of(g1)) - row0;
+    float2 *o = a.out + (size_t)(row0 - row_of(a.a0)) * a.ne + e;
+    DatEntry d{0.0f, 0.0f, 0.0f};
+    if (e < a.ne) d = a.ent[e];
+    const bool on = d.w != 0.0f && d.tau > 0.0f && isfinite(d.tau);
+    if (!__syncthreads_or(on)) {  // terms outside the aperture
+        if (e < a.ne)
+            for (int r = j; r < nrow; r += T) o[(size_t)r * a.ne] = make_float2(0.0f, 0.0f);
+        return;
+    }
+    for (int i = threadIdx.x; i < (g1 - g0) * 2 * Q; i += 256) tw[i] = a.tw[(size_t)g0 * 2 * Q + i];
+    for (int i = threadIdx.x; i < Q; i += 256) {
+        double s, c;
+        sincospi(2.0 * i / Q, &s, &c);
+        wq[i] = {c, -s};
+    }
+    const float fden = __fmul_rn((float)a.nfft, a.dt);
+    for (int i = threadIdx.x; i < nrow; i += 256) {
+        const int r = row0 + i;  // the inverse of dat_row
+        int iw = r * M;
+        if (r > Q / 2) {
+            const int res = (r - Q / 2 - 1) / Q + 1, b = (r - Q / 2 - 1) % Q;
+            iw = 2 * res == M || b < Q / 2 ? res + M * b : M - res + M * (b - Q / 2);
+        }
+        fq[i] = __fdiv_rn((float)iw, fden);
+    }
+    // roots sqrt(t^2 - 1) of the filter, shared by the entry's sub-threads
+    const double rr = on ? (double)a.dt / (double)d.tau : 0.0, inv_dt = 1.0 / (double)a.dt;
+    for (int k = j; k < K; k += T) root[k * EB + en] = dat_root(k, rr);
+    const double q = on ? (double)d.tau * inv_dt : 1.0, mceil = ceil(q), delta = mceil - q;
+    const long long n0 = (long long)mceil - 1;  // first sample of the filter, >= 0
+    // phases W_M^(residue t0) of the samples' whole turns t0 = n0 / Q
+    for (int g = j; g < g1 - g0; g += T) {
+        const long long t = ((n0 / Q) % M) * (g0 + g) % M;
+        double s, c;
+        sincospi(2.0 * (double)t / (double)M, &s, &c);
+        ph[g * EB + en] = {c, -s};
+    }
+    __syncthreads();
+    // sample at place p = j + T i of the circle: G[k] = delta F[k] + (1 - delta) F[k - 1], k = p - n0 mod Q
+    const int p0 = (int)(n0 & (Q - 1));
+    double g[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int k = (j + T * i - p0) & (Q - 1);
+        auto R = [&](int n) { return n >= 0 && n < K ? root[n * EB + en] : 0.0; };
+        const double c0 = R(k), c1 = R(k - 1), c2 = R(k - 2), c3 = R(k - 3);
+        const double f0 = k < K ? c0 - 2.0 * c1 + c2 : 0.0;                // F[k] dt
+        const double f1 = k >= 1 && k <= K ? c1 - 2.0 * c2 + c3 : 0.0;     // F[k - 1] dt
+        g[i] = on && k <= K ? (delta * f0 + (1.0 - delta) * f1) * inv_dt : 0.0;
+    }
+    const DatAa aa = dat_aa_term(a.antialias, d.dtau, a.dt);
+    for (int r = g0; r < g1; r++) {
+        __syncthreads();  // the roots, or the last residue's exchange, are read
+        const C64 *tr = tw + (r - g0) * 2 * Q;
+        C64 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int p = j + T * i;
+            const C64 z = tr[p < p0 ? p + Q : p];
+            v[i] = {g[i] * z.x, g[i] * z.y};
+        }
+        dft8(v);
+        if (T > 1) {
+#pragma unroll
+            for (int m = 0; m < 8; m++) xch[(m * T + j) * EB + en] = m ? v[m] * wq[j * m] : v[m];
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = xch[(j * 8 + i) * EB + en];  // m = j (8 / T) + i / T, its T sub-threads
+#pragma unroll
+            for (int i = 0; i < 8; i += T) {
+                if (T == 8) dft8(v + i);
+                else if (T == 4) dft4(v + i);
+                else dft2(v + i);
+            }
+        }
+        const C64 c = ph[(r - g0) * EB + en];
+        const int base = row_of(r) - row0;
+        if (e < a.ne) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                // output b = m + 8 l
+                const int b = T > 1 ? j * (8 / T) + i / T + 8 * (i % T) : i;
+                int slot = b;
+                bool conj = false;
+                if (b >= Q / 2 && !(r == 0 && b == Q / 2)) {
+                    if (r == 0 || 2 * r == M) continue;  // its own mirror image
+                    slot = Q / 2 + Q - 1 - b;
+                    conj = true;
+                }
+                // (r = 0, b = 0 is frequency 0: fq = 0, below every fpass)
+                const C64 h = v[i] * c;
+                const float wa = __fmul_rn(d.w, aa.mode == 1 ? 1.0f : dat_aa_at(aa, r + slot, fq[base + slot]));
+                o[(size_t)(base + slot) * a.ne] =
+                    !on || fabsf(wa) < 1e-20f  // the reference skips these terms (:525)
+                        ? make_float2(0.0f, 0.0f)
+                        : make_float2((float)(wa * h.x), (float)(conj ? -(wa * h.y) : wa * h.y));
+            }
+        }
     }
 }
 
@@ -544,108 +763,137 @@ __global__ void __launch_bounds__(tcg::THREADS, 1) k_cgemm_tc(const CGemmArgs a,
     if (warp == PRODUCERS) tc::tmem_free(tmem, TMEM_COLS);
 }
 
+// Frequencies a thread of the cmp = 1 sums carries in registers: the term's
+// indices and weight (table lookups, a double product on the source side) are
+// formed once for all of them, and as many independent loads are in flight.
+constexpr int kCmp1F = 4;
+
 // cmp = 1 receiver side (:493-546 with s_abs = s0 + is ds): one thread per
-// (frequency, shot, trace), the sum over the aperture of
-// geom[ih][ic] tau (aH)[pair], pair = (table row cc = cabs[is][ic], column
+// (shot, trace) and kCmp1F frequencies, the sum over the aperture of
+// geom[ic][ih] tau (aH)[pair], pair = (table row cc = cabs[is][ic], column
 // c = cabs[is][ih]) looked up in the chunk's band table P[c][row][j],
-// j = c - cc + band.
+// j = c - cc + band.  Lanes along ih: the pair table, geom and tau are read
+// coalesced, the input spectrum is one value per warp.
 struct RcvCmp1Args {
     const float2 *U;   // [nf][ns][nh] (the chunk's input spectra)
     float2 *Utmp;      // [nf][ns][nh]
     const float2 *P;   // [nf][nrow * (2 band + 1)]
     const float *Ptau; // [nrow * (2 band + 1)]
     const int *cabs;   // [ns][nh]
-    const float *geom; // [nh][nh]
-    int ns, nh, aper, band, row0, nrow;
+    const float *geom; // [nh][nh], the input trace first
+    int ns, nh, aper, band, row0, nrow, nf;
     long long sU;      // U batch stride
 };
 
 __global__ void __launch_bounds__(128) k_dat_rcv_cmp1(const RcvCmp1Args a)
 {
-    const int tr = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    const int tr = blockIdx.x * blockDim.x + threadIdx.x, f0 = blockIdx.y * kCmp1F;
     const int ntr = a.ns * a.nh;
     if (tr >= ntr) return;
     const int is = tr / a.nh, ih = tr - is * a.nh;
-    const float2 *U = a.U + (size_t)c * a.sU + (size_t)is * a.nh;
     const int wid = 2 * a.band + 1;
-    const float2 *P = a.P + (size_t)c * a.nrow * wid;
-    const int cih = a.cabs[tr];
-    float sr = 0.0f, si = 0.0f;
-    const int left = max(0, ih - a.aper), right = min(a.nh - 1, ih + a.aper);
-    for (int ic = left; ic <= right; ic++) {
-        const float g = a.geom[(size_t)ih * a.nh + ic];
-        if (g == 0.0f) continue;
-        const int cc = a.cabs[(size_t)is * a.nh + ic];
-        const size_t pi = (size_t)(cc - a.row0) * wid + (cih - cc + a.band);
-        const float w = __fmul_rn(g, a.Ptau[pi]);
-        const float2 h = P[pi], u = U[ic];
-        sr = fmaf(w, u.x * h.x - u.y * h.y, sr);
-        si = fmaf(w, u.x * h.y + u.y * h.x, si);
+    const size_t sP = (size_t)a.nrow * wid;
+    const float2 *U[kCmp1F], *P[kCmp1F];
+    float sr[kCmp1F], si[kCmp1F];
+#pragma unroll
+    for (int j = 0; j < kCmp1F; j++) {
+        const size_t f = min(f0 + j, a.nf - 1);  // past the chunk: the last frequency again, not stored
+        U[j] = a.U + f * a.sU + (size_t)is * a.nh;
+        P[j] = a.P + f * sP;
+        sr[j] = si[j] = 0.0f;
     }
-    a.Utmp[(size_t)c * ntr + tr] = make_float2(sr, si);
+    const int cih = a.cabs[tr];
+    const int left = max(0, ih - a.aper), right = min(a.nh - 1, ih + a.aper);
+    // no branch on a zero weight (its term is dropped by selection, so a NaN
+    // trace outside the taper stays outside): the loads of several terms overlap
+#pragma unroll 4
+    for (int ic = left; ic <= right; ic++) {
+        const float g = __ldg(a.geom + (size_t)ic * a.nh + ih);
+        const int cc = __ldg(a.cabs + (size_t)is * a.nh + ic);
+        const size_t pi = (size_t)(cc - a.row0) * wid + (cih - cc + a.band);
+        const float w = __fmul_rn(g, __ldg(a.Ptau + pi));
+#pragma unroll
+        for (int j = 0; j < kCmp1F; j++) {
+            const float2 h = __ldg(P[j] + pi), u = __ldg(U[j] + ic);
+            const float xr = fmaf(w, u.x * h.x - u.y * h.y, sr[j]), xi = fmaf(w, u.x * h.y + u.y * h.x, si[j]);
+            sr[j] = g != 0.0f ? xr : sr[j];
+            si[j] = g != 0.0f ? xi : si[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kCmp1F; j++)
+        if (f0 + j < a.nf) a.Utmp[(size_t)(f0 + j) * ntr + tr] = make_float2(sr[j], si[j]);
 }
 
-// cmp = 1 source side (:556-619): one thread per (frequency, shot); it walks
-// the common-receiver gathers r that hold the shot (ir in [ir_lo, ir_hi]),
-// and adds the sum over the gather's neighbouring shots to its own trace
-// ih(r) of the output, so every output row has one writer and a fixed order.
+// cmp = 1 source side (:556-619): one thread per output trace (shot is, trace
+// ih) and kCmp1F frequencies.  The common-receiver gathers r that send the
+// shot to this trace are listed per trace (cnt in gath, in order of r; one
+// gather when |ds| >= |dh|): each gather's neighbouring shots are summed, and
+// the gathers' sums added in that order.  Lanes along ih take neighbouring
+// gathers, so ihmap[ic][r] and the input spectra are read coalesced.
+// It was one thread per (frequency, shot) walking every gather that holds
+// the shot, a few hundred threads a chunk: 19.4 ms of a 64 x 96 trace call
+// with 513 frequencies, now 0.55 ms (receiver side 2.0 -> 0.82 ms).
 struct SrcCmp1Args {
     const float2 *Utmp;  // [nf][ns][nh]
-    float2 *Uout;        // [nf][ns][nh] (zeroed)
+    float2 *Uout;        // [nf][ns][nh]
     const float2 *P;     // [nf][ns][ns]: aH of pair (c_s[ic], c_s[is]) at [is][ic]
-    const float *Ptau;   // [ns][ns]
+    const double *gw;    // [ns][ns]: ds sdatum tau / (pi dist) at [is][ic]
     const int *sleft, *sright;  // [nr] the gather's shot range
-    const int *ihmap;    // [nr][ns]: trace of shot is in gather r, -1 outside
-    const int *ir_lo, *ir_hi;   // [ns]
-    int ns, nh, nr, aper, jump, tap;
-    float ds, sdatum;
+    const int *ihmap;    // [ns][nr]: trace of shot is in gather r, -1 outside
+    const int *goff;     // [ns * nh + 1] first entry of each output trace in gath
+    const int *gath;     // gathers, in order
+    const float *ramp;   // [nramp] edge taper by the distance from the window's end; past it 1
+    int ns, nh, nr, aper, jump, nramp, nf;
     long long sUout;
 };
 
-__device__ __forceinline__ float dat_taper(int left, int center, int right, int tap, int stride)
-{
-    if (center < left || center > right) return 0.0f;
-    if (tap <= 0) return 1.0f;
-    if (stride < 1) stride = 1;
-    const float width = __fmul_rn((float)tap, (float)stride);
-    const float ul = fminf(1.0f, fmaxf(0.0f, __fdiv_rn((float)(center - left), width)));
-    const float ur = fminf(1.0f, fmaxf(0.0f, __fdiv_rn((float)(right - center), width)));
-    return __fmul_rn(__fmul_rn(__fmul_rn(0.5f, __fsub_rn(1.0f, cospif(ul))), 0.5f), __fsub_rn(1.0f, cospif(ur)));
-}
-
 __global__ void __launch_bounds__(128) k_dat_src_cmp1(const SrcCmp1Args a)
 {
-    const int is = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-    if (is >= a.ns) return;
+    const int tr = blockIdx.x * blockDim.x + threadIdx.x, f0 = blockIdx.y * kCmp1F;
     const int ntr = a.ns * a.nh;
-    const float2 *Ut = a.Utmp + (size_t)c * ntr;
-    float2 *Uo = a.Uout + (size_t)c * a.sUout + (size_t)is * a.nh;
-    const float2 *P = a.P + (size_t)c * a.ns * a.ns + (size_t)is * a.ns;
-    const float *Pt = a.Ptau + (size_t)is * a.ns;
-    const double kw = (double)a.ds * (double)a.sdatum / 3.14159265358979323846;
-    for (int ir = a.ir_lo[is]; ir <= a.ir_hi[is]; ir++) {
-        const int sl = a.sleft[ir], sr = a.sright[ir];
-        if (is < sl || is > sr || (is - sl) % a.jump) continue;
-        const int ih = a.ihmap[(size_t)ir * a.ns + is];
-        if (ih < 0) continue;
-        const int il = max(sl, is - a.jump * a.aper), iu = min(sr, is + a.jump * a.aper);
-        float accr = 0.0f, acci = 0.0f;
-        for (int ic = il; ic <= iu; ic += a.jump) {
-            const int hh = a.ihmap[(size_t)ir * a.ns + ic];
-            if (hh < 0) continue;
-            const float coef = dat_taper(il, ic, iu, a.tap, a.jump);
-            const float dist = __fadd_rn(__fmul_rn(a.sdatum, a.sdatum),
-                                         __fmul_rn(__fmul_rn((float)((ic - is) * (ic - is)), a.ds), a.ds));
-            const float w = (float)((double)coef * kw * (double)Pt[ic] / (double)dist);
-            const float2 h = P[ic], u = Ut[(size_t)ic * a.nh + hh];
-            accr = fmaf(w, u.x * h.x - u.y * h.y, accr);
-            acci = fmaf(w, u.x * h.y + u.y * h.x, acci);
-        }
-        float2 o = Uo[ih];
-        o.x += accr;
-        o.y += acci;
-        Uo[ih] = o;
+    if (tr >= ntr) return;
+    const int is = tr / a.nh;
+    const float2 *Ut[kCmp1F], *P[kCmp1F];
+    float2 o[kCmp1F];
+#pragma unroll
+    for (int j = 0; j < kCmp1F; j++) {
+        const size_t f = min(f0 + j, a.nf - 1);
+        Ut[j] = a.Utmp + f * ntr;
+        P[j] = a.P + f * a.ns * a.ns + (size_t)is * a.ns;
+        o[j] = make_float2(0.0f, 0.0f);
     }
+    const double *gw = a.gw + (size_t)is * a.ns;
+    for (int q = a.goff[tr]; q < a.goff[tr + 1]; q++) {
+        const int ir = a.gath[q];
+        const int il = max(a.sleft[ir], is - a.jump * a.aper), iu = min(a.sright[ir], is + a.jump * a.aper);
+        float accr[kCmp1F], acci[kCmp1F];
+#pragma unroll
+        for (int j = 0; j < kCmp1F; j++) accr[j] = acci[j] = 0.0f;
+#pragma unroll 4
+        for (int ic = il; ic <= iu; ic += a.jump) {
+            const int hh = __ldg(a.ihmap + (size_t)ic * a.nr + ir);
+            const float cl = ic - il < a.nramp ? __ldg(a.ramp + (ic - il)) : 1.0f;
+            const float cu = iu - ic < a.nramp ? __ldg(a.ramp + (iu - ic)) : 1.0f;
+            const float w = (float)((double)__fmul_rn(cl, cu) * __ldg(gw + ic));
+            const size_t at = (size_t)ic * a.nh + max(hh, 0);
+#pragma unroll
+            for (int j = 0; j < kCmp1F; j++) {
+                const float2 h = __ldg(P[j] + ic), u = __ldg(Ut[j] + at);
+                const float xr = fmaf(w, u.x * h.x - u.y * h.y, accr[j]), xi = fmaf(w, u.x * h.y + u.y * h.x, acci[j]);
+                accr[j] = hh >= 0 ? xr : accr[j];  // a shot the gather does not hold
+                acci[j] = hh >= 0 ? xi : acci[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kCmp1F; j++) {
+            o[j].x += accr[j];
+            o[j].y += acci[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kCmp1F; j++)
+        if (f0 + j < a.nf) a.Uout[(size_t)(f0 + j) * a.sUout + tr] = o[j];
 }
 
 // reverse in time, edge taper and zero-pad one batch of traces (:287-306):
@@ -685,8 +933,9 @@ __global__ void k_dat_finish(const float *pad, float *out, int tr0, int nb, int 
         out[(size_t)(tr0 + b) * nt + t] = __fmul_rn(pad[(size_t)b * nfft + ts], scale);
 }
 
-// tiled transposes between spec[b][nw] (a batch of traces) and U[iw][ntr]
-__global__ void k_dat_to_fmajor(const float2 *spec, float2 *U, int tr0, int nb, int nw, int ntr)
+// tiled transposes between spec[b][nw] (a batch of traces) and U[row][ntr],
+// the rows in dat_row's order
+__global__ void k_dat_to_fmajor(const float2 *spec, float2 *U, int tr0, int nb, int nw, int ntr, int Q, int M)
 {
     __shared__ float2 tile[32][33];
     const int w0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
@@ -697,17 +946,17 @@ __global__ void k_dat_to_fmajor(const float2 *spec, float2 *U, int tr0, int nb, 
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int w = w0 + r, b = b0 + threadIdx.x;
-        if (b < nb && w < nw) U[(size_t)w * ntr + tr0 + b] = tile[threadIdx.x][r];
+        if (b < nb && w < nw) U[(size_t)dat_row(w, Q, M) * ntr + tr0 + b] = tile[threadIdx.x][r];
     }
 }
 
-__global__ void k_dat_to_tmajor(const float2 *U, float2 *spec, int tr0, int nb, int nw, int ntr)
+__global__ void k_dat_to_tmajor(const float2 *U, float2 *spec, int tr0, int nb, int nw, int ntr, int Q, int M)
 {
     __shared__ float2 tile[32][33];
     const int w0 = blockIdx.y * 32, b0 = blockIdx.x * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int w = w0 + r, b = b0 + threadIdx.x;
-        if (b < nb && w < nw) tile[r][threadIdx.x] = U[(size_t)w * ntr + tr0 + b];
+        if (b < nb && w < nw) tile[r][threadIdx.x] = U[(size_t)dat_row(w, Q, M) * ntr + tr0 + b];
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -851,12 +1100,14 @@ enum CacheSlot {
     CB_CABS,
     CB_GEOM,
     CB_RTAU,
-    CB_STAU,
+    CB_SGW,
     CB_SL,
     CB_SR,
     CB_IHM,
-    CB_IRL,
-    CB_IRH,
+    CB_GOFF,
+    CB_GATH,
+    CB_RAMP,
+    CB_TW,      // twiddles of the operators' FFTs
     CB_COUNT
 };
 
@@ -865,7 +1116,8 @@ const char *const kSlotName[CB_COUNT] = {
     "the source operator", "the transform buffer", "the transform buffer", "the transform work area",
     "the input traces", "the output traces", "the intermediate traces", "a status word", "trace weights",
     "receiver terms", "source terms", "receiver indices", "receiver weights", "receiver pair times",
-    "source pair times", "gather ranges", "gather ranges", "gather traces", "gather ranges", "gather ranges"};
+    "source pair weights", "gather ranges", "gather ranges", "gather traces", "gather lists", "gather lists",
+    "the edge taper", "twiddles"};
 
 struct CBuf {
     void *p = nullptr;
@@ -1040,11 +1292,13 @@ struct Host {
     std::vector<DatEntry> rcv, src;
     // cmp = 1 receiver side
     std::vector<int> cabs;        // [ns][nh]
-    std::vector<float> geom, rtau;  // [nh][nh], [nrow][2 band + 1]
+    std::vector<float> geom, rtau;  // [nh][nh] (input trace first), [nrow][2 band + 1]
     int band = 0, row0 = 0, nrow = 0;
     // cmp = 1 source side
-    std::vector<float> stau;  // [ns][ns]
-    std::vector<int> sleft, sright, ihmap, ir_lo, ir_hi;
+    std::vector<double> sgw;   // [ns][ns] geometric weight times tau
+    std::vector<float> ramp;   // edge taper by the distance from a window's end
+    std::vector<int> sleft, sright, ihmap;  // [nr], [nr], [ns][nr]
+    std::vector<int> goff, gath;            // the gathers of each output trace, in order
     int nr = 0, jump = 1;
 };
 
@@ -1087,7 +1341,7 @@ int build_receiver(const kcig_datum_params &p, const float *rt, Host &h)
         for (int ic = left; ic <= right; ic++) {
             const float coef = taper_host(left, ic, right, p.taper, 1);
             const float dist = p.rdatum * p.rdatum + (float)((ic - ih) * (ic - ih)) * p.dh * p.dh;
-            h.geom[(size_t)ih * nh + ic] = (float)(coef / M_PI * p.dh * p.rdatum / dist);
+            h.geom[(size_t)ic * nh + ih] = (float)(coef / M_PI * p.dh * p.rdatum / dist);
         }
         for (int is = 0; is < ns && left <= right; is++) {
             const int c = h.cabs[(size_t)is * nh + ih];
@@ -1156,8 +1410,7 @@ int build_source(const kcig_datum_params &p, const float *st, Host &h)
     h.sleft.resize(nr);
     h.sright.resize(nr);
     h.ihmap.assign((size_t)nr * ns, -1);
-    h.ir_lo.assign(ns, 0);
-    h.ir_hi.assign(ns, -1);
+    h.goff.assign((size_t)ns * nh + 1, 0);
     const float as = ds <= 0.f ? -1.f : 0.f, ah = dh <= 0.f ? -1.f : 0.f, bl = ds <= 0.f ? 0.f : -1.f;
     for (int ir = 0; ir < nr; ir++) {
         const float r = (float)ir * dr + as * s + ah * hl;
@@ -1176,13 +1429,29 @@ int build_source(const kcig_datum_params &p, const float *st, Host &h)
             const int c = cs[is];
             if (c < 0 || c >= nsg) return set_error(KCIG_ERR_ARG, "Source table too small.");
             const int ih = f2i((r - (float)is * ds) / dh + 0.5f);
-            h.ihmap[(size_t)ir * ns + is] = (ih >= 0 && ih < nh) ? ih : -1;
-            if (h.ir_hi[is] < h.ir_lo[is]) h.ir_lo[is] = ir;
-            h.ir_hi[is] = ir;
+            if (ih < 0 || ih >= nh) continue;
+            h.ihmap[(size_t)is * nr + ir] = ih;
+            h.goff[(size_t)is * nh + ih + 1]++;
         }
     }
+    // the gathers that hold each output trace, in order of r
+    for (size_t t = 0; t < (size_t)ns * nh; t++) h.goff[t + 1] += h.goff[t];
+    h.gath.resize(h.goff.back());
+    std::vector<int> at(h.goff.begin(), h.goff.end() - 1);
+    for (int ir = 0; ir < nr; ir++)
+        for (int is = std::max(0, h.sleft[ir]); is <= std::min(ns - 1, h.sright[ir]); is++) {
+            const int ih = h.ihmap[(size_t)is * nr + ir];
+            if (ih >= 0) h.gath[at[(size_t)is * nh + ih]++] = ir;
+        }
+    // half of taper_weight (:229-240), by the distance from a window's end
+    if (p.taper > 0) {
+        const float width = (float)p.taper * (float)jump;
+        for (int k = 0; k < ns && (float)k < width; k++)
+            h.ramp.push_back((float)(0.5 * (1.0 - cos(M_PI * (double)((float)k / width)))));
+    }
+    const double kw = (double)ds * (double)p.sdatum / M_PI;
     h.src.assign((size_t)ns * ns, DatEntry{0.0f, 0.0f, 0.0f});
-    h.stau.assign((size_t)ns * ns, 0.0f);
+    h.sgw.assign((size_t)ns * ns, 0.0);
     const float jds = fabsf((float)jump * ds);
     for (int is = 0; is < ns; is++)
         for (int ic = std::max(0, is - jump * aper); ic <= std::min(ns - 1, is + jump * aper); ic++) {
@@ -1192,7 +1461,8 @@ int build_source(const kcig_datum_params &p, const float *st, Host &h)
             e.w = 1.0f;
             e.tau = st[(size_t)cc * nsg + c];
             e.dtau = slope_host(st, nsg, cc, c, p.dsg) * jds;
-            h.stau[(size_t)is * ns + ic] = e.tau;
+            const float dist = p.sdatum * p.sdatum + (float)((ic - is) * (ic - is)) * ds * ds;
+            h.sgw[(size_t)is * ns + ic] = kw * (double)e.tau / (double)dist;
         }
     return KCIG_OK;
 }
@@ -1220,6 +1490,51 @@ int launch_op(const DatEntry *ent, int ne, float2 *out, int f0, int nf, int nfft
     launches++;
     KCIG_CUDA(cudaGetLastError());
     return KCIG_OK;
+}
+
+// Q of the FFT form: the smallest of 8 .. 64 that holds the filter's K + 1
+// samples, with at least two residues; 0 (longer filters): Horner's rule
+int op_points(int K, int nfft)
+{
+    if (K < 1) return 0;
+    for (int Q = 8; Q <= 64; Q *= 2)
+        if (K + 1 <= Q) return nfft >= 2 * Q ? Q : 0;
+    return 0;
+}
+
+template <int Q>
+int launch_op_q(const DatFftArgs &a, cudaStream_t st)
+{
+    KCIG_TRY(set_dyn_smem((const void *)k_dat_op_fft<Q>, dat_op_smem<Q>()));
+    constexpr int EB = 2048 / Q;
+    k_dat_op_fft<Q><<<dim3((a.ne + EB - 1) / EB, (a.na + kOpGroup - 1) / kOpGroup), 256, dat_op_smem<Q>(), st>>>(a);
+    KCIG_CUDA(cudaGetLastError());
+    return KCIG_OK;
+}
+
+int launch_op_fft(const DatEntry *ent, int ne, float2 *out, const C64 *tw, int Q, int M, int a0, int na, int nfft, int K,
+                  const kcig_datum_params &p, cudaStream_t st, int &launches)
+{
+    if (ne <= 0) return KCIG_OK;
+    DatFftArgs a;
+    a.ent = ent;
+    a.tw = tw;
+    a.out = out;
+    a.ne = ne;
+    a.a0 = a0;
+    a.na = na;
+    a.M = M;
+    a.K = K;
+    a.nfft = nfft;
+    a.dt = p.dt;
+    a.antialias = p.antialias;
+    launches++;
+    switch (Q) {
+    case 8: return launch_op_q<8>(a, st);
+    case 16: return launch_op_q<16>(a, st);
+    case 32: return launch_op_q<32>(a, st);
+    default: return launch_op_q<64>(a, st);
+    }
 }
 
 int launch_gemm(const float2 *A, long long sA, int lda, const float2 *B, long long sB, int ldb, float2 *C,
@@ -1466,6 +1781,26 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
     const size_t per_f = (interm ? 0 : (size_t)ntr * sizeof(float2)) + (op_r + op_s) * sizeof(float2);
     int chunk = (int)std::max<size_t>(1, std::min<size_t>(256, ((size_t)1536 << 20) / std::max<size_t>(per_f, 1)));
     chunk = std::min(chunk, nw);
+    // rows of the spectra in residue order when the operators come from FFTs:
+    // a chunk is then a group of residues (Q rows each; the first Q / 2 + 1,
+    // the last Q / 2)
+    const int Q = op_points(K, nfft), M = Q ? nfft / Q : 0;
+    const int chunk_res = Q ? std::max(1, chunk / Q) : 0;
+    struct Chunk {
+        int f0, nf, a0, na;
+    };
+    std::vector<Chunk> chunks;
+    if (Q) {
+        auto row_of = [&](int r) { return r == 0 ? 0 : r > M / 2 ? nw : Q / 2 + 1 + (r - 1) * Q; };
+        for (int a0 = 0; a0 <= M / 2; a0 += chunk_res) {
+            const int a1 = std::min(M / 2 + 1, a0 + chunk_res);
+            chunks.push_back({row_of(a0), row_of(a1) - row_of(a0), a0, a1 - a0});
+        }
+        chunk = 0;
+        for (const Chunk &k : chunks) chunk = std::max(chunk, k.nf);
+    } else {
+        for (int f0 = 0; f0 < nw; f0 += chunk) chunks.push_back({f0, std::min(chunk, nw - f0), 0, 0});
+    }
     // transform batches
     const int B = (int)transform_batch(ntr, nfft);
     const int tail = (int)(ntr % B);
@@ -1494,6 +1829,7 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
         if (interm) need[CB_INTERM] = (size_t)ntr * nt * 4;
     }
     need[CB_STATUS] = sizeof(int);
+    need[CB_TW] = Q ? (size_t)(M / 2 + 1) * 2 * Q * sizeof(C64) : 16;
     need[CB_WTR] = upload_bytes(wtr);
     need[CB_RCV] = upload_bytes(h.rcv);
     need[CB_SRC] = upload_bytes(h.src);
@@ -1501,12 +1837,13 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
         need[CB_CABS] = upload_bytes(h.cabs);
         need[CB_GEOM] = upload_bytes(h.geom);
         need[CB_RTAU] = upload_bytes(h.rtau);
-        need[CB_STAU] = upload_bytes(h.stau);
+        need[CB_SGW] = upload_bytes(h.sgw);
         need[CB_SL] = upload_bytes(h.sleft);
         need[CB_SR] = upload_bytes(h.sright);
         need[CB_IHM] = upload_bytes(h.ihmap);
-        need[CB_IRL] = upload_bytes(h.ir_lo);
-        need[CB_IRH] = upload_bytes(h.ir_hi);
+        need[CB_GOFF] = upload_bytes(h.goff);
+        need[CB_GATH] = upload_bytes(h.gath);
+        need[CB_RAMP] = upload_bytes(h.ramp);
     }
     KCIG_TRY(ensure_buffers(c, need));
     const CBuf *bf = c.buf;
@@ -1536,12 +1873,13 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
         KCIG_TRY(upload_to(bf[CB_CABS], h.cabs, st));
         KCIG_TRY(upload_to(bf[CB_GEOM], h.geom, st));
         KCIG_TRY(upload_to(bf[CB_RTAU], h.rtau, st));
-        KCIG_TRY(upload_to(bf[CB_STAU], h.stau, st));
+        KCIG_TRY(upload_to(bf[CB_SGW], h.sgw, st));
         KCIG_TRY(upload_to(bf[CB_SL], h.sleft, st));
         KCIG_TRY(upload_to(bf[CB_SR], h.sright, st));
         KCIG_TRY(upload_to(bf[CB_IHM], h.ihmap, st));
-        KCIG_TRY(upload_to(bf[CB_IRL], h.ir_lo, st));
-        KCIG_TRY(upload_to(bf[CB_IRH], h.ir_hi, st));
+        KCIG_TRY(upload_to(bf[CB_GOFF], h.goff, st));
+        KCIG_TRY(upload_to(bf[CB_GATH], h.gath, st));
+        KCIG_TRY(upload_to(bf[CB_RAMP], h.ramp, st));
     }
     float2 *const U = bf[CB_U].as<float2>();
     float2 *const Kr = bf[CB_KR].as<float2>(), *const Ks = bf[CB_KS].as<float2>();
@@ -1552,7 +1890,7 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
     // the call has finished, so the chunks are queued back to back), and for
     // host-memory calls per batch of traces: its input copied, its interm
     // and output traces finished
-    const int nchunk = (nw + chunk - 1) / chunk;
+    const int nchunk = (int)chunks.size();
     const int nbatch = (int)((ntr + B - 1) / B);
     while (c.ev.size() < 4 + 4 * (size_t)nchunk + 3 * (size_t)nbatch) {
         cudaEvent_t e;
@@ -1585,21 +1923,32 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
             return cufft_error(cr, "cufftExecR2C");
         launches++;
         k_dat_to_fmajor<<<dim3((nw + 31) / 32, (nb + 31) / 32), dim3(32, 8), 0, st>>>(spec, U, (int)t0, nb, nw,
-                                                                                     (int)ntr);
+                                                                                     (int)ntr, Q, M);
         launches++;
         KCIG_CUDA(cudaGetLastError());
         if (cs && ib + 1 < nbatch) KCIG_TRY(copy_in((int)ib + 1));
     }
     KCIG_CUDA(cudaEventRecord(ev[1], st));
     // ---- per chunk of frequencies: operators, receiver side, source side
-    for (int f0 = 0, ic = 0; f0 < nw; f0 += chunk, ic++) {
-        const int nf = std::min(chunk, nw - f0);
+    if (Q) {
+        const int n = (M / 2 + 1) * 2 * Q;
+        k_dat_twiddles<<<(n + 255) / 256, 256, 0, st>>>(bf[CB_TW].as<C64>(), Q, M);
+        launches++;
+        KCIG_CUDA(cudaGetLastError());
+    }
+    auto build_op = [&](const DatEntry *ent, size_t ne, float2 *K_out, const Chunk &k) -> int {
+        if (Q)
+            return launch_op_fft(ent, (int)ne, K_out, bf[CB_TW].as<C64>(), Q, M, k.a0, k.na, nfft, K, p, st, launches);
+        return launch_op(ent, (int)ne, K_out, k.f0, k.nf, nfft, K, p, st, launches);
+    };
+    for (int ic = 0; ic < nchunk; ic++) {
+        const int f0 = chunks[ic].f0, nf = chunks[ic].nf;
         cudaEvent_t *const ce = ev + 4 + 4 * ic;
         float2 *Uc = U + (size_t)f0 * ntr;
         float2 *Utc = interm ? bf[CB_UFULL].as<float2>() + (size_t)f0 * ntr : bf[CB_UT].as<float2>();
         KCIG_CUDA(cudaEventRecord(ce[0], st));
-        KCIG_TRY(launch_op(bf[CB_RCV].as<DatEntry>(), (int)op_r, Kr, f0, nf, nfft, K, p, st, launches));
-        if (op_s) KCIG_TRY(launch_op(bf[CB_SRC].as<DatEntry>(), (int)op_s, Ks, f0, nf, nfft, K, p, st, launches));
+        KCIG_TRY(build_op(bf[CB_RCV].as<DatEntry>(), op_r, Kr, chunks[ic]));
+        if (op_s) KCIG_TRY(build_op(bf[CB_SRC].as<DatEntry>(), op_s, Ks, chunks[ic]));
         KCIG_CUDA(cudaEventRecord(ce[1], st));
         if (p.cmp == 0) {
             if (tcore)
@@ -1622,8 +1971,9 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
             a.band = h.band;
             a.row0 = h.row0;
             a.nrow = h.nrow;
+            a.nf = nf;
             a.sU = ntr;
-            k_dat_rcv_cmp1<<<dim3((unsigned)((ntr + 127) / 128), nf), 128, 0, st>>>(a);
+            k_dat_rcv_cmp1<<<dim3((unsigned)((ntr + 127) / 128), (nf + kCmp1F - 1) / kCmp1F), 128, 0, st>>>(a);
             launches++;
             KCIG_CUDA(cudaGetLastError());
         }
@@ -1639,27 +1989,26 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
                 KCIG_TRY(launch_gemm(Ks, (long long)ns * ns, ns, Utc, ntr, nh, Uc, ntr, nh, ns, nh, ns,
                                      p.aperture >= 0 ? p.aperture : 0, 1, nf, st, launches));
         } else {
-            KCIG_CUDA(cudaMemsetAsync(Uc, 0, (size_t)nf * ntr * sizeof(float2), st));
             SrcCmp1Args a;
             a.Utmp = Utc;
             a.Uout = Uc;
             a.P = Ks;
-            a.Ptau = bf[CB_STAU].as<float>();
+            a.gw = bf[CB_SGW].as<double>();
             a.sleft = bf[CB_SL].as<int>();
             a.sright = bf[CB_SR].as<int>();
             a.ihmap = bf[CB_IHM].as<int>();
-            a.ir_lo = bf[CB_IRL].as<int>();
-            a.ir_hi = bf[CB_IRH].as<int>();
+            a.goff = bf[CB_GOFF].as<int>();
+            a.gath = bf[CB_GATH].as<int>();
+            a.ramp = bf[CB_RAMP].as<float>();
             a.ns = ns;
             a.nh = nh;
             a.nr = h.nr;
             a.aper = p.aperture;
             a.jump = h.jump;
-            a.tap = p.taper;
-            a.ds = p.ds;
-            a.sdatum = p.sdatum;
+            a.nramp = (int)h.ramp.size();
+            a.nf = nf;
             a.sUout = ntr;
-            k_dat_src_cmp1<<<dim3((ns + 127) / 128, nf), 128, 0, st>>>(a);
+            k_dat_src_cmp1<<<dim3((unsigned)((ntr + 127) / 128), (nf + kCmp1F - 1) / kCmp1F), 128, 0, st>>>(a);
             launches++;
             KCIG_CUDA(cudaGetLastError());
         }
@@ -1671,7 +2020,7 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
         for (long long t0 = 0, ib = 0; t0 < ntr; t0 += B, ib++) {
             const int nb = (int)std::min<long long>(B, ntr - t0);
             k_dat_to_tmajor<<<dim3((nb + 31) / 32, (nw + 31) / 32), dim3(32, 8), 0, st>>>(Usrc, spec, (int)t0, nb, nw,
-                                                                                         (int)ntr);
+                                                                                         (int)ntr, Q, M);
             launches++;
             KCIG_CUDA(cudaGetLastError());
             if ((cr = cufftExecC2R(nb == B ? c.full.b : c.tail.b, (cufftComplex *)spec, (cufftReal *)pad)) != CUFFT_SUCCESS)
