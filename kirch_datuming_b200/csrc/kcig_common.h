@@ -102,6 +102,22 @@ int launch_surrogate_fields(kcig_surrogate *s, const LegInterp *legs, int nlegs,
 int sg_reset_status(kcig_surrogate *s, cudaStream_t st);
 int sg_check_status(kcig_surrogate *s, cudaStream_t st);
 
+// Reciprocal traces of a survey that shoots from its own stations (cmp = 0).
+// Where shot s stands on receiver s + off with the same leg (position, table,
+// spacing), the traces (s, r) and (r - off, s + off) have the same traveltime
+// sum, angle, window and weights at every image point: their samples are
+// added once and the pair is migrated once.  Shots go in groups of kFoldGroup
+// (a block of the summation lies in one group); groups ga .. gb - 1 have all
+// their shots on receivers.  Of two traces whose shots' groups differ the one
+// of the smaller group is kept; traces inside a group stay apart.  Half the
+// pairs and half the leg fields of such a survey are left (601 x 1601, 400
+// shots on 400 receivers: summation 385 -> 190 ms, leg fields 32 -> 16 ms).
+constexpr int kFoldGroup = 4;
+struct Fold {
+    int on, off, ga, gb;
+    int ns;  // shots of the call (the last group may be partial)
+};
+
 struct PreludeArgs {
     const float *data;      // [ns][nh][nt] whole data cube on the device
     double2 *D;             // [ntr][nt] {D[i], D[i+1]}, ntr = nshots * nhc
@@ -115,6 +131,7 @@ struct PreludeArgs {
     // sample count (<= nt, the row stride of D)
     const long long *toff;
     const int *tnt;
+    Fold fold;  // reciprocal traces added to the kept ones, the others skipped
 };
 int launch_prelude(const PreludeArgs &a, cudaStream_t st);
 int launch_doubint_plain(const float *in, double *out, int ntr, int nt, int isdiff, double dt,
@@ -150,6 +167,9 @@ struct SumArgs {
     float dtf, aal, g0, dg;
     float oazmin, oazmax, oaztaper, ats, ate;
     int gchunk0, gchunk1;  // bin range handled by this launch
+    Fold fold;             // pairs of skipped reciprocal traces are left out
+    int shot0, rcv0;       // first shot and receiver of the batch in the call
+    int trs;               // traces per shot in D and the per-trace arrays (nh, or more)
 };
 int launch_sum(const SumArgs &a, cudaStream_t st, int *launches);
 // Tile variants the summation can be launched with (the autotuner's choices):

@@ -200,6 +200,15 @@ __global__ void __launch_bounds__(32 * kPreludeWarps) k_prelude_cta(PreludeArgs 
         x = a.data + off;
         nt = a.tnt[tr];
     }
+    const float *x2 = nullptr;  // the reciprocal trace (same mute: the same offset)
+    if (a.fold.on) {
+        const int s = a.shot0 + k, r = a.rcv0 + rr, s2 = r - a.fold.off;
+        const int g = s / kFoldGroup, g2 = s2 >= 0 && s2 < a.fold.ns ? s2 / kFoldGroup : -1;
+        if (g >= a.fold.ga && g < a.fold.gb && g2 >= a.fold.ga && g2 < a.fold.gb && g != g2) {
+            if (g2 < g) return;  // migrated with its reciprocal
+            x2 = a.data + ((size_t)s2 * a.nh + (s + a.fold.off)) * a.nt;
+        }
+    }
     double boundary = 0.0;
     const bool mute = a.mute_sx != nullptr;
     if (mute) {
@@ -208,6 +217,7 @@ __global__ void __launch_bounds__(32 * kPreludeWarps) k_prelude_cta(PreludeArgs 
     }
     for (int i = tid; i < nt; i += PT) {
         double v = (double)__ldg(x + i);
+        if (x2) v += (double)__ldg(x2 + i);
         if (mute) {
             const double t = a.t0 + (double)i * a.dt;
             double w = 0.0;
@@ -1055,7 +1065,7 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 #define KCIG_SUM_MINB_UNSHARED KCIG_SUM_MINB
 #endif
 
-template <int TZ, int TX, int KB, bool SHARED_R, int MODE>
+template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool FOLD>
 __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_MINB_UNSHARED) * 128 / (TZ * TX))
     k_sum(const __grid_constant__ SumArgs a)
 {
@@ -1070,13 +1080,18 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     const int nzx = a.nz * a.nx;
     const int i = valid ? ix * a.nz + iz : 0;
     const int gc0 = a.gchunk0, nb = a.gchunk1 - a.gchunk0;
-    // this CTA row's share of the shots (whole blocks of KB)
+    // this CTA row's share of the shots (whole blocks of KB); of folded
+    // surveys, whose later blocks have fewer receivers left, every nsplit-th
     int s_lo = 0, s_hi = a.nsb;
     float *out = a.image;
     if (a.nsplit > 1) {
         const int nblk = (a.nsb + KB - 1) / KB;
-        s_lo = (int)((long long)nblk * blockIdx.y / a.nsplit) * KB;
-        s_hi = min(a.nsb, (int)((long long)nblk * (blockIdx.y + 1) / a.nsplit) * KB);
+        if (FOLD) {
+            s_lo = (int)blockIdx.y * KB;
+        } else {
+            s_lo = (int)((long long)nblk * blockIdx.y / a.nsplit) * KB;
+            s_hi = min(a.nsb, (int)((long long)nblk * (blockIdx.y + 1) / a.nsplit) * KB);
+        }
         out = a.partial + (size_t)blockIdx.y * a.ng * nzx;
     }
     const bool fresh = a.zero_init || a.nsplit > 1;
@@ -1104,7 +1119,14 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     // shot (receivers not shared), so that KB independent (shot, receiver)
     // gather chains are in flight per thread either way
     constexpr int KR = SHARED_R ? 1 : KB;
-    for (int sb = s_lo; sb < s_hi; sb += KB) {
+    for (int sb = s_lo; sb < s_hi; sb += FOLD ? KB * a.nsplit : KB) {
+        // first receiver: a folded block starts at its own shots' receivers
+        // (the traces before them are migrated with their reciprocals)
+        int r0 = 0;
+        if (FOLD) {
+            const int g = (a.shot0 + sb) / kFoldGroup;
+            if (g > a.fold.ga && g < a.fold.gb) r0 = max(0, kFoldGroup * g + a.fold.off - a.rcv0);
+        }
         double2 sTP[KB];
         float2 sXW[KB];
 #pragma unroll
@@ -1140,15 +1162,15 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
             fnext[j] = 0;
             nTP[j] = make_double2(0.0, 0.0);
             nXW[j] = make_float2(0.f, 0.f);
-            if (nrk[j] > 0) {
+            if (FOLD ? r0 < nrk[j] : nrk[j] > 0) {
                 const int *rfi_j = a.rfi + (size_t)(sb + j) * a.nh;
-                const size_t f0 = SHARED_R ? 0 : (size_t)__ldg(rfi_j);
+                const size_t f0 = SHARED_R ? (FOLD ? (size_t)r0 : 0) : (size_t)__ldg(rfi_j);
                 nTP[j] = __ldg(a.RTP + f0 * nzx + i);
                 nXW[j] = __ldg(a.RXW + f0 * nzx + i);
                 if (!SHARED_R && nrk[j] > 1) fnext[j] = __ldg(rfi_j + 1);
             }
         }
-        for (int r = 0; r < nr; r++) {
+        for (int r = FOLD ? r0 : 0; r < nr; r++) {
             double2 rTP[KR];
             float2 rXW[KR];
 #pragma unroll
@@ -1173,7 +1195,7 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 const double2 rTPk = rTP[j];
                 const float2 rXWk = rXW[j];
                 const double topj = topk[j];
-                const int trc = (sb + k) * a.nh + r;
+                const int trc = (sb + k) * a.trs + r;
                 const float tw = a.unit_tw ? 1.0f : __ldg(a.trw + trc);
                 if (tw == 0.0f) continue;  // trace removed by aperture_trace / offset bin
                 const float apw = sXW[k].y * rXWk.y;
@@ -1405,12 +1427,12 @@ __global__ void k_sum_reduce(float *image, const float *partial, int nsplit, siz
     image[j] = v;
 }
 
-template <int TZ, int TX, int KB, bool SR, int MODE>
+template <int TZ, int TX, int KB, bool SR, int MODE, bool FOLD = false>
 static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 {
     constexpr int P = TZ * TX;
     const size_t sm = (size_t)nb * P * sizeof(float);
-    auto kern = k_sum<TZ, TX, KB, SR, MODE>;
+    auto kern = k_sum<TZ, TX, KB, SR, MODE, FOLD>;
     // all of the unified L1/shared memory as shared: the accumulators of as
     // many CTAs as the registers allow (the driver's own choice held 8x8
     // tiles to 10 CTAs per SM)
@@ -1430,6 +1452,11 @@ static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 template <int TZ, int TX, int KB>
 static int launch_sum_mode(const SumArgs &a, int nb, cudaStream_t st)
 {
+    if (a.shared_r && a.fold.on) {
+        if (a.mode == 0) return launch_sum_t<TZ, TX, KB, true, 0, true>(a, nb, st);
+        if (a.mode == 1) return launch_sum_t<TZ, TX, KB, true, 1, true>(a, nb, st);
+        return launch_sum_t<TZ, TX, KB, true, 2, true>(a, nb, st);
+    }
     if (a.shared_r) {
         if (a.mode == 0) return launch_sum_t<TZ, TX, KB, true, 0>(a, nb, st);
         if (a.mode == 1) return launch_sum_t<TZ, TX, KB, true, 1>(a, nb, st);
@@ -1461,6 +1488,30 @@ const int kSumTileShape[kSumTiles][3] = {{0, 0, 0}, {16, 8, 4}, {8, 8, 4}, {8, 1
 
 int launch_sum(const SumArgs &a0, cudaStream_t st, int *launches)
 {
+    if (a0.fold.on) {
+        // receivers before the first folded group's: no trace of theirs has a
+        // reciprocal among the shots, they go as an unfolded summation first
+        const int lead = min(a0.nh, kFoldGroup * a0.fold.ga + a0.fold.off - a0.rcv0);
+        if (lead > 0) {
+            SumArgs a = a0;
+            a.fold.on = 0;
+            a.nh = lead;
+            KCIG_TRY(launch_sum(a, st, launches));
+            if (lead == a0.nh) return KCIG_OK;
+            a = a0;
+            const size_t nzx = (size_t)a.nz * a.nx;
+            a.rcv0 += lead;
+            a.nh -= lead;
+            a.RTP += lead * nzx;
+            a.RXW += lead * nzx;
+            a.D += (size_t)lead * a.nt;
+            a.trw += lead;
+            a.rfi += lead;
+            a.igo += lead;
+            a.zero_init = 0;
+            return launch_sum(a, st, launches);
+        }
+    }
     const int maxb = 384;
     for (int g = 0; g < a0.ng; g += maxb) {
         SumArgs a = a0;

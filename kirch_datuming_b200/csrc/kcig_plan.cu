@@ -217,6 +217,24 @@ int leg_interp(const kcig_plan *P, int is_source, float posf, double pos, LegInt
     return ret;
 }
 
+// The same leg fields: every value the leg kernels read.
+bool same_leg(const LegInterp &a, const LegInterp &b)
+{
+    bool eq = a.i0 == b.i0 && a.i1 == b.i1 && a.type == b.type && a.k1 == b.k1 && a.k2 == b.k2 && a.t == b.t &&
+              a.dxp == b.dxp && a.gi0 == b.gi0 && a.gi1 == b.gi1 && a.gw == b.gw && a.pos == b.pos &&
+              a.scale == b.scale && a.posf == b.posf && a.cexact == b.cexact && a.cs == b.cs && a.ch == b.ch;
+    for (int q = 0; q < 4; q++) eq = eq && a.c[q] == b.c[q] && a.e[q] == b.e[q];
+    return eq;
+}
+
+// Whether both sides take their leg fields from the same tables (or surrogate).
+bool same_sides(const kcig_plan *P)
+{
+    const kcig_geometry &g = P->g;
+    return P->sg_src == P->sg_rcv && P->stab == P->rtab && P->sder == P->rder && P->sgx == P->rgx && P->sgz == P->rgz &&
+           g.sny == g.rny && g.sy0 == g.ry0 && g.sdy == g.rdy && P->p.tool == 0;
+}
+
 // Legs per field launch and the FP64 work planes they need (4 per leg).
 int field_batch(const kcig_plan *P, size_t nlegs)
 {
@@ -693,6 +711,45 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
 
     // scratch plan: receivers shared across shots (cmp=0) are computed once
     const bool shared_r = !p.cmp;
+    // shots on receivers (struct Fold): off by the positions, then every shot
+    // group checked leg for leg; the traces' weights and bins have to be
+    // reciprocal too (they are all alike without a trace aperture)
+    std::vector<LegInterp> rlegs;
+    Fold fold = {0, 0, 0, 0, ns};
+    bool all_on_receivers = false;  // every shot of the call: its fields are a receiver's
+    if (shared_r) {
+        rlegs.resize(g.nh);
+        for (int r = 0; r < g.nh; r++) {
+            leg_interp(P, 0, hxf[r], hx[r], &rlegs[r]);
+            rlegs[r].scale = (float)dh;
+        }
+        const double q = dh != 0.0 ? rint((sx[0] - hx[0]) / dh) : 1e18;
+        if (same_sides(P) && (float)ds == (float)dh && fabs(q) < 1e9) {
+            fold.off = (int)q;
+            auto on = [&](int s) {
+                const long long r = (long long)s + fold.off;
+                return r >= 0 && r < g.nh && same_leg(slegs[s], rlegs[r]);
+            };
+            const int ngr = (ns + kFoldGroup - 1) / kFoldGroup;
+            auto group_on = [&](int k) {
+                for (int s = k * kFoldGroup; s < std::min(ns, (k + 1) * kFoldGroup); s++)
+                    if (!on(s)) return false;
+                return true;
+            };
+            while (fold.ga < ngr && !group_on(fold.ga)) fold.ga++;
+            fold.gb = fold.ga;
+            while (fold.gb < ngr && group_on(fold.gb)) fold.gb++;
+            all_on_receivers = fold.ga == 0 && fold.gb == ngr;
+            fold.on = fold.gb - fold.ga >= 2 && !(p.cig && !p.cig_is_angle);
+            if (fold.on && p.aperture_trace != -1)
+                for (int s = fold.ga * kFoldGroup; fold.on && s < std::min(ns, fold.gb * kFoldGroup); s++)
+                    for (int s2 = fold.ga * kFoldGroup; s2 < s; s2++)
+                        if (trw[(size_t)s * g.nh + s2 + fold.off] != trw[(size_t)s2 * g.nh + s + fold.off]) {
+                            fold.on = 0;
+                            break;
+                        }
+        }
+    }
     const size_t leg_bytes = nzx * (sizeof(double2) + sizeof(float2));
     const unsigned long long budget = P->budget;
     int nhc = g.nh;
@@ -705,6 +762,12 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     long long room = (long long)budget - (long long)fixed;
     int nsb = (int)std::max<long long>(1, room / (long long)per_shot);
     nsb = std::min(nsb, ns);
+    if (fold.on && nsb < ns) {  // shot batches of whole groups
+        if (nsb >= kFoldGroup) nsb -= nsb % kFoldGroup;
+        else fold.on = 0;
+    }
+    // every shot's fields are among the receivers' when those are all resident
+    const bool alias_src = all_on_receivers && nhc == g.nh;
 
     if (shared_r) {
         KCIG_TRY(P->d_rT.ensure((size_t)nhc * nzx * sizeof(double2)));
@@ -713,8 +776,10 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
         KCIG_TRY(P->d_rT.ensure((size_t)nsb * g.nh * nzx * sizeof(double2)));
         KCIG_TRY(P->d_rF.ensure((size_t)nsb * g.nh * nzx * sizeof(float2)));
     }
-    KCIG_TRY(P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2)));
-    KCIG_TRY(P->d_sF.ensure((size_t)nsb * nzx * sizeof(float2)));
+    if (!alias_src) {
+        KCIG_TRY(P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2)));
+        KCIG_TRY(P->d_sF.ensure((size_t)nsb * nzx * sizeof(float2)));
+    }
     KCIG_TRY(P->d_D.ensure((size_t)nsb * nhc * g.nt * sizeof(double2)));
     const size_t trn = (size_t)nsb * nhc;
     // one allocation: doubles first (8-byte aligned), then floats and ints
@@ -747,19 +812,22 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     for (int r0 = 0; r0 < g.nh && rc == KCIG_OK; r0 += nhc) {
         const int nhb = std::min(nhc, g.nh - r0);
         if (shared_r) {
-            std::vector<LegInterp> rl(nhb);
-            for (int r = 0; r < nhb; r++) {
-                leg_interp(P, 0, hxf[r0 + r], hx[r0 + r], &rl[r]);
-                rl[r].scale = (float)dh;
-            }
+            const std::vector<LegInterp> rl(rlegs.begin() + r0, rlegs.begin() + r0 + nhb);
             rc = fields(0, rl, P->d_rT.as<double2>(), P->d_rF.as<float2>());
             if (rc) break;
         }
         for (int s0 = 0; s0 < ns && rc == KCIG_OK; s0 += nsb) {
             const int nsh = std::min(nsb, ns - s0);
-            std::vector<LegInterp> sl(slegs.begin() + s0, slegs.begin() + s0 + nsh);
-            rc = fields(1, sl, P->d_sT.as<double2>(), P->d_sF.as<float2>());
-            if (rc) break;
+            const double2 *sT = P->d_sT.as<double2>();
+            const float2 *sF = P->d_sF.as<float2>();
+            if (alias_src) {
+                sT = P->d_rT.as<double2>() + (size_t)(s0 + fold.off) * nzx;
+                sF = P->d_rF.as<float2>() + (size_t)(s0 + fold.off) * nzx;
+            } else {
+                std::vector<LegInterp> sl(slegs.begin() + s0, slegs.begin() + s0 + nsh);
+                rc = fields(1, sl, P->d_sT.as<double2>(), P->d_sF.as<float2>());
+                if (rc) break;
+            }
             // per-trace arrays of this (shot batch, receiver chunk)
             std::vector<LegInterp> rl;
             // receiver legs by (FP64, float) position; kirchmig2d's cmp=1 cone
@@ -827,6 +895,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             pa.slope = p.direct_mute_slope;
             pa.intercept = p.direct_mute_intercept;
             pa.taper = p.direct_mute_taper;
+            pa.fold = fold;
             if (data_pending) {  // the traces have landed before their first use
                 cudaError_t e = cudaStreamWaitEvent(st, P->copy_ev, 0);
                 if (e != cudaSuccess) {
@@ -841,8 +910,12 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
 
             SumArgs sa;
             memset(&sa, 0, sizeof sa);
-            sa.STP = P->d_sT.as<double2>();
-            sa.SXW = P->d_sF.as<float2>();
+            sa.STP = sT;
+            sa.SXW = sF;
+            sa.fold = fold;
+            sa.shot0 = s0;
+            sa.rcv0 = r0;
+            sa.trs = nhb;
             sa.RTP = P->d_rT.as<double2>();
             sa.RXW = P->d_rF.as<float2>();
             sa.D = P->d_D.as<double2>();
@@ -1270,7 +1343,7 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.nx = g.nx;
     sa.nt = S->ntmax;
     sa.nsb = B.ns;
-    sa.nh = B.nhb;
+    sa.nh = sa.trs = B.nhb;
     sa.ng = P->ng;
     sa.mode = angle ? (p.angle_interp ? 0 : 1) : 2;
     sa.unit_tw = B.unit_tw;
