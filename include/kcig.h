@@ -499,7 +499,8 @@ int kcig_datum_freq(const kcig_datum_params *p, const float *stable, const float
                     float *interm, int memory, void *stream);
 
 /* Frees the buffers and plans kcig_datum_freq keeps for the calling thread's
- * current device (the next call allocates them again). */
+ * current device, and the memory kcig_eikods keeps there between calls (up to
+ * a sixteenth of the device); the next calls allocate them again. */
 int kcig_datum_release(void);
 
 /* Device time of the stages of the last kcig_datum_freq call on this thread

@@ -194,6 +194,9 @@ struct SprayArgs {
 int launch_spray(const SprayArgs &a, cudaStream_t st);
 int launch_doubint_f32(const double *in, float *out, int ntr, int nt, cudaStream_t st);
 
+// Gives back the memory kcig_eikods keeps between calls on the current device.
+int eik_release_pool();
+
 // How many shot splits a summation over nsb shots on an nz x nx image needs
 // to give the GPU at least two waves of CTAs (1: none).
 int sum_nsplit(int nz, int nx, int nsb, bool shared_r);

@@ -1670,7 +1670,7 @@ extern "C" int kcig_datum_release(void)
     c.ev.clear();
     if (c.copy) cudaStreamDestroy(c.copy);
     c.copy = nullptr;
-    return KCIG_OK;
+    return eik_release_pool();
 }
 
 extern "C" int kcig_datum_last_timing(float *ms5, int *launches)

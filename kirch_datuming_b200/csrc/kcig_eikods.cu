@@ -20,23 +20,29 @@
 // solved the same way: sweeps until nothing changes give exactly the ordered
 // result.
 //
-// Execution: one CTA per source.  Step k of a sweep updates anti-diagonal k
-// (local row r at local column k - r); a point's upwind neighbours (one and two
-// samples back along each axis) lie on diagonals k-1 and k-2, its downwind
-// neighbours on k+1 and k+2.  Diagonals k-2 .. k+D sit in a shared-memory ring
-// indexed by row; diagonal k+D is fetched from global memory with cp.async
-// while step k computes, so a step costs one barrier and no global-memory
-// round trip.  Thread t owns rows t, t + blockDim, ...  A point whose inputs
-// did not change since its previous evaluation is skipped (a per-point stamp
-// of the sweep of its last change), which changes no result.  There is no
-// wait other than the barriers and every loop has a fixed bound.
+// Execution: a CTA solves one source at a time, one anti-diagonal per step (the
+// points of a diagonal depend on others' only), thread t taking rows t,
+// t + blockDim, ...  Two sweep orderings run along the diagonals iz + ix =
+// const, two along iz - ix = const, so every source's working values are kept
+// in both diagonal-major layouts: the rows a step needs are contiguous and
+// come by 16-byte cp.async into a shared-memory ring (diagonals p - 2 .. p + D
+// around the current one), fetched D steps ahead.  A value that changes is
+// written to the ring and to both layouts.  In the plain layout every row of
+// a diagonal is a cache line of its own, and a sweep ran at one L1 wavefront
+// per row and step: 400 sources of 601 x 1601 in 83 ms, 169 ms with
+// tdl1/tds1, now 28 and 66 ms.
 //
-// Cost: a step gathers one anti-diagonal, one cache line per row, so the
-// passes run at about one L1 wavefront per row and step (400 sources of the
-// 601 x 1601 salt model in 83 ms for the time, 182 ms with tdl1/tds1).
+// Points whose inputs did not change since their previous evaluation are
+// skipped (a stamp of the sweep of its last change beside every value), and
+// so are whole blocks of diagonals without a change in reach: both change no
+// result.  The quiet sweeps that end a pass cost only that test.  There is no
+// wait other than the barriers and every loop has a fixed bound.
 #include <float.h>
 #include <math.h>
 
+#include <algorithm>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "kcig_common.h"
@@ -52,30 +58,62 @@ struct EikSource {
     float xs0, xs1, xs2;     // source minus origin: depth, lateral, third axis
 };
 
-struct EikArgs {
-    const float *vv;    // slowness squared [nx][nz]
-    const double *dw;   // derivative of vv along axis l [nx][nz]
-    const EikSource *src;
-    float *T, *dl1, *ds1;  // [nsrc][nx][nz]
-    int *status;           // set to 1 when a source has no fixed point within max_iter
-    int *iters;            // [nsrc] sweeps the traveltime pass took (0: no fixed point)
-    unsigned *stamp;       // [nsrc][nx][nz] 1 + the sweep of a point's last change (0: none)
-    int nz, nx, order, l, max_iter;
-    float d0, d1, d2;  // sampling: depth, lateral, third axis
-    float rdx0, rdx1;  // 1 / d^2 rounded to float (neighbors.cpp:19-30)
+// the same in FP32 for a = 0 or |a| >= 2^-80 (below, the remainder could underflow)
+__device__ __forceinline__ float div_by(float a, float b, float y)
+{
+    if (fabsf(a) < 8.27e-25f && a != 0.0f) return __fdiv_rn(a, b);
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// Reciprocals of the divisors of the local problem; [second order on axis 0]
+// [on axis 1] of the two-axis sum, [axis][second order] of one axis
+struct EikRecip {
+    double two[2][2], one[2][2];
 };
 
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
+struct EikArgs {
+    const float *vv;   // [2][nd + 2 kEikBorder][np] slowness squared, both layouts (skew_index)
+    const double *dw;  // [2][nd + 2 kEikBorder][np] derivative of vv along axis l
+    const float *vplain;  // [nx][nz]
+    const EikSource *src;
+    float *T, *dl1;    // [nsrc][nx][nz]
+    unsigned char *work;  // per CTA: slot_bytes
+    size_t slot_bytes;
+    int *next;         // sources handed out so far
+    int *status;       // set to 1 when a source has no fixed point within max_iter
+    int *iters;        // [nsrc] sweeps the traveltime pass took (0: no fixed point)
+    int nsrc, nz, nx, np, nd, order, max_iter;
+    int blk_shift, nblk;  // diagonals per skipping block (a power of two), blocks
+    float d0, d1, d2;  // sampling: depth, lateral, third axis
+    float rdx0, rdx1;  // 1 / d^2 rounded to float (neighbors.cpp:19-30)
+    float dd0, dd1, yd0, yd1;  // d^2 of both axes and its reciprocal
+    EikRecip rc;
+};
+
+// Diagonal-major layouts: family 0 holds diagonal p = iz + ix, family 1 p = iz
+// - ix + nx - 1, each as a row of np >= nz + 2 entries (np a multiple of 16)
+// indexed by iz; kEikBorder border rows before and after, and every entry
+// outside the grid, keep the border value for good.
+constexpr int kEikBorder = 8;
+__host__ __device__ __forceinline__ size_t skew_row(int p, int np) { return (size_t)(p + kEikBorder) * np; }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+__device__ __forceinline__ uint2 lds64(uint32_t addr)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float lds32(uint32_t addr)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -84,77 +122,73 @@ __device__ __forceinline__ void cp_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// one axis of the local problem (neighbors.cpp struct Upd)
-struct Upd {
-    double stencil, value, delta;
-};
+// a / b correctly rounded, y = RN(1 / b): Markstein's theorem (IBM J. Res.
+// Dev. 34, 1990) -- with q within an ulp of a / b and r = a - b q exact, q +
+// r y rounds to RN(a / b); the first correction brings q within an ulp.
+// The divisors of a point's update are few (sums of the axes' weights), so
+// their reciprocals come from the host, and the serial chain that bounds a
+// step shortens: five dependent operations for a general division's dozen.
+__device__ __forceinline__ double div_by(double a, double b, double y)
+{
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
 
 // neighbors.cpp:106-160 for one axis, with stencil() (:271-276): the
 // smaller neighbour, or the second-order one-sided value when the sample two
-// steps further is not larger
-__device__ __forceinline__ void upd_axis(Upd &x, float a, float b, float a2, float b2, float rdx, int order)
+// steps further is not larger.  a2 / b2 are kFar where that sample is outside
+// the grid or not reached, which fails the comparisons exactly as the marching
+// code's bounds and status checks do.
+__device__ __forceinline__ bool upd_axis(float a, float b, float a2, float b2, int order, double &stencil, float &value)
 {
-    const float m = (a < b) ? a : b;
-    const double v = (double)m;
-    x.value = x.stencil = v;
-    x.delta = (double)rdx;
-    if (order > 1) {
-        // a2 / b2 are kFar where the sample two steps away is outside the grid
-        // or not reached, which fails the comparisons exactly as the marching
-        // code's bounds and status checks do
-        const float t2 = (a < b) ? a2 : b2;
-        if ((a < b && a >= a2) || (a > b && b >= b2)) {
-            x.stencil = __ddiv_rn(__dsub_rn(__dmul_rn(4.0, v), (double)t2), 3.0);
-            x.delta = __dmul_rn(x.delta, 2.25);
-        }
-    }
+    value = fminf(a, b);  // never NaN
+    const double v = (double)value;
+    const float t2 = (a < b) ? a2 : b2;
+    const bool second = order > 1 && a != b && value >= t2;
+    const double s2 = div_by(__fma_rn(4.0, v, -(double)t2), 3.0, 1.0 / 3.0);  // 4 v is exact
+    stencil = second ? s2 : v;
+    return second;
 }
 
-// neighbors.cpp:278-302 updaten(): root of sum_j delta_j (t - stencil_j)^2 =
-// v1 over the first m axes in increasing order of value; false if not causal
-__device__ __forceinline__ bool upd_solve(int m, const Upd &p, const Upd &q, double v1, float &res)
+// neighbors.cpp:278-302 updaten() past its sums: root of A t^2 - 2 B t + C =
+// v1, `false` if it is not above `value` (not causal)
+__device__ __forceinline__ bool upd_root(double A, double B, double C, double y, double v1, float value, float &res)
 {
-    double A = __dadd_rn(0.0, p.delta);
-    double B = __dadd_rn(0.0, __dmul_rn(p.stencil, p.delta));
-    double C = __dadd_rn(0.0, __dmul_rn(__dmul_rn(p.stencil, p.stencil), p.delta));
-    if (m > 1) {
-        A = __dadd_rn(A, q.delta);
-        B = __dadd_rn(B, __dmul_rn(q.stencil, q.delta));
-        C = __dadd_rn(C, __dmul_rn(__dmul_rn(q.stencil, q.stencil), q.delta));
-    }
-    B = __ddiv_rn(B, A);
-    const double discr = __dadd_rn(__dmul_rn(B, B), __ddiv_rn(__dsub_rn(v1, C), A));
-    if (discr < 0.0) return false;
+    B = div_by(B, A, y);
+    const double discr = __dadd_rn(__dmul_rn(B, B), div_by(__dsub_rn(v1, C), A, y));
     const double t = __dadd_rn(B, __dsqrt_rn(discr));
-    if (t <= (m > 1 ? q.value : p.value)) return false;
     res = __double2float_rn(t);
-    return true;
+    return !(discr < 0.0) && !(t <= (double)value);
 }
 
-// neighbors.cpp:106-188 qsolve() on a 2-D grid (the third axis never contributes)
+// neighbors.cpp:106-188 qsolve() on a 2-D grid (the third axis never
+// contributes): the two-axis root, else the one of the smaller axis alone.
+// (The sums over the axes do not depend on their order.)
 __device__ __forceinline__ float qsolve2d(float zm, float zp, float zm2, float zp2, float xm, float xp, float xm2,
-                                          float xp2, float vv, float rdx0, float rdx1, int order)
+                                          float xp2, float vv, float rdx0, float rdx1, int order, const EikRecip &rc)
 {
-    Upd x0, x1;
-    upd_axis(x0, zm, zp, zm2, zp2, rdx0, order);
-    upd_axis(x1, xm, xp, xm2, xp2, rdx1, order);
-    // the marching code sorts the three axes by value; with the third axis at
-    // FLT_MAX the first two keep their order unless x1 < x0
-    const bool swap = !(x0.value <= x1.value);
-    Upd p, q;  // selected field by field: no address of a local is taken
-    p.stencil = swap ? x1.stencil : x0.stencil;
-    p.value = swap ? x1.value : x0.value;
-    p.delta = swap ? x1.delta : x0.delta;
-    q.stencil = swap ? x0.stencil : x1.stencil;
-    q.value = swap ? x0.value : x1.value;
-    q.delta = swap ? x0.delta : x1.delta;
-    const double v1 = (double)vv;
-    float res;
-    if (q.value < (double)kFar) {
-        if (upd_solve(2, p, q, v1, res) || upd_solve(1, p, q, v1, res)) return res;
-    } else if (p.value < (double)kFar) {
-        if (upd_solve(1, p, q, v1, res)) return res;
-    }
+    double s0, s1;
+    float v0, v1;
+    const bool o0 = upd_axis(zm, zp, zm2, zp2, order, s0, v0), o1 = upd_axis(xm, xp, xm2, xp2, order, s1, v1);
+    const double d0 = o0 ? __dmul_rn((double)rdx0, 2.25) : (double)rdx0;
+    const double d1 = o1 ? __dmul_rn((double)rdx1, 2.25) : (double)rdx1;
+    const double b0 = __dmul_rn(s0, d0), b1 = __dmul_rn(s1, d1);
+    const double c0 = __dmul_rn(__dmul_rn(s0, s0), d0), c1 = __dmul_rn(__dmul_rn(s1, s1), d1);
+    // the marching code sorts the axes by value: the first keeps its place
+    // unless the second is smaller
+    const bool swap = !(v0 <= v1);
+    const float lo = swap ? v1 : v0, hi = swap ? v0 : v1;
+    const double w = (double)vv;
+    float t;
+    if (upd_root(__dadd_rn(d0, d1), __dadd_rn(b0, b1), __dadd_rn(c0, c1),
+                 o0 ? (o1 ? rc.two[1][1] : rc.two[1][0]) : (o1 ? rc.two[0][1] : rc.two[0][0]), w, hi, t) &&
+        hi < kFar)
+        return t;
+    if (upd_root(swap ? d1 : d0, swap ? b1 : b0, swap ? c1 : c0,
+                 swap ? (o1 ? rc.one[1][1] : rc.one[1][0]) : (o0 ? rc.one[0][1] : rc.one[0][0]), w, lo, t) &&
+        lo < kFar)
+        return t;
     return kFar;
 }
 
@@ -190,254 +224,390 @@ __global__ void k_dw(const float *__restrict__ vv, double *__restrict__ dw, int 
     dw[i0] = w;
 }
 
-// Sweeps of one source per CTA.  MODE 0: traveltime; MODE 1: the source
-// derivative recursion on the final traveltime.  S: ring slots (a power of
-// two), D: prefetch distance in diagonals (S >= D + 3), ROWS: rows per thread
-// (blockDim * ROWS >= nz); a thread's rows of one step are independent and
-// their branch-free updates interleave.
-template <int MODE, int S, int D, int ROWS>
-__global__ void __launch_bounds__(ROWS == 1 ? 1024 : 512) k_eik_sweep(EikArgs a)
+// a plain [nx][nz] array into both layouts, `border` outside the grid
+template <class V>
+__global__ void k_skew(const V *__restrict__ in, V *__restrict__ out, int nz, int nx, int np, int nd, V border)
 {
-    static_assert((S & (S - 1)) == 0 && S >= D + 3 && D >= 3, "ring too small");
-    extern __shared__ __align__(16) unsigned char eik_smem[];
-    const int nz = a.nz, nx = a.nx, NR = nz + 4;  // ring rows -2 .. nz+1
-    float *RT = reinterpret_cast<float *>(eik_smem);            // [S][NR] traveltime
-    unsigned *RS = reinterpret_cast<unsigned *>(RT + S * NR);   // [S][NR] change stamps
-    float *RL = reinterpret_cast<float *>(RS + S * NR);         // [S][NR] tdl1 (MODE 1)
-    double *RW = reinterpret_cast<double *>(RL + S * NR);       // [S][NR] dw (MODE 1); offset 12*S*NR bytes
-    const int js = blockIdx.x;
-    const size_t nzx = (size_t)nz * nx;
-    float *T = a.T + (size_t)js * nzx;
-    float *DL = MODE == 1 ? a.dl1 + (size_t)js * nzx : nullptr;
-    float *DS = MODE == 1 ? a.ds1 + (size_t)js * nzx : nullptr;
-    unsigned *ST = a.stamp + (size_t)js * nzx;
-    const EikSource sc = a.src[js];
-    const int nthr = blockDim.x, tid = threadIdx.x;
+    const int iz = blockIdx.y * blockDim.x + threadIdx.x, p = (int)blockIdx.x - kEikBorder, fam = blockIdx.z;
+    if (iz >= np) return;
+    const int ix = fam == 0 ? p - iz : iz + nx - 1 - p;
+    out[((size_t)fam * (nd + 2 * kEikBorder)) * np + skew_row(p, np) + iz] =
+        iz < nz && ix >= 0 && ix < nx ? in[(size_t)ix * nz + iz] : border;
+}
 
-    // pad rows stay constant for the whole kernel
-    for (int q = tid; q < S * 4; q += nthr) {
-        const int slot = q >> 2, pr = q & 3, row = pr < 2 ? pr : nz + pr;
-        RT[slot * NR + row] = kFar;
-        RS[slot * NR + row] = 0u;
-        if (MODE == 1) {
-            RL[slot * NR + row] = 0.0f;
-            RW[slot * NR + row] = 0.0;
-        }
-    }
-    if (MODE == 0) {
-        // initial state: nothing reached, the box at straight-ray times
-        // (neighbors.cpp:418-484)
-        for (size_t i = tid; i < nzx; i += nthr) T[i] = kFar;
-        __syncthreads();
-        const double v1 = (double)a.vv[sc.ic];
-        const int bz = sc.en0 - sc.st0 + 1, nb = bz * (sc.en1 - sc.st1 + 1);
-        for (int q = tid; q < nb; q += nthr) {
-            const int iz = sc.st0 + q % bz, iy = sc.st1 + q / bz;
-            const double e0 = (double)__fsub_rn(sc.xs0, __fmul_rn((float)iz, a.d0));
-            const double e1 = (double)__fsub_rn(sc.xs1, __fmul_rn((float)iy, a.d1));
-            const double e2 = (double)__fsub_rn(sc.xs2, __fmul_rn(0.0f, a.d2));
-            double d2 = __dadd_rn(0.0, __dmul_rn(e0, e0));
-            d2 = __dadd_rn(d2, __dmul_rn(e1, e1));
-            d2 = __dadd_rn(d2, __dmul_rn(e2, e2));
-            T[(size_t)iy * nz + iz] = __fsqrt_rn(__double2float_rn(__dmul_rn(v1, d2)));
-        }
-    }
-    __syncthreads();
+constexpr int kEikS = 8, kEikD = 5;  // ring slots (a power of two), prefetch distance: kEikS >= kEikD + 3
+static_assert((kEikS & (kEikS - 1)) == 0 && kEikS >= kEikD + 3 && kEikD >= 3, "ring too small");
+static_assert(kEikBorder >= kEikD + 1, "the last steps fetch border rows");
+constexpr int kEikPad = 2;           // rows -2, -1 in front of a ring row (16 bytes of pairs)
 
-    const int ndiag = nz + nx - 1;
-    int quiet = 0, nsweep = 0;
-    for (int sweep = 0; sweep < 4 * a.max_iter; sweep++) {
-        const int dir = sweep & 3;
-        const bool fz = (dir & 1) == 0, fx = (dir & 2) == 0;
-        const int sz = fz ? 1 : -1, sx = fx ? 1 : -1;
-        // diagonal kk of this sweep into its ring slot (async where inside the grid)
-        auto fetch = [&](int kk) {
-            const int slot = kk & (S - 1);
-#pragma unroll
-            for (int qr = 0; qr < ROWS; qr++) {
-                const int r = tid + qr * nthr;
-                if (r >= nz) continue;
-                const int c = kk - r;
-                const int ri = slot * NR + r + 2;
-                if (c >= 0 && c < nx) {
-                    const size_t i = (size_t)(fx ? c : nx - 1 - c) * nz + (fz ? r : nz - 1 - r);
-                    cp_async4(RT + ri, T + i);
-                    cp_async4(RS + ri, ST + i);
-                    if (MODE == 1) {
-                        cp_async4(RL + ri, DL + i);
-                        cp_async8(RW + ri, a.dw + i);
-                    }
-                } else {
-                    RT[ri] = kFar;
-                    RS[ri] = 0u;
-                    if (MODE == 1) {
-                        RL[ri] = 0.0f;
-                        RW[ri] = 0.0;
-                    }
-                }
+// bytes of one CTA's working values: {value, stamp} pairs in both layouts,
+// and with derivatives the final time in both
+inline size_t eik_slot_bytes(int nd, int np, bool deriv)
+{
+    return 2 * (size_t)(nd + 2 * kEikBorder) * np * (deriv ? 12 : 8);
+}
+// shared memory: the pair ring, the time ring (derivative pass; its border
+// pads four floats), the blocks' last changes
+inline size_t eik_smem(int np, int nblk, bool deriv)
+{
+    const size_t rings = (size_t)kEikS * ((np + kEikPad) * 8 + (deriv ? (np + 4) * 4 : 0)) + 2 * (size_t)nblk * 4;
+    return std::max(rings, (size_t)32 * 33 * 4);  // at least one window of eik_unskew
+}
+
+// What a sweep works on: one source's pairs ({value, stamp}: the time or tdl1,
+// and 1 + the sweep of its last change, 0: none) and final times in both
+// layouts, the rings, the blocks' last changes.
+struct EikMem {
+    uint2 *W;
+    const float *TT;
+    uint2 *RP;
+    float *RT;
+    unsigned *last;
+};
+
+// One sweep along the diagonals of family FAM, ST = +1 or -1 its direction.
+// MODE 0: traveltime; MODE 1: the source derivative recursion on the final
+// traveltime.  Every address advances by a constant per step and the ring
+// slots rotate through registers: the loop is bound by instructions (a point
+// takes 2.9 evaluations a pass on the salt model, 30 of 32 lanes busy) and by
+// the serial chain of one step.  One CTA of 19 warps without spills per SM is
+// as fast for 400 sources as two at 48 registers (66 ms against 78) and faster
+// for 148 (28 against 38), with half the working memory.
+template <int MODE, int ROWS, int FAM, int ST>
+__device__ __forceinline__ bool eik_sweep(const EikArgs &a, const EikSource &sc, const EikMem &m, int sweep)
+{
+    const int nz = a.nz, nx = a.nx, np = a.np, nd = a.nd, nthr = blockDim.x, tid = threadIdx.x;
+    const int NR = np + kEikPad, NT = np + 4;
+    const size_t fam_len = (size_t)(nd + 2 * kEikBorder) * np;
+    uint2 *Wf = m.W + FAM * fam_len, *Wo = m.W + (1 - FAM) * fam_len;
+    const unsigned *lastf = m.last + FAM * a.nblk;
+    const uint32_t rp = (uint32_t)__cvta_generic_to_shared(m.RP + kEikPad), rt = (uint32_t)__cvta_generic_to_shared(m.RT + 4);
+    const bool f_on = tid < np / 2, g_on = MODE == 1 && tid < np / 4;  // blockDim >= np / 2 (the launcher)
+    bool changed = false, piped = false;
+    for (int bi = 0; bi < a.nblk; bi++) {
+        const int blk = ST > 0 ? bi : a.nblk - 1 - bi;
+        // a change of this sweep or the one before, here or next door
+        // (blocks are at least as long as the stencil's reach)
+        bool need = sweep == 0 || lastf[blk] >= (unsigned)sweep;
+        if (!need && blk > 0) need = lastf[blk - 1] >= (unsigned)sweep;
+        if (!need && blk + 1 < a.nblk) need = lastf[blk + 1] >= (unsigned)sweep;
+        if (!need) {
+            piped = false;
+            continue;
+        }
+        const int b0 = blk << a.blk_shift, b1 = min(nd, b0 + (1 << a.blk_shift));
+        const int p0 = ST > 0 ? b0 : b1 - 1, n = b1 - b0;
+        // diagonal p sits in ring slot p mod kEikS; its rows are fetched kEikD steps ahead
+        const uint2 *src = Wf + skew_row(p0 + ST * kEikD, np) + 2 * tid;
+        const float *srcT = MODE == 1 ? m.TT + FAM * fam_len + skew_row(p0 + ST * kEikD, np) + 4 * tid : nullptr;
+        if (!piped) {  // fill the ring
+            cp_wait<0>();
+            __syncthreads();
+            for (int q = -2; q < kEikD; q++) {
+                const int p = p0 + ST * q, slot = p & (kEikS - 1);
+                if (f_on) cp_async16(rp + (slot * NR + 2 * tid) * 8, Wf + skew_row(p, np) + 2 * tid);
+                if (g_on) cp_async16(rt + (slot * NT + 4 * tid) * 4, m.TT + FAM * fam_len + skew_row(p, np) + 4 * tid);
             }
-        };
-        for (int r = tid; r < nz; r += nthr) {  // diagonals -2 and -1
-            RT[(S - 2) * NR + r + 2] = kFar;
-            RT[(S - 1) * NR + r + 2] = kFar;
-            RS[(S - 2) * NR + r + 2] = 0u;
-            RS[(S - 1) * NR + r + 2] = 0u;
+            cp_commit();
+            cp_wait<0>();
+            __syncthreads();
+            piped = true;
+        }
+        // slots of p + ST d, d = -2 .. 2, as byte offsets of a row's first pair
+        uint32_t o[5];
+#pragma unroll
+        for (int d = 0; d < 5; d++) o[d] = (uint32_t)((p0 + ST * (d - 2)) & (kEikS - 1)) * (uint32_t)NR * 8u;
+        uint32_t oD = (uint32_t)((p0 + ST * kEikD) & (kEikS - 1));  // slot being fetched
+        const float *vp = a.vv + FAM * fam_len + skew_row(p0, np) + tid;
+        const double *wp = MODE == 1 ? a.dw + FAM * fam_len + skew_row(p0, np) + tid : nullptr;
+        float v_nxt[ROWS];  // the model's values one step ahead
+        double w_nxt[ROWS];
+#pragma unroll
+        for (int qr = 0; qr < ROWS; qr++) {
+            const bool in = tid + qr * nthr < np;
+            if (MODE == 0) v_nxt[qr] = in ? __ldg(vp + qr * nthr) : 0.0f;
+            else w_nxt[qr] = in ? __ldg(wp + qr * nthr) : 0.0;
+        }
+        int p = p0;
+        for (int k = 0; k < n; k++, p += ST) {
+            if (f_on) cp_async16(rp + oD * (uint32_t)NR * 8u + tid * 16, src);
+            src += ST * np;
             if (MODE == 1) {
-                RL[(S - 2) * NR + r + 2] = 0.0f;
-                RL[(S - 1) * NR + r + 2] = 0.0f;
+                if (g_on) cp_async16(rt + oD * (uint32_t)NT * 4u + tid * 16, srcT);
+                srcT += ST * np;
             }
-        }
-        for (int kk = 0; kk < D; kk++) {
-            fetch(kk);
+            oD = (oD + (uint32_t)ST) & (kEikS - 1);
             cp_commit();
-        }
-        cp_wait<D - 3>();
-        __syncthreads();
-        bool changed = false;
-        for (int k = 0; k < ndiag; k++) {
-            fetch(k + D);
-            cp_commit();
-            const int s0 = k & (S - 1);
+            float v_cur[ROWS];
+            double w_cur[ROWS];
+            if (MODE == 0) vp += ST * np;
+            else wp += ST * np;
 #pragma unroll
             for (int qr = 0; qr < ROWS; qr++) {
-                const int r0 = tid + qr * nthr, c0 = k - r0;
-                const bool act = r0 < nz && c0 >= 0 && c0 < nx;
-                // inactive rows compute on a valid point and store nothing
-                const int r = act ? r0 : 0, c = act ? c0 : 0;
-                const int iz = fz ? r : nz - 1 - r, ix = fx ? c : nx - 1 - c;
-                const size_t i = (size_t)ix * nz + iz;
-                const int R = r + 2;
-                // physical neighbours: z -/+ one and two samples, x -/+ one and two
-                const float t0 = RT[s0 * NR + R];
-                const float zm = RT[((k - sz) & (S - 1)) * NR + R - sz];
-                const float zp = RT[((k + sz) & (S - 1)) * NR + R + sz];
-                const float zm2 = RT[((k - 2 * sz) & (S - 1)) * NR + R - 2 * sz];
-                const float zp2 = RT[((k + 2 * sz) & (S - 1)) * NR + R + 2 * sz];
-                const float xm = RT[((k - sx) & (S - 1)) * NR + R];
-                const float xp = RT[((k + sx) & (S - 1)) * NR + R];
-                const float xm2 = RT[((k - 2 * sx) & (S - 1)) * NR + R];
-                const float xp2 = RT[((k + 2 * sx) & (S - 1)) * NR + R];
-                // A point whose inputs did not change since its evaluation in
-                // the previous sweep would come out the same: it is skipped.
-                // Its inputs are the neighbours one step away (both passes)
-                // and two steps away (traveltime pass); stamps >= sweep mark
-                // a change in the previous sweep or earlier in this one.
-                const unsigned szm = RS[((k - sz) & (S - 1)) * NR + R - sz];
-                const unsigned szp = RS[((k + sz) & (S - 1)) * NR + R + sz];
-                const unsigned sxm = RS[((k - sx) & (S - 1)) * NR + R];
-                const unsigned sxp = RS[((k + sx) & (S - 1)) * NR + R];
-                unsigned snew = max(max(szm, szp), max(sxm, sxp));
+                const bool in = tid + qr * nthr < np;
                 if (MODE == 0) {
-                    const unsigned szm2 = RS[((k - 2 * sz) & (S - 1)) * NR + R - 2 * sz];
-                    const unsigned szp2 = RS[((k + 2 * sz) & (S - 1)) * NR + R + 2 * sz];
-                    const unsigned sxm2 = RS[((k - 2 * sx) & (S - 1)) * NR + R];
-                    const unsigned sxp2 = RS[((k + 2 * sx) & (S - 1)) * NR + R];
-                    snew = max(snew, max(max(szm2, szp2), max(sxm2, sxp2)));
+                    v_cur[qr] = v_nxt[qr];
+                    if (in) v_nxt[qr] = __ldg(vp + qr * nthr);
+                } else {
+                    w_cur[qr] = w_nxt[qr];
+                    if (in) w_nxt[qr] = __ldg(wp + qr * nthr);
                 }
-                const bool need = act && (sweep == 0 || snew >= (unsigned)sweep);
-                if (!need) continue;
+            }
+            // physical diagonals p - 2 .. p + 2, and the two an x step leads to
+            const uint32_t m2 = ST > 0 ? o[0] : o[4], m1 = ST > 0 ? o[1] : o[3];
+            const uint32_t p1 = ST > 0 ? o[3] : o[1], p2 = ST > 0 ? o[4] : o[0];
+#pragma unroll
+            for (int qr = 0; qr < ROWS; qr++) {
+                const int iz = tid + qr * nthr, ix = FAM ? iz + nx - 1 - p : p - iz;
+                if (iz >= nz || (unsigned)ix >= (unsigned)nx) continue;
+                const uint32_t r = rp + iz * 8;
+                const uint2 zm = lds64(r + m1 - 8), zp = lds64(r + p1 + 8);
+                const uint2 xm = lds64(r + (FAM ? p1 : m1)), xp = lds64(r + (FAM ? m1 : p1));
+                unsigned snew = max(max(zm.y, zp.y), max(xm.y, xp.y));
+                float nv;
                 if (MODE == 0) {
+                    const uint2 zm2 = lds64(r + m2 - 16), zp2 = lds64(r + p2 + 16);
+                    const uint2 xm2 = lds64(r + (FAM ? p2 : m2)), xp2 = lds64(r + (FAM ? m2 : p2));
+                    snew = max(snew, max(max(zm2.y, zp2.y), max(xm2.y, xp2.y)));
+                    // inputs as at its previous evaluation: it would come out the same
+                    if (sweep > 0 && snew < (unsigned)sweep) continue;
                     const bool in_box = iz >= sc.st0 && iz <= sc.en0 && ix >= sc.st1 && ix <= sc.en1;
                     if (in_box) continue;
-                    const float q = qsolve2d(zm, zp, zm2, zp2, xm, xp, xm2, xp2, a.vv[i], a.rdx0, a.rdx1, a.order);
-                    if (q < t0) {
-                        RT[s0 * NR + R] = q;
-                        T[i] = q;
-                        RS[s0 * NR + R] = (unsigned)sweep + 1u;
-                        ST[i] = (unsigned)sweep + 1u;
-                        changed = true;
-                    }
+                    nv = qsolve2d(__uint_as_float(zm.x), __uint_as_float(zp.x), __uint_as_float(zm2.x),
+                                  __uint_as_float(zp2.x), __uint_as_float(xm.x), __uint_as_float(xp.x),
+                                  __uint_as_float(xm2.x), __uint_as_float(xp2.x), v_cur[qr], a.rdx0, a.rdx1, a.order, a.rc);
+                    if (!(nv < __uint_as_float(lds64(r + o[2]).x))) continue;
                 } else {
-                    // eikods.cpp:149-211 (eikods_dt1) for point i, branch-free
-                    const float lzm = RL[((k - sz) & (S - 1)) * NR + R - sz];
-                    const float lzp = RL[((k + sz) & (S - 1)) * NR + R + sz];
-                    const float lxm = RL[((k - sx) & (S - 1)) * NR + R];
-                    const float lxp = RL[((k + sx) & (S - 1)) * NR + R];
-                    double rhs = 0.0, den = 0.0, dt = 0.0;
+                    if (sweep > 0 && snew < (unsigned)sweep) continue;
+                    // eikods.cpp:149-211 (eikods_dt1) for one point, branch-free; tds1 follows from the
+                    // final tdl1 (k_tds1)
+                    const uint32_t q = (uint32_t)NT * 4u, t = rt + iz * 4;
+                    const uint32_t tm = ((p - 1) & (kEikS - 1)) * q, tp = ((p + 1) & (kEikS - 1)) * q;
+                    const float t0 = lds32(t + (p & (kEikS - 1)) * q);
+                    double rhs = 0.0, den = 0.0;
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
-                        const int ii = j == 0 ? iz : ix, n = j == 0 ? nz : nx;
-                        const float ta = j == 0 ? zm : xm, tb = j == 0 ? zp : xp;
-                        const float ta2 = j == 0 ? zm2 : xm2, tb2 = j == 0 ? zp2 : xp2;
-                        const float la = j == 0 ? lzm : lxm, lb = j == 0 ? lzp : lxp;
-                        const float dj = j == 0 ? a.d0 : a.d1;
-                        const bool use_b = ii == 0 || (ii != n - 1 && ta > tb);
+                        const int ii = j == 0 ? iz : ix, len = j == 0 ? nz : nx;
+                        const float ta = lds32(j == 0 ? t + tm - 4 : t + (FAM ? tp : tm));
+                        const float tb = lds32(j == 0 ? t + tp + 4 : t + (FAM ? tm : tp));
+                        const float la = __uint_as_float(j == 0 ? zm.x : xm.x);
+                        const float lb = __uint_as_float(j == 0 ? zp.x : xp.x);
+                        const bool use_b = ii == 0 || (ii != len - 1 && ta > tb);
                         const float t1 = use_b ? tb : ta, l1 = use_b ? lb : la;
                         const bool up = t1 < t0;
-                        const float dd = __fmul_rn(dj, dj);
-                        const float e = __fsub_rn(t0, t1);
-                        const double term = (double)__fdiv_rn(__fmul_rn(e, l1), dd);
-                        const double dterm = (double)__fdiv_rn(e, dd);
+                        const float dd = j == 0 ? a.dd0 : a.dd1, yd = j == 0 ? a.yd0 : a.yd1;
+                        const float e = up ? __fsub_rn(t0, t1) : 0.0f;
+                        const double term = (double)div_by(__fmul_rn(e, l1), dd, yd);
+                        const double dterm = (double)div_by(e, dd, yd);
                         rhs = up ? __dadd_rn(rhs, term) : rhs;
                         den = up ? __dadd_rn(den, dterm) : den;
-                        if (a.l == j) {
-                            const float t2 = use_b ? tb2 : ta2;
-                            const bool three = use_b ? (ii < n - 2 && t1 > tb2) : (ii > 1 && t1 > ta2);
-                            const double num3 =
-                                use_b ? __dsub_rn(__dadd_rn(-(double)t2, __dmul_rn(4.0, (double)t1)),
-                                                  __dmul_rn(3.0, (double)t0))
-                                      : __dadd_rn(__dsub_rn(__dmul_rn(3.0, (double)t0), __dmul_rn(4.0, (double)t1)),
-                                                  (double)t2);
-                            const double d3 = __ddiv_rn(num3, __dmul_rn(2.0, (double)dj));
-                            const double d2p = (double)__fdiv_rn(use_b ? __fsub_rn(t1, t0) : __fsub_rn(t0, t1), dj);
-                            dt = up ? (three ? d3 : d2p) : dt;
-                        }
                     }
-                    const double w = RW[s0 * NR + R];
-                    const bool has = den != 0.0;
-                    const float nl0 = __double2float_rn(__ddiv_rn(__dadd_rn(__dmul_rn(0.5, w), rhs), den));
-                    const float nl = has ? nl0 : 0.0f;
-                    const float ns = has ? __double2float_rn(__dsub_rn((double)nl0, dt)) : 0.0f;
-                    // tds1 follows tdl1 (dt is fixed by the final time), so
-                    // after the first visit only a change of tdl1 is news
-                    const float ol = RL[s0 * NR + R];
-                    if (sweep == 0 || nl != ol) {
-                        RL[s0 * NR + R] = nl;
-                        DL[i] = nl;
-                        DS[i] = ns;
-                    }
-                    if (nl != ol) {
-                        RS[s0 * NR + R] = (unsigned)sweep + 1u;
-                        ST[i] = (unsigned)sweep + 1u;
-                        changed = true;
-                    }
+                    nv = den != 0.0 ? __double2float_rn(__ddiv_rn(__dadd_rn(__dmul_rn(0.5, w_cur[qr]), rhs), den)) : 0.0f;
+                    if (!(nv != __uint_as_float(lds64(r + o[2]).x))) continue;
                 }
+                const uint2 e = make_uint2(__float_as_uint(nv), (unsigned)sweep + 1u);
+                const int op = FAM ? iz + ix : iz - ix + nx - 1;
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(r + o[2]), "r"(e.x), "r"(e.y) : "memory");
+                Wf[skew_row(p, np) + iz] = e;
+                Wo[skew_row(op, np) + iz] = e;
+                m.last[FAM * a.nblk + blk] = e.y;
+                m.last[(1 - FAM) * a.nblk + (op >> a.blk_shift)] = e.y;
+                changed = true;
             }
-            cp_wait<D - 3>();
+            const uint32_t nxt = (uint32_t)((p + 3 * ST) & (kEikS - 1)) * (uint32_t)NR * 8u;
+            o[0] = o[1];
+            o[1] = o[2];
+            o[2] = o[3];
+            o[3] = o[4];
+            o[4] = nxt;
+            cp_wait<kEikD - 3>();
             __syncthreads();
         }
-        cp_wait<0>();
-        const bool any = __syncthreads_or(changed);
+    }
+    cp_wait<0>();
+    return __syncthreads_or(changed) != 0;
+}
+
+// One pass over one source: sweeps in the four orderings (z+ x+), (z- x+),
+// (z+ x-), (z- x-) until each has changed nothing.  Returns the sweeps it
+// took, 0 without a fixed point.
+template <int MODE, int ROWS>
+__device__ __forceinline__ int eik_pass(const EikArgs &a, const EikSource &sc, const EikMem &m)
+{
+    const int nthr = blockDim.x, tid = threadIdx.x;
+    const unsigned border = MODE == 0 ? __float_as_uint(kFar) : 0u;
+    for (int q = tid; q < kEikS * kEikPad; q += nthr)
+        m.RP[(q / kEikPad) * (a.np + kEikPad) + q % kEikPad] = make_uint2(border, 0u);
+    if (MODE == 1)
+        for (int q = tid; q < kEikS * 4; q += nthr) m.RT[(q >> 2) * (a.np + 4) + (q & 3)] = kFar;
+    for (int q = tid; q < 2 * a.nblk; q += nthr) m.last[q] = 0u;
+    __syncthreads();
+    int quiet = 0;
+    for (int sweep = 0; sweep < 4 * a.max_iter; sweep++) {
+        bool any;
+        switch (sweep & 3) {
+        case 0: any = eik_sweep<MODE, ROWS, 0, 1>(a, sc, m, sweep); break;
+        case 1: any = eik_sweep<MODE, ROWS, 1, -1>(a, sc, m, sweep); break;
+        case 2: any = eik_sweep<MODE, ROWS, 1, 1>(a, sc, m, sweep); break;
+        default: any = eik_sweep<MODE, ROWS, 0, -1>(a, sc, m, sweep); break;
+        }
         quiet = any ? 0 : quiet + 1;
         // four quiet sweeps in a row (one of each ordering): a fixed point
-        if (quiet >= 4) {
-            nsweep = sweep + 1;
-            break;
-        }
+        if (quiet >= 4) return sweep + 1;
     }
-    if (tid == 0) {
-        if (nsweep == 0) atomicExch(a.status, 1);
-        if (MODE == 0) a.iters[js] = nsweep;
+    return 0;
+}
+
+// The values of a layout-0 pair array into the plain [nx][nz] order: a warp
+// takes 32 rows and walks the diagonals, a window of 32 of them in shared
+// memory (33 floats a row); column ix of the rows is complete once diagonal
+// ix + r0 + 31 has been read.  Reads and writes are whole 32-row segments.
+__device__ __forceinline__ void eik_unskew(const uint2 *W, float *out, int nz, int nx, int np, int nd, float *sh,
+                                           int warps)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp >= warps) return;
+    float *win = sh + warp * 32 * 33;
+    for (int r0 = warp * 32; r0 < nz; r0 += warps * 32) {
+        const int row = min(r0 + lane, np - 1);
+        const int d1 = r0 + 31 + nx;  // one past the last diagonal read
+        constexpr int U = 16;  // diagonals in flight
+        for (int d = r0; d < d1; d += U) {
+            float v[U];
+#pragma unroll
+            for (int q = 0; q < U; q++)
+                v[q] = __uint_as_float(__ldcg(&W[skew_row(min(d + q, nd + kEikBorder - 1), np) + row].x));
+#pragma unroll
+            for (int q = 0; q < U; q++) {
+                if (d + q >= d1) break;
+                win[((d + q) & 31) * 33 + lane] = v[q];
+                __syncwarp();
+                const int ix = d + q - r0 - 31;
+                if (ix >= 0 && r0 + lane < nz) out[(size_t)ix * nz + r0 + lane] = win[((ix + r0 + lane) & 31) * 33 + lane];
+                __syncwarp();
+            }
+        }
     }
 }
 
-// launch of one pass: one row per thread up to 1024 rows, else four
-template <int MODE, int S, int D>
-int launch_sweep(const EikArgs &a, int nshot, cudaStream_t st)
+// Sources one after another per CTA: the time pass, its result to the plain
+// layout, then (DERIV) the derivative pass in the same working memory.  RPT:
+// rows per thread; MAXT: the block sizes it is compiled for.
+template <int RPT, int MAXT, bool DERIV>
+__global__ void __launch_bounds__(MAXT) k_eik_solve(const EikArgs a)
 {
-    const int nz = a.nz, rows = nz <= 1024 ? 1 : 4;
-    const size_t smem =
-        (size_t)S * (nz + 4) * (MODE == 0 ? 2 * sizeof(float) : 3 * sizeof(float) + sizeof(double));
-    const int threads = (((nz + rows - 1) / rows + 31) / 32) * 32;
-    if (rows == 1) {
-        KCIG_TRY(set_dyn_smem((const void *)k_eik_sweep<MODE, S, D, 1>, (int)smem));
-        k_eik_sweep<MODE, S, D, 1><<<nshot, threads, smem, st>>>(a);
-    } else {
-        KCIG_TRY(set_dyn_smem((const void *)k_eik_sweep<MODE, S, D, 4>, (int)smem));
-        k_eik_sweep<MODE, S, D, 4><<<nshot, threads, smem, st>>>(a);
+    extern __shared__ __align__(16) unsigned char eik_smem_raw[];
+    __shared__ int cur;
+    const int nz = a.nz, nx = a.nx, np = a.np, nd = a.nd, nthr = blockDim.x, tid = threadIdx.x;
+    uint2 *RP = reinterpret_cast<uint2 *>(eik_smem_raw);                       // [kEikS][np + kEikPad]
+    float *RT = reinterpret_cast<float *>(RP + kEikS * (np + kEikPad));        // [kEikS][np + 4] (DERIV)
+    unsigned *last = reinterpret_cast<unsigned *>(RT + (DERIV ? kEikS * (np + 4) : 0));
+    const size_t fam_len = (size_t)(nd + 2 * kEikBorder) * np;
+    uint2 *W = reinterpret_cast<uint2 *>(a.work + (size_t)blockIdx.x * a.slot_bytes);
+    float *TT = reinterpret_cast<float *>(W + 2 * fam_len);
+    const int uwarps = max(1, min(nthr / 32, (int)((unsigned)(kEikS * (np + kEikPad) * 8) / (32 * 33 * 4))));
+    for (;;) {
+        if (tid == 0) cur = atomicAdd(a.next, 1);
+        __syncthreads();
+        const int js = cur;
+        __syncthreads();
+        if (js >= a.nsrc) return;
+        const EikSource sc = a.src[js];
+        const size_t nzx = (size_t)nz * nx;
+        // initial state: nothing reached, the box at straight-ray times
+        // (neighbors.cpp:418-484)
+        const unsigned far = __float_as_uint(kFar);
+        for (size_t i = tid; i < fam_len; i += nthr) reinterpret_cast<uint4 *>(W)[i] = make_uint4(far, 0u, far, 0u);
+        __syncthreads();
+        {
+            const double v1 = (double)a.vplain[sc.ic];
+            const int bz = sc.en0 - sc.st0 + 1, nb = bz * (sc.en1 - sc.st1 + 1);
+            for (int q = tid; q < nb; q += nthr) {
+                const int iz = sc.st0 + q % bz, iy = sc.st1 + q / bz;
+                const double e0 = (double)__fsub_rn(sc.xs0, __fmul_rn((float)iz, a.d0));
+                const double e1 = (double)__fsub_rn(sc.xs1, __fmul_rn((float)iy, a.d1));
+                const double e2 = (double)__fsub_rn(sc.xs2, __fmul_rn(0.0f, a.d2));
+                double d2 = __dadd_rn(0.0, __dmul_rn(e0, e0));
+                d2 = __dadd_rn(d2, __dmul_rn(e1, e1));
+                d2 = __dadd_rn(d2, __dmul_rn(e2, e2));
+                const uint2 e = make_uint2(__float_as_uint(__fsqrt_rn(__double2float_rn(__dmul_rn(v1, d2)))), 0u);
+                W[skew_row(iz + iy, np) + iz] = e;
+                W[fam_len + skew_row(iz - iy + nx - 1, np) + iz] = e;
+            }
+        }
+        __syncthreads();
+        const EikMem mem = {W, TT, RP, RT, last};
+        const int n = eik_pass<0, RPT>(a, sc, mem);
+        if (tid == 0) {
+            a.iters[js] = n;
+            if (n == 0) atomicExch(a.status, 1);
+        }
+        __syncthreads();
+        eik_unskew(W, a.T + (size_t)js * nzx, nz, nx, np, nd, reinterpret_cast<float *>(RP), uwarps);
+        __syncthreads();
+        if (DERIV) {
+            // two pairs a thread, eight loads in flight (fam_len is a multiple of 16)
+            uint4 *W4 = reinterpret_cast<uint4 *>(W);
+            uint2 *T2 = reinterpret_cast<uint2 *>(TT);
+            for (size_t i = tid; i < fam_len; i += 8 * (size_t)nthr) {
+                uint4 v[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (i + q * (size_t)nthr < fam_len) v[q] = W4[i + q * (size_t)nthr];
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (i + q * (size_t)nthr < fam_len) {
+                        T2[i + q * (size_t)nthr] = make_uint2(v[q].x, v[q].z);
+                        W4[i + q * (size_t)nthr] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+            }
+            __syncthreads();
+            if (eik_pass<1, RPT>(a, sc, mem) == 0 && tid == 0) atomicExch(a.status, 1);
+            __syncthreads();
+            eik_unskew(W, a.dl1 + (size_t)js * nzx, nz, nx, np, nd, reinterpret_cast<float *>(RP), uwarps);
+            __syncthreads();
+        }
     }
-    KCIG_CUDA(cudaGetLastError());
-    return KCIG_OK;
+}
+
+// tds1 from the final time and tdl1 (eikods.cpp:149-211): tdl1 minus the
+// time's derivative along axis l where the point has an upwind neighbour
+__global__ void k_tds1(const float *__restrict__ T, const float *__restrict__ dl1, float *__restrict__ ds1, int nz,
+                       int nx, int l, float d0, float d1)
+{
+    const size_t nzx = (size_t)nz * nx;
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nzx) return;
+    const float *t = T + (size_t)blockIdx.y * nzx;
+    const size_t o = (size_t)blockIdx.y * nzx + i;
+    const int iz = (int)(i % nz), ix = (int)(i / nz);
+    const float t0 = t[i];
+    double den = 0.0, dt = 0.0;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const int ii = j == 0 ? iz : ix, n = j == 0 ? nz : nx;
+        const size_t s = j == 0 ? 1 : (size_t)nz;
+        const float dj = j == 0 ? d0 : d1;
+        const float ta = ii > 0 ? t[i - s] : kFar, tb = ii < n - 1 ? t[i + s] : kFar;
+        const bool use_b = ii == 0 || (ii != n - 1 && ta > tb);
+        const float t1 = use_b ? tb : ta;
+        const bool up = t1 < t0;
+        const double dterm = (double)__fdiv_rn(__fsub_rn(t0, t1), __fmul_rn(dj, dj));
+        den = up ? __dadd_rn(den, dterm) : den;
+        if (l == j) {
+            const float ta2 = ii > 1 ? t[i - 2 * s] : kFar, tb2 = ii < n - 2 ? t[i + 2 * s] : kFar;
+            const float t2 = use_b ? tb2 : ta2;
+            const bool three = use_b ? (ii < n - 2 && t1 > tb2) : (ii > 1 && t1 > ta2);
+            const double num3 = use_b ? __dsub_rn(__dadd_rn(-(double)t2, __dmul_rn(4.0, (double)t1)),
+                                                  __dmul_rn(3.0, (double)t0))
+                                      : __dadd_rn(__dsub_rn(__dmul_rn(3.0, (double)t0), __dmul_rn(4.0, (double)t1)),
+                                                  (double)t2);
+            const double d3 = __ddiv_rn(num3, __dmul_rn(2.0, (double)dj));
+            const double d2p = (double)__fdiv_rn(use_b ? __fsub_rn(t1, t0) : __fsub_rn(t0, t1), dj);
+            dt = up ? (three ? d3 : d2p) : dt;
+        }
+    }
+    ds1[o] = den != 0.0 ? __double2float_rn(__dsub_rn((double)dl1[o], dt)) : 0.0f;
 }
 
 // branch-aware spatial gradient along one axis (eikods2d.cpp:30-68)
@@ -515,7 +685,47 @@ struct DevBuf {
     }
 };
 
+// The calls' device memory comes from a stream-ordered pool of the library,
+// one per device, that keeps up to a sixteenth of the device between calls
+// (mapping and unmapping memory anew cost more than the solve on small
+// grids: ~16 ms per GB); eik_release_pool gives all of it back.
+std::mutex g_pool_mu;
+std::map<int, cudaMemPool_t> g_pools;
+
+int eik_pool(cudaMemPool_t *out)
+{
+    int dev = 0;
+    KCIG_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    auto it = g_pools.find(dev);
+    if (it == g_pools.end()) {
+        cudaMemPoolProps pr = {};
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        cudaMemPool_t pool;
+        KCIG_CUDA(cudaMemPoolCreate(&pool, &pr));
+        cudaDeviceProp dp;
+        KCIG_CUDA(cudaGetDeviceProperties(&dp, dev));
+        uint64_t keep = (uint64_t)dp.totalGlobalMem / 16;
+        KCIG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        it = g_pools.emplace(dev, pool).first;
+    }
+    *out = it->second;
+    return KCIG_OK;
+}
+
 }  // namespace
+
+int eik_release_pool()
+{
+    int dev = 0;
+    KCIG_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    auto it = g_pools.find(dev);
+    if (it != g_pools.end()) KCIG_CUDA(cudaMemPoolTrimTo(it->second, 0));
+    return KCIG_OK;
+}
 }  // namespace kcig
 
 using namespace kcig;
@@ -530,7 +740,7 @@ extern "C" int kcig_eikods(const float *vel, int nz, int nx, float o1, float o2,
     if (opt->l != 0 && opt->l != 1) return set_error(KCIG_ERR_ARG, "kcig_eikods: l must be 0 or 1");
     if ((tdl1 == nullptr) != (tds1 == nullptr))
         return set_error(KCIG_ERR_ARG, "kcig_eikods: tdl1 and tds1 go together");
-    // the rings hold 16 (time) and 8 (derivative pass) diagonals of nz + 4 rows
+    // the rings hold kEikS diagonals of nz rows, 12 bytes a row
     if (nz > 1400) return set_error(KCIG_ERR_ARG, "kcig_eikods: nz=%d above 1400", nz);
     const int max_iter = opt->max_iter > 0 ? opt->max_iter : 256;
     const int b0 = opt->b1 < 1 ? 1 : opt->b1, b1 = opt->b2 < 1 ? 1 : opt->b2;
@@ -541,48 +751,113 @@ extern "C" int kcig_eikods(const float *vel, int nz, int nx, float o1, float o2,
     for (int j = 0; j < nshot; j++)
         hs[j] = source_box(shots[3 * j], shots[3 * j + 1], shots[3 * j + 2], o1, o2, o3, d1, d2, nz, nx, b0, b1);
 
-    DevBuf bvv, bdw, bsrc, bstat, bit, bstamp;
-    bvv.st = bdw.st = bsrc.st = bstat.st = bit.st = bstamp.st = st;
-    KCIG_CUDA(cudaMallocAsync(&bvv.p, nzx * sizeof(float), st));
-    KCIG_CUDA(cudaMallocAsync(&bsrc.p, nshot * sizeof(EikSource), st));
-    KCIG_CUDA(cudaMallocAsync(&bstat.p, sizeof(int), st));
-    KCIG_CUDA(cudaMallocAsync(&bit.p, nshot * sizeof(int), st));
-    KCIG_CUDA(cudaMallocAsync(&bstamp.p, (size_t)nshot * nzx * sizeof(unsigned), st));
-    KCIG_CUDA(cudaMemsetAsync(bstamp.p, 0, (size_t)nshot * nzx * sizeof(unsigned), st));
-    if (tdl1) KCIG_CUDA(cudaMallocAsync(&bdw.p, nzx * sizeof(double), st));
+    const bool deriv = tdl1 != nullptr;
+    const int np = (nz + 2 + 15) / 16 * 16, nd = nz + nx - 1;
+    const size_t fam_len = (size_t)(nd + 2 * kEikBorder) * np;
+    // skipping blocks of 16 diagonals (more on grids that would need over 1024)
+    int blk_shift = 4;
+    while (((nd - 1) >> blk_shift) + 1 > 1024) blk_shift++;
+    const int nblk = ((nd - 1) >> blk_shift) + 1;
+    const int rows = nz <= 1024 ? 1 : 2;
+    const int threads = ((std::max((nz + rows - 1) / rows, np / 2) + 31) / 32) * 32;
+    const size_t smem = eik_smem(np, nblk, deriv), slot = (eik_slot_bytes(nd, np, deriv) + 255) / 256 * 256;
+    const void *kern =
+        threads <= 640 && rows == 1
+            ? (deriv ? (const void *)k_eik_solve<1, 640, true> : (const void *)k_eik_solve<1, 640, false>)
+            : rows == 1 ? (deriv ? (const void *)k_eik_solve<1, 1024, true> : (const void *)k_eik_solve<1, 1024, false>)
+                        : (deriv ? (const void *)k_eik_solve<2, 704, true> : (const void *)k_eik_solve<2, 704, false>);
+    KCIG_TRY(set_dyn_smem(kern, (int)smem));
+    // one CTA per source up to the resident ones, and to half of the free
+    // memory (32 MB of working values a source on 601 x 1601)
+    int per_sm = 0, sms = 0, dev = 0;
+    KCIG_CUDA(cudaGetDevice(&dev));
+    KCIG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    KCIG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    int slots = std::min(nshot, std::max(1, per_sm) * sms);
+    if (slots * slot > ((size_t)256 << 20)) {
+        size_t fr = 0, tot = 0;
+        KCIG_CUDA(cudaMemGetInfo(&fr, &tot));
+        slots = (int)std::max<size_t>(1, std::min<size_t>(slots, fr / 2 / slot));
+    }
+
+    cudaMemPool_t pool;
+    KCIG_TRY(eik_pool(&pool));
+    DevBuf bvv, bsk, bdw, bdp, bsrc, bstat, bit, bwork;
+    bvv.st = bsk.st = bdw.st = bdp.st = bsrc.st = bstat.st = bit.st = bwork.st = st;
+    KCIG_CUDA(cudaMallocFromPoolAsync(&bvv.p, nzx * sizeof(float), pool, st));
+    KCIG_CUDA(cudaMallocFromPoolAsync(&bsk.p, 2 * fam_len * sizeof(float), pool, st));
+    KCIG_CUDA(cudaMallocFromPoolAsync(&bsrc.p, nshot * sizeof(EikSource), pool, st));
+    KCIG_CUDA(cudaMallocFromPoolAsync(&bstat.p, 2 * sizeof(int), pool, st));
+    KCIG_CUDA(cudaMallocFromPoolAsync(&bit.p, nshot * sizeof(int), pool, st));
+    for (;; slots /= 2) {  // fewer sources at a time where memory is short
+        const cudaError_t e = cudaMallocFromPoolAsync(&bwork.p, slots * slot, pool, st);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation || slots == 1) return cuda_error(e, "cudaMallocFromPoolAsync(work)");
+        cudaGetLastError();
+        bwork.p = nullptr;
+    }
+    if (deriv) {
+        KCIG_CUDA(cudaMallocFromPoolAsync(&bdp.p, nzx * sizeof(double), pool, st));
+        KCIG_CUDA(cudaMallocFromPoolAsync(&bdw.p, 2 * fam_len * sizeof(double), pool, st));
+    }
     KCIG_CUDA(cudaMemcpyAsync(bsrc.p, hs.data(), nshot * sizeof(EikSource), cudaMemcpyHostToDevice, st));
-    KCIG_CUDA(cudaMemsetAsync(bstat.p, 0, sizeof(int), st));
+    KCIG_CUDA(cudaMemsetAsync(bstat.p, 0, 2 * sizeof(int), st));
 
     EikArgs a;
-    a.vv = (const float *)bvv.p;
+    a.vv = (const float *)bsk.p;
     a.dw = (const double *)bdw.p;
+    a.vplain = (const float *)bvv.p;
     a.src = (const EikSource *)bsrc.p;
     a.T = time;
     a.dl1 = tdl1;
-    a.ds1 = tds1;
+    a.work = (unsigned char *)bwork.p;
+    a.slot_bytes = slot;
     a.status = (int *)bstat.p;
+    a.next = a.status + 1;
     a.iters = (int *)bit.p;
-    a.stamp = (unsigned *)bstamp.p;
+    a.nsrc = nshot;
     a.nz = nz;
     a.nx = nx;
+    a.np = np;
+    a.nd = nd;
     a.order = opt->order;
-    a.l = opt->l;
     a.max_iter = max_iter;
+    a.blk_shift = blk_shift;
+    a.nblk = nblk;
     a.d0 = d1;
     a.d1 = d2;
     a.d2 = d3;
     a.rdx0 = (float)(1. / (d1 * d1));
     a.rdx1 = (float)(1. / (d2 * d2));
+    a.dd0 = d1 * d1;
+    a.dd1 = d2 * d2;
+    a.yd0 = 1.0f / a.dd0;
+    a.yd1 = 1.0f / a.dd1;
+    for (int i = 0; i < 2; i++) {
+        const double w0 = (double)a.rdx0 * (i ? 2.25 : 1.0);
+        a.rc.one[0][i] = 1.0 / w0;
+        a.rc.one[1][i] = 1.0 / ((double)a.rdx1 * (i ? 2.25 : 1.0));
+        for (int j = 0; j < 2; j++) a.rc.two[i][j] = 1.0 / (w0 + (double)a.rdx1 * (j ? 2.25 : 1.0));
+    }
 
     const unsigned g1 = (unsigned)((nzx + 255) / 256);
+    const dim3 gs(nd + 2 * kEikBorder, (np + 127) / 128, 2);
     k_slowness2<<<g1, 256, 0, st>>>(vel, (float *)bvv.p, nzx, opt->vel_is_slowness2);
-    KCIG_TRY((launch_sweep<0, 16, 8>(a, nshot, st)));
-    if (tdl1) {
-        k_dw<<<g1, 256, 0, st>>>((const float *)bvv.p, (double *)bdw.p, nz, nx, opt->l, opt->l == 0 ? d1 : d2);
-        KCIG_CUDA(cudaMemsetAsync(tdl1, 0, (size_t)nshot * nzx * sizeof(float), st));
-        KCIG_CUDA(cudaMemsetAsync(tds1, 0, (size_t)nshot * nzx * sizeof(float), st));
-        KCIG_CUDA(cudaMemsetAsync(bstamp.p, 0, (size_t)nshot * nzx * sizeof(unsigned), st));
-        KCIG_TRY((launch_sweep<1, 8, 5>(a, nshot, st)));
+    k_skew<float><<<gs, 128, 0, st>>>((const float *)bvv.p, (float *)bsk.p, nz, nx, np, nd, 0.0f);
+    if (deriv) {
+        k_dw<<<g1, 256, 0, st>>>((const float *)bvv.p, (double *)bdp.p, nz, nx, opt->l, opt->l == 0 ? d1 : d2);
+        k_skew<double><<<gs, 128, 0, st>>>((const double *)bdp.p, (double *)bdw.p, nz, nx, np, nd, 0.0);
+    }
+    KCIG_CUDA(cudaGetLastError());
+    void *args[] = {&a};
+    KCIG_CUDA(cudaLaunchKernel(kern, dim3(slots), dim3(threads), args, smem, st));
+    if (deriv) {
+        for (int j = 0; j < nshot; j += 65535) {
+            const size_t o = (size_t)j * nzx;
+            k_tds1<<<dim3(g1, std::min(65535, nshot - j)), 256, 0, st>>>(time + o, tdl1 + o, tds1 + o, nz, nx, opt->l, d1,
+                                                                       d2);
+            KCIG_CUDA(cudaGetLastError());
+        }
     }
     if (gradz || gradx) {
         k_upwind_grads<<<dim3(g1, nshot), 256, 0, st>>>(time, gradz, gradx, nz, nx, d1, d2);
@@ -622,8 +897,11 @@ extern "C" int kcig_eikonal_tables(const float *vel, int nz, int nx, float dz, f
     o.max_iter = iterations;
     float *dl1 = nullptr;
     if (deriv) {
-        cudaError_t e = cudaMallocAsync((void **)&dl1, (size_t)npos * nz * nx * sizeof(float), (cudaStream_t)stream);
-        if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(tdl1)");
+        cudaMemPool_t pool;
+        KCIG_TRY(eik_pool(&pool));
+        cudaError_t e = cudaMallocFromPoolAsync((void **)&dl1, (size_t)npos * nz * nx * sizeof(float), pool,
+                                                (cudaStream_t)stream);
+        if (e != cudaSuccess) return cuda_error(e, "cudaMallocFromPoolAsync(tdl1)");
     }
     const int rc = kcig_eikods(vel, nz, nx, z0, x0, dz, dx, 0.0f, 1.0f, shots.data(), npos, &o, time, dl1, deriv,
                                nullptr, nullptr, nullptr, stream);
