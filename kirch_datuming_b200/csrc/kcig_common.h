@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/kcig.h"
+#include "kcig_aperture.h"
 
 namespace kcig {
 
@@ -72,6 +73,7 @@ struct FieldArgs {
     float dz, dx, x0;
     int radius, smooth, angle, use_grad;
     float aper, aper_taper, rmin, rtaper;
+    ApertureBounds apb;  // aperture_bounds(aper, aper_taper)
     int cone;  // kirchmig2d: the w field holds the leg's two cone flags (see k_leg_interp)
     int *status;  // device flag a kernel sets when a bounded wait gives up (may be null)
     int type_p;   // the legs use the partial-shift interpolation ('p')

@@ -412,7 +412,7 @@ __global__ void k_leg_interp(FieldArgs a, LegFields out, double *work)
         const bool rcut = (double)atanf(__fdiv_rn(rnum, zi)) * 180. / M_PI > (double)a.aper;
         w = (lcut ? 0.0 : 1.0) + (rcut ? 0.0 : 2.0);
     } else {
-        w = leg_aperture_weight(L.pos, iz, ix, a.dz, a.x0, a.dx, a.aper, a.aper_taper, a.rmin, a.rtaper);
+        w = leg_aperture_weight(L.pos, iz, ix, a.dz, a.x0, a.dx, a.aper, a.aper_taper, a.rmin, a.rtaper, a.apb);
     }
     out.TP[base + i] = make_double2(T, 0.0);
     // reference: stablex[i]*ds, an FP32 product of the FP32 table derivative
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(256, 3) k_leg_tile(FieldArgs a, LegFields out)
             }
             const int iz = gz0 + lz, ix = gx0 + lx;
             const double w = leg_aperture_weight(L.pos, iz, ix, a.dz, a.x0, a.dx, a.aper, a.aper_taper, a.rmin,
-                                                 a.rtaper);
+                                                 a.rtaper, a.apb);
             TPo[(size_t)ix * nz + iz].x = T;
             out.XW[(size_t)blockIdx.y * nzx + (size_t)ix * nz + iz] = make_float2((float)Tx * L.scale, (float)w);
         }

@@ -290,6 +290,58 @@ __device__ __forceinline__ float sg_epi_back(uint32_t tG, uint32_t tZ, const flo
     return dot;
 }
 
+// The epilogues of the leg-field kernel.  Its time is the epilogues' -- 38 k
+// cycles a tile against 2 k of MMAs, two special-function operations per
+// SiLU and per SiLU' -- so the forward pass forms both from one sigmoid and
+// leaves SiLU' (KEEP) in TMEM where the pre-activation was: the backward pass
+// only multiplies (the same values as forming it again): leg fields of 265
+// legs on 201 x 401 points 23.5 -> 17 ms, with the background's FP64 beside
+// the first MMAs.  Biases come as 16-byte words (16-byte aligned).
+template <bool KEEP>
+__device__ __forceinline__ void sg_fwd_epi(uint32_t tacc, const float *bias, unsigned char *dst, int r, int c0)
+{
+    float v[32];
+    tc::tmem_ld32(tacc + c0, v);
+    float d[32];
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+        const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 4 * g);
+        const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int j = 4 * g + k;
+            const float z = v[j] + bb[k], sg = sg_sig(z);
+            v[j] = z * sg;
+            if (KEEP) d[j] = sg * (1.0f + z * (1.0f - sg));
+        }
+    }
+    if (KEEP) tc::tmem_st32(tacc + c0, d);
+#pragma unroll
+    for (int g = 0; g < 4; g++) sg_store8(dst, r, c0 + 8 * g, v + 8 * g);
+}
+
+// g = G * SiLU' as BF16 into dst (STORE), SiLU' as sg_fwd_epi left it; the
+// sum over the thread's columns of bf16(g) * vdot (vdot may be null)
+template <bool STORE>
+__device__ __forceinline__ float sg_back_epi(uint32_t tG, uint32_t tD, unsigned char *dst, int r, int c0,
+                                             const float *vdot)
+{
+    float G[32], d[32], dot = 0.0f;
+    tc::tmem_ld32(tG + c0, G);
+    tc::tmem_ld32(tD + c0, d);
+#pragma unroll
+    for (int j = 0; j < 32; j++) G[j] *= d[j];
+    if (vdot) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) dot += __bfloat162float(__float2bfloat16_rn(G[j])) * vdot[c0 + j];
+    }
+    if (STORE) {
+#pragma unroll
+        for (int g = 0; g < 4; g++) sg_store8(dst, r, c0 + 8 * g, G + 8 * g);
+    }
+    return dot;
+}
+
 // all threads' shared-memory operand writes and TMEM reads are done; the
 // tensor core may start
 __device__ __forceinline__ void sg_sync_for_mma()
@@ -323,6 +375,7 @@ struct SgFieldArgs {
     int nlegs, nz, nx;
     float z0, dz, x0, dx;
     float aper, aper_taper, rmin, rtaper;
+    ApertureBounds apb;
     LegFields out;
     int *status;
 };
@@ -344,7 +397,7 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
     unsigned char *actA = dsm + 5 * TB, *actB = dsm + 6 * TB;
     // the dynamic tiles take 224 of the 227 KB a CTA may hold; the small
     // per-leg arrays fit in the rest
-    __shared__ float b1p[H], vleg[H];
+    __shared__ __align__(16) float b1p[H], vleg[H];
     __shared__ float fx[H], dfx[H];  // per-leg xs features and their derivatives
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tslot;
@@ -427,22 +480,29 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
             tc::gemm(T1, aB, LBO_K, SBO_K, aW1x, LBO_K, SBO_K, 128, ID_KK, true);
             tc::commit(&bar);
         }
+        // beside the first MMAs: the background (FP64) by one group of warps,
+        // the aperture weight by another
+        double Tb = 0.0, bxs = 0.0, bz = 0.0, bx = 0.0;
+        float apw = 0.0f;
+        if (h == 0) sg_background<double>(n, (double)L.pos, (double)zf, (double)xf, Tb, bxs, bz, bx);
+        if (MODE != SGF_T && h == 1)
+            apw = (float)leg_aperture_weight(L.pos, iz, ix, a.dz, a.x0, a.dx, a.aper, a.aper_taper, a.rmin, a.rtaper, a.apb);
         if (!(ok = sg_wait(&bar, phase))) break;
-        sg_epi_silu(D1, b1p, actA, r, 32 * h, 1);
+        sg_fwd_epi<MODE != SGF_T>(D1, b1p, actA, r, 32 * h);
         sg_sync_for_mma();
         if (warp == 0 && tc::elect_one()) {
             tc::gemm(T2, aA, LBO_K, SBO_K, aW2, LBO_K, SBO_K, 128, ID_KK, false);
             tc::commit(&bar);
         }
         if (!(ok = sg_wait(&bar, phase))) break;
-        sg_epi_silu(D2, bias2, actB, r, 32 * h, 1);
+        sg_fwd_epi<MODE != SGF_T>(D2, bias2, actB, r, 32 * h);
         sg_sync_for_mma();
         if (warp == 0 && tc::elect_one()) {
             tc::gemm(T3, aB, LBO_K, SBO_K, aW3, LBO_K, SBO_K, 128, ID_KK, false);
             tc::commit(&bar);
         }
         if (!(ok = sg_wait(&bar, phase))) break;
-        sg_epi_silu(D3, bias3, actA, r, 32 * h, 1);
+        sg_fwd_epi<MODE != SGF_T>(D3, bias3, actA, r, 32 * h);
         sg_sync_for_mma();
         if (warp == 0 && tc::elect_one()) {
             tc::gemm(T4, aA, LBO_K, SBO_K, aW4, LBO_K, SBO_K, 128, ID_KK, false);
@@ -455,10 +515,17 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
             const int c0 = 32 * h;
             tc::tmem_ld32(D4 + c0, v);
 #pragma unroll
-            for (int jj = 0; jj < 32; jj++) {
-                const float z = v[jj] + bias4[c0 + jj];
-                part += sg_silu(z) * wo[c0 + jj];
-                v[jj] = wo[c0 + jj] * sg_dsilu(z);
+            for (int g = 0; g < 8; g++) {
+                const float4 b = *reinterpret_cast<const float4 *>(bias4 + c0 + 4 * g);
+                const float4 o = *reinterpret_cast<const float4 *>(wo + c0 + 4 * g);
+                const float bb[4] = {b.x, b.y, b.z, b.w}, oo[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int jj = 4 * g + k;
+                    const float z = v[jj] + bb[k], sg = sg_sig(z);
+                    part += z * sg * oo[k];
+                    v[jj] = oo[k] * (sg * (1.0f + z * (1.0f - sg)));
+                }
             }
             if (MODE != SGF_T) {
 #pragma unroll
@@ -473,21 +540,21 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
                 tc::commit(&bar);
             }
             if (!(ok = sg_wait(&bar, phase))) break;
-            sg_epi_back(D4, D3, bias3, actA, r, 32 * h, 1, nullptr, nullptr);
+            sg_back_epi<true>(D4, D3, actA, r, 32 * h, nullptr);
             sg_sync_for_mma();
             if (warp == 0 && tc::elect_one()) {
                 tc::gemm(T3, aA, LBO_K, SBO_K, aW3, LBO_M, SBO_M, 128, ID_KM, false);
                 tc::commit(&bar);
             }
             if (!(ok = sg_wait(&bar, phase))) break;
-            sg_epi_back(D3, D2, bias2, actB, r, 32 * h, 1, nullptr, nullptr);
+            sg_back_epi<true>(D3, D2, actB, r, 32 * h, nullptr);
             sg_sync_for_mma();
             if (warp == 0 && tc::elect_one()) {
                 tc::gemm(T2, aB, LBO_K, SBO_K, aW2, LBO_M, SBO_M, 128, ID_KM, false);
                 tc::commit(&bar);
             }
             if (!(ok = sg_wait(&bar, phase))) break;
-            xs_part = sg_epi_back(D2, D1, b1p, actA, r, 32 * h, 1, vleg, nullptr);
+            xs_part = sg_back_epi<MODE == SGF_ALL>(D2, D1, actA, r, 32 * h, vleg);
         }
         if (MODE == SGF_ALL) {
             sg_sync_for_mma();
@@ -521,8 +588,7 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
                          (xq[(k * 4 + 2) * 128 + r] + xq[(k * 4 + 3) * 128 + r]);
             const float out = sum[0] + bo;
             // the traveltime in FP64: background plus the network's term
-            double Tb, bxs, bz, bx, m;
-            sg_background<double>(n, (double)L.pos, (double)zf, (double)xf, Tb, bxs, bz, bx);
+            double m;
             const double osc = sg_out_scale<double>(n, Tb, m);
             const double T = Tb + osc * (double)out;
             const size_t o = (size_t)j * nzx + i;
@@ -538,11 +604,11 @@ __global__ void __launch_bounds__(512, 1) k_sg_fields(SgFieldArgs a)
                     phi = (sqrt(Tx * Tx + Tz * Tz) <= 1.0e-12) ? __longlong_as_double(0x7ff8000000000000ll)
                                                                : atan2(Tz, Tx);
                 }
-                const double w = leg_aperture_weight(L.pos, iz, ix, a.dz, a.x0, a.dx, a.aper, a.aper_taper, a.rmin,
-                                                     a.rtaper);
                 a.out.TP[o] = make_double2(T, phi);
-                a.out.XW[o] = make_float2((float)Txs * L.scale, (float)w);
+                a.out.XW[o].x = (float)Txs * L.scale;
             }
+        } else if (MODE != SGF_T && h == 1 && valid) {
+            a.out.XW[(size_t)j * nzx + i].y = apw;
         }
         __syncthreads();
     }
@@ -912,6 +978,7 @@ static int launch_sg_fields(const SgNet &net, const LegInterp *legs, int nlegs, 
     a.aper_taper = p.aperture_taper;
     a.rmin = p.aperture_rmin;
     a.rtaper = p.aperture_rtaper;
+    a.apb = aperture_bounds(a.aper, a.aper_taper);
     a.out = out;
     a.status = status;
     const long long items = (long long)nlegs * ((g.nz * g.nx + 127) / 128);

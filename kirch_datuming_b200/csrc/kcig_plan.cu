@@ -292,6 +292,7 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
         a.aper_taper = P->p.aperture_taper;
         a.rmin = P->p.aperture_rmin;
         a.rtaper = P->p.aperture_rtaper;
+        a.apb = aperture_bounds(a.aper, a.aper_taper);
         a.status = P->d_status.as<int>();
         a.type_p = P->p.interp_type == 'p';
         if (tx_table) {
@@ -345,6 +346,7 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
         a.aper_taper = P->p.aperture_taper;
         a.rmin = P->p.aperture_rmin;
         a.rtaper = P->p.aperture_rtaper;
+        a.apb = aperture_bounds(a.aper, a.aper_taper);
         a.cone = P->p.tool == 1;
         a.status = P->d_status.as<int>();
         a.type_p = P->p.interp_type == 'p';
@@ -1928,6 +1930,7 @@ extern "C" int kcig_leg_fields_noalloc(const kcig_params *p, const kcig_geometry
     a.aper_taper = p->aperture_taper;
     a.rmin = p->aperture_rmin;
     a.rtaper = p->aperture_rtaper;
+    a.apb = aperture_bounds(a.aper, a.aper_taper);
     a.cone = p->tool == 1;
     a.status = d_status;
     a.type_p = p->interp_type == 'p';
