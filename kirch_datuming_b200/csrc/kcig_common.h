@@ -122,7 +122,7 @@ struct Fold {
 
 struct PreludeArgs {
     const float *data;      // [ns][nh][nt] whole data cube on the device
-    double2 *D;             // [ntr][nt] {D[i], D[i+1]}, ntr = nshots * nhc
+    double2 *D;             // [ntr][nt] segments {D[i] - i dD[i], dD[i]}, ntr = nshots * nhc
     const double *mute_sx;  // [ntr] source x (mute)   (null: no mute)
     const double *mute_rx;  // [ntr] receiver x (mute)
     int ntr, nt, isdiff, invert;
@@ -171,6 +171,7 @@ struct SumArgs {
     int gchunk0, gchunk1;  // bin range handled by this launch
     Fold fold;             // pairs of skipped reciprocal traces are left out
     int shot0, rcv0;       // first shot and receiver of the batch in the call
+    double uk, ub, utop, uhi, top;  // set by launch_sum: u = theta uk + ub, ng - 1 (+ 1e-5), nt - 1
     int trs;               // traces per shot in D and the per-trace arrays (nh, or more)
 };
 int launch_sum(const SumArgs &a, cudaStream_t st, int *launches);

@@ -1,9 +1,10 @@
 // sm_100a kernels of the adjoint angle-domain Kirchhoff summation.
 //
 //   K1 k_prelude_cta  per-trace direct mute + doubint (FP64 running sums) +
-//                     optional diff2, written as {D[i], D[i+1]-D[i]} pairs so
-//                     a linear-interpolated pick is one 16-byte load and one
-//                     fused multiply-add.
+//                     optional diff2, written as line segments {D[i] - i dD[i],
+//                     dD[i]}, dD[i] = D[i+1] - D[i], so a linear-interpolated
+//                     pick at position f is one 16-byte load and one fused
+//                     multiply-add with f itself.
 //   K2 k_leg_*        per source/receiver position: table interpolation along
 //                     the position axis, traveltime gradient, triangle
 //                     smoothing and the aperture leg weight ("leg fields").
@@ -296,8 +297,8 @@ __global__ void __launch_bounds__(32 * kPreludeWarps) k_prelude_cta(PreludeArgs 
     double2 *out = a.D + (size_t)tr * a.nt;
     for (int i = tid; i < nt; i += PT) {
         double2 e;
-        e.x = D[i];
         e.y = (i + 1 < nt) ? D[i + 1] - D[i] : 0.0;
+        e.x = fma(-(double)i, e.y, D[i]);  // the segment's line at sample 0
         out[i] = e;
     }
 }
@@ -1065,7 +1066,9 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 #define KCIG_SUM_MINB_UNSHARED KCIG_SUM_MINB
 #endif
 
-template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool FOLD>
+// PLAIN: every trace weight of the launch is 1 and it holds all angle bins
+// (one chunk), so neither a weight nor a bin's range is tested per pair.
+template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool FOLD, bool PLAIN>
 __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_MINB_UNSHARED) * 128 / (TZ * TX))
     k_sum(const __grid_constant__ SumArgs a)
 {
@@ -1108,9 +1111,9 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     // continuous at the cutoff, so the comparison's rounding is immaterial)
     const bool no_taper = a.ats < 0.0f || a.ate <= a.ats;
     const double th_one = no_taper ? (double)cutoff / a.deg : -1.0;
-    const double ulo = -1.0e-5, uhi = (double)(a.ng - 1) + 1.0e-5;
-    const double uk = a.deg * a.uinv, ub = a.ug0 * a.uinv;  // u = th*uk - ub
-    const double top = (double)(a.nt - 1);
+    // the bin coordinate u = th*uk + ub and its limits, and the last sample,
+    // are operands from the launch's constants, not registers of every thread
+    const double ulo = -1.0e-5;
     const float inv_dt_f = (float)a.inv_dt;
     const bool aal_pos = a.aal >= 0.0f;
     const float aal_abs = fabsf(a.aal), aal_sgn = aal_pos ? 1.0f : -1.0f;
@@ -1156,7 +1159,7 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
 #pragma unroll
         for (int j = 0; j < KR; j++) {
             const bool live = SHARED_R || sb + j < s_hi;
-            topk[j] = (!SHARED_R && a.stop && live) ? (double)__ldg(a.stop + sb + j) : top;
+            topk[j] = (!SHARED_R && a.stop && live) ? (double)__ldg(a.stop + sb + j) : a.top;
             nrk[j] = !live ? 0 : ((!SHARED_R && a.snh) ? __ldg(a.snh + sb + j) : a.nh);
             nr = max(nr, nrk[j]);
             fnext[j] = 0;
@@ -1194,10 +1197,10 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 if (!SHARED_R && r >= nrk[j]) continue;
                 const double2 rTPk = rTP[j];
                 const float2 rXWk = rXW[j];
-                const double topj = topk[j];
+                const double topj = SHARED_R ? a.top : topk[j];
                 const int trc = (sb + k) * a.trs + r;
-                const float tw = a.unit_tw ? 1.0f : __ldg(a.trw + trc);
-                if (tw == 0.0f) continue;  // trace removed by aperture_trace / offset bin
+                const float tw = PLAIN || a.unit_tw ? 1.0f : __ldg(a.trw + trc);
+                if (!PLAIN && tw == 0.0f) continue;  // trace removed by aperture_trace / offset bin
                 const float apw = sXW[k].y * rXWk.y;
                 if (!(apw > 0.0f)) continue;
                 int b0 = 0;
@@ -1221,18 +1224,18 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                     // difference of the gradient directions folded to [0, pi]
                     double th = fabs(sTP[k].y - rTPk.y);
                     th = (th > kPiD) ? kTwoPi - th : th;
-                    const double u = fma(th, uk, -ub);  // bin coordinate; NaN: vanishing gradient
+                    const double u = fma(th, a.uk, a.ub);  // bin coordinate; NaN: vanishing gradient
                     double fl = 0.0;
                     if (MODE == 0) {
                         // value_to_linear_bins (:54-79)
-                        if (!(u >= ulo && u <= uhi)) continue;
+                        if (!(u >= ulo && u <= a.uhi)) continue;
                     } else {
                         // value_to_nearest_bin (:35-41)
                         fl = floor(u + 0.5);
-                        if (!(fl >= 0.0 && fl < (double)a.ng)) continue;
+                        if (!(fl >= 0.0 && fl <= a.utop)) continue;
                     }
                     if (th <= th_one) {
-                        aw = tw * apw;
+                        aw = PLAIN ? apw : tw * apw;
                     } else {
                         const float ang = (float)(th * a.deg);
                         aw = taper_weight(ang, a.ats, a.ate) * depth_weight(ang, cutoff, a.oaztaper) * tw * apw;
@@ -1240,7 +1243,7 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                     }
                     if (MODE == 0) {
                         if (u <= 0.0) { b0 = 0; w0 = 1.0f; w1 = 0.0f; }
-                        else if (u >= (double)(a.ng - 1)) { b0 = a.ng - 1; w0 = 1.0f; w1 = 0.0f; }
+                        else if (u >= a.utop) { b0 = a.ng - 1; w0 = 1.0f; w1 = 0.0f; }
                         else {
                             const double fu = floor_shift(u);  // u in (0, ng - 1)
                             b0 = __double2loint(fu);
@@ -1250,7 +1253,7 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                     } else {
                         b0 = (int)fl;
                     }
-                    b0 -= gc0;
+                    if (!PLAIN) b0 -= gc0;
                 }
                 // kirmig_pick (kirmig.cpp:34-58): sample positions of t,
                 // t-deltat-dt and t+deltat+dt in FP64; every test fails on NaN
@@ -1281,13 +1284,13 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 const double2 qm = __ldg(Dk + __double2loint(fms));
                 const double2 qp = __ldg(Dk + __double2loint(fps));
                 const float r1 = __fdividef(1.0f, fmaf(2.0f, shf, 1.0f));  // dt / (dt + tp - tm), 2 ulp
-                const double sum = 2.0 * fma(ft0 - (f0s - kFloorShift), q0.y, q0.x) -
-                                   fma(ftm0 - (fms - kFloorShift), qm.y, qm.x) -
-                                   fma(ftp0 - (fps - kFloorShift), qp.y, qp.x);
+                // each segment's line at the position itself: no fraction is formed
+                const double sum = 2.0 * fma(ft0, q0.y, q0.x) - fma(ftm0, qm.y, qm.x) - fma(ftp0, qp.y, qp.x);
                 const float picked = (float)sum * (r1 * r1 * aw);
-                // 0 <= b < nb as one unsigned test each
-                if ((unsigned)b0 < (unsigned)nb) acc[b0 * P + tid] += w0 * picked;
-                if (MODE == 0 && w1 > 0.0f && (unsigned)(b0 + 1) < (unsigned)nb) acc[(b0 + 1) * P + tid] += w1 * picked;
+                // 0 <= b < nb as one unsigned test each (u <= ng - 1: w1 > 0 has its bin)
+                if (PLAIN || (unsigned)b0 < (unsigned)nb) acc[b0 * P + tid] += w0 * picked;
+                if (MODE == 0 && w1 > 0.0f && (PLAIN || (unsigned)(b0 + 1) < (unsigned)nb))
+                    acc[(b0 + 1) * P + tid] += w1 * picked;
             }
         }
     }
@@ -1432,7 +1435,8 @@ static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 {
     constexpr int P = TZ * TX;
     const size_t sm = (size_t)nb * P * sizeof(float);
-    auto kern = k_sum<TZ, TX, KB, SR, MODE, FOLD>;
+    auto kern = k_sum<TZ, TX, KB, SR, MODE, FOLD, false>;
+    if (MODE <= 1 && a.unit_tw && nb == a.ng) kern = k_sum<TZ, TX, KB, SR, MODE, FOLD, MODE <= 1>;
     // all of the unified L1/shared memory as shared: the accumulators of as
     // many CTAs as the registers allow (the driver's own choice held 8x8
     // tiles to 10 CTAs per SM)
@@ -1486,8 +1490,14 @@ static int launch_sum_mode(const SumArgs &a, int nb, cudaStream_t st)
 // most 384 bins.
 const int kSumTileShape[kSumTiles][3] = {{0, 0, 0}, {16, 8, 4}, {8, 8, 4}, {8, 16, 4}, {16, 8, 2}};
 
-int launch_sum(const SumArgs &a0, cudaStream_t st, int *launches)
+int launch_sum(const SumArgs &args, cudaStream_t st, int *launches)
 {
+    SumArgs a0 = args;
+    a0.uk = a0.deg * a0.uinv;
+    a0.ub = -(a0.ug0 * a0.uinv);
+    a0.utop = (double)(a0.ng - 1);
+    a0.uhi = a0.utop + 1.0e-5;
+    a0.top = (double)(a0.nt - 1);
     if (a0.fold.on) {
         // receivers before the first folded group's: no trace of theirs has a
         // reciprocal among the shots, they go as an unfolded summation first
