@@ -160,7 +160,7 @@ struct SumArgs {
     int zero_init;
     int nz, nx, nt, nsb, nh, ng;
     int mode;              // 0 angle two-bin, 1 angle nearest, 2 single bin (offset/stack), 3 kirchmig2d cone + bin
-    int unit_tw;           // every trace weight of the batch is 1: trw is not read
+    int unit_tw;           // every trace weight of the batch is 1 or 0: k_sum does not read trw
     int shared_r;          // receiver fields indexed by ih only (cmp=0)
     int half;
     double t0, dt, inv_dt, tau;
@@ -172,9 +172,16 @@ struct SumArgs {
     Fold fold;             // pairs of skipped reciprocal traces are left out
     int shot0, rcv0;       // first shot and receiver of the batch in the call
     double uk, ub, utop, uhi, top;  // set by launch_sum: u = theta uk + ub, ng - 1 (+ 1e-5), nt - 1
-    int trs;               // traces per shot in D and the per-trace arrays (nh, or more)
+    void *cull;            // scratch of sum_cull_bytes
+    int nrl;               // receiver legs (RTP, RXW)
+    int unit_all;          // every trace weight is 1, none is 0 (unit_tw: every one that is not 0)
+    int nblk;              // set by launch_sum: blocks of shots, and per tile and block the
+    const int *cnt;        // [tiles][nblk] number of receivers with a pair that may reach the tile
+    const unsigned *list;  // [tiles][nblk][nh] and those receivers: r << 4 | shots of the block
 };
-int launch_sum(const SumArgs &a, cudaStream_t st, int *launches);
+// launches: k_sum launches added; aux: the launches that prepare them added
+int launch_sum(const SumArgs &a, cudaStream_t st, int *launches, int *aux = nullptr);
+size_t sum_cull_bytes(int nz, int nx, int nsb, int nh, int nrl, int ng, int tile, bool shared_r);
 // Tile variants the summation can be launched with (the autotuner's choices):
 // {TZ, TX, shots per block on the receiver-shared path}.
 // Forward modelling (adj=0): the picks of k_sum run backwards, each image

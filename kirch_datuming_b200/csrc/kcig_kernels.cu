@@ -1068,7 +1068,7 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 
 // PLAIN: every trace weight of the launch is 1 and it holds all angle bins
 // (one chunk), so neither a weight nor a bin's range is tested per pair.
-template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool FOLD, bool PLAIN>
+template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_MINB_UNSHARED) * 128 / (TZ * TX))
     k_sum(const __grid_constant__ SumArgs a)
 {
@@ -1083,25 +1083,13 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     const int nzx = a.nz * a.nx;
     const int i = valid ? ix * a.nz + iz : 0;
     const int gc0 = a.gchunk0, nb = a.gchunk1 - a.gchunk0;
-    // this CTA row's share of the shots (whole blocks of KB); of folded
-    // surveys, whose later blocks have fewer receivers left, every nsplit-th
-    int s_lo = 0, s_hi = a.nsb;
-    float *out = a.image;
-    if (a.nsplit > 1) {
-        const int nblk = (a.nsb + KB - 1) / KB;
-        if (FOLD) {
-            s_lo = (int)blockIdx.y * KB;
-        } else {
-            s_lo = (int)((long long)nblk * blockIdx.y / a.nsplit) * KB;
-            s_hi = min(a.nsb, (int)((long long)nblk * (blockIdx.y + 1) / a.nsplit) * KB);
-        }
-        out = a.partial + (size_t)blockIdx.y * a.ng * nzx;
-    }
+    // this CTA row's share of the blocks of KB shots: every nsplit-th
+    float *out = a.nsplit > 1 ? a.partial + (size_t)blockIdx.y * a.ng * nzx : a.image;
     const bool fresh = a.zero_init || a.nsplit > 1;
 
     for (int b = 0; b < nb; b++)
         acc[b * P + tid] = (fresh || !valid) ? 0.0f : a.image[(size_t)(gc0 + b) * nzx + i];
-    if (!valid) return;  // no block-wide synchronisation follows
+    if (!valid) return;  // no synchronisation follows
 
     // cutoff of angle_depth_mute_weight (:200-211) depends only on depth
     const float zf = (a.nz > 1) ? (float)iz / (float)(a.nz - 1) : 0.0f;
@@ -1122,19 +1110,19 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     // shot (receivers not shared), so that KB independent (shot, receiver)
     // gather chains are in flight per thread either way
     constexpr int KR = SHARED_R ? 1 : KB;
-    for (int sb = s_lo; sb < s_hi; sb += FOLD ? KB * a.nsplit : KB) {
-        // first receiver: a folded block starts at its own shots' receivers
-        // (the traces before them are migrated with their reciprocals)
-        int r0 = 0;
-        if (FOLD) {
-            const int g = (a.shot0 + sb) / kFoldGroup;
-            if (g > a.fold.ga && g < a.fold.gb) r0 = max(0, kFoldGroup * g + a.fold.off - a.rcv0);
-        }
+    for (int blk = blockIdx.y; blk < a.nblk; blk += gridDim.y) {
+        // the block's receivers with a pair that may reach this tile, in
+        // order, each with the shots it may do so with (k_cull)
+        const size_t lb = (size_t)blockIdx.x * a.nblk + blk;
+        const int cnt = __ldg(a.cnt + lb);
+        if (cnt == 0) continue;
+        const unsigned *lst = a.list + lb * a.nh;
+        const int sb = blk * KB;
         double2 sTP[KB];
         float2 sXW[KB];
 #pragma unroll
         for (int k = 0; k < KB; k++) {
-            if (sb + k < s_hi) {
+            if (sb + k < a.nsb) {
                 sTP[k] = __ldg(a.STP + (size_t)(sb + k) * nzx + i);
                 sXW[k] = __ldg(a.SXW + (size_t)(sb + k) * nzx + i);
                 // the shot's share of the pick position and of the
@@ -1146,34 +1134,34 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 sXW[k] = make_float2(0.f, 0.f);
             }
         }
-        // per stream: the last usable sample of its traces and its receiver
-        // count (ragged shots carry their own), and its fields loaded one
-        // receiver ahead of use (through the trace's field index when not
-        // shared, with the index of the receiver after next loaded too, so
-        // the index load does not stand in front of the field load)
+        // per stream: the last usable sample of its traces (ragged shots carry
+        // their own) and its fields, loaded one list entry ahead of use; with
+        // receivers of its own, through the trace's field index, loaded one
+        // entry earlier still (the entry itself another one)
         double topk[KR];
-        int nrk[KR], fnext[KR];
+        int fnext[KR];
         double2 nTP[KR];
         float2 nXW[KR];
-        int nr = 0;
+        unsigned e1 = __ldg(lst), e2 = cnt > 1 ? __ldg(lst + 1) : 0u, e3 = !SHARED_R && cnt > 2 ? __ldg(lst + 2) : 0u;
 #pragma unroll
         for (int j = 0; j < KR; j++) {
-            const bool live = SHARED_R || sb + j < s_hi;
-            topk[j] = (!SHARED_R && a.stop && live) ? (double)__ldg(a.stop + sb + j) : a.top;
-            nrk[j] = !live ? 0 : ((!SHARED_R && a.snh) ? __ldg(a.snh + sb + j) : a.nh);
-            nr = max(nr, nrk[j]);
+            topk[j] = (!SHARED_R && a.stop && sb + j < a.nsb) ? (double)__ldg(a.stop + sb + j) : a.top;
             fnext[j] = 0;
             nTP[j] = make_double2(0.0, 0.0);
             nXW[j] = make_float2(0.f, 0.f);
-            if (FOLD ? r0 < nrk[j] : nrk[j] > 0) {
-                const int *rfi_j = a.rfi + (size_t)(sb + j) * a.nh;
-                const size_t f0 = SHARED_R ? (FOLD ? (size_t)r0 : 0) : (size_t)__ldg(rfi_j);
+            if (SHARED_R || (e1 >> j & 1u)) {
+                const size_t f0 = SHARED_R ? (size_t)(e1 >> 4) : (size_t)__ldg(a.rfi + (size_t)(sb + j) * a.nh + (e1 >> 4));
                 nTP[j] = __ldg(a.RTP + f0 * nzx + i);
                 nXW[j] = __ldg(a.RXW + f0 * nzx + i);
-                if (!SHARED_R && nrk[j] > 1) fnext[j] = __ldg(rfi_j + 1);
             }
+            if (!SHARED_R && (e2 >> j & 1u)) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + (e2 >> 4));
         }
-        for (int r = FOLD ? r0 : 0; r < nr; r++) {
+        for (int q = 0; q < cnt; q++) {
+            const unsigned e0 = e1;
+            const int r = (int)(e0 >> 4);
+            e1 = e2;  // 0 past the end
+            e2 = SHARED_R ? (q + 2 < cnt ? __ldg(lst + q + 2) : 0u) : e3;
+            if (!SHARED_R) e3 = q + 3 < cnt ? __ldg(lst + q + 3) : 0u;
             double2 rTP[KR];
             float2 rXW[KR];
 #pragma unroll
@@ -1183,24 +1171,22 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 // the receiver's share, once per receiver for the stream's shots
                 rTP[j].x *= a.inv_dt;
                 rXW[j].x = fabsf(rXW[j].x) * aal_abs * inv_dt_f;
-                if (r + 1 < nrk[j]) {  // next receiver, one ahead of use
-                    const size_t f1 = SHARED_R ? (size_t)(r + 1) : (size_t)fnext[j];
+                if (SHARED_R ? e1 != 0u : (e1 >> j & 1u) != 0u) {
+                    const size_t f1 = SHARED_R ? (size_t)(e1 >> 4) : (size_t)fnext[j];
                     nTP[j] = __ldg(a.RTP + f1 * nzx + i);
                     nXW[j] = __ldg(a.RXW + f1 * nzx + i);
-                    if (!SHARED_R && r + 2 < nrk[j]) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + r + 2);
                 }
+                if (!SHARED_R && (e2 >> j & 1u)) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + (e2 >> 4));
             }
 #pragma unroll
             for (int k = 0; k < KB; k++) {
-                if (sb + k >= s_hi) break;
+                if (!(e0 >> k & 1u)) continue;
                 const int j = SHARED_R ? 0 : k;  // this shot's receiver stream
-                if (!SHARED_R && r >= nrk[j]) continue;
                 const double2 rTPk = rTP[j];
                 const float2 rXWk = rXW[j];
                 const double topj = SHARED_R ? a.top : topk[j];
-                const int trc = (sb + k) * a.trs + r;
-                const float tw = PLAIN || a.unit_tw ? 1.0f : __ldg(a.trw + trc);
-                if (!PLAIN && tw == 0.0f) continue;  // trace removed by aperture_trace / offset bin
+                const int trc = (sb + k) * a.nh + r;
+                const float tw = PLAIN || a.unit_tw ? 1.0f : __ldg(a.trw + trc);  // not 0: k_cull
                 const float apw = sXW[k].y * rXWk.y;
                 if (!(apw > 0.0f)) continue;
                 int b0 = 0;
@@ -1430,13 +1416,137 @@ __global__ void k_sum_reduce(float *image, const float *partial, int nsplit, siz
     image[j] = v;
 }
 
-template <int TZ, int TX, int KB, bool SR, int MODE, bool FOLD = false>
+// ---- pairs that cannot reach a tile -------------------------------------------
+// Most pairs of a survey miss most tiles: the opening angle of a wide pair is
+// past the last bin, its reflection time past the record's end (of the
+// production survey's pairs 2.7% contribute, of the 201 x 401 survey's 35%).
+// Per leg and tile, the ranges of direction and time over the tile's points
+// bound both; k_cull lists, per tile and block of shots, the receivers with a
+// pair that may contribute.  Ranges are rounded outward and compared with a
+// margin, so no contributing pair is dropped: the sums are unchanged, pair for
+// pair and in order.
+
+// {direction lo, hi, time lo, hi} of leg j over tile t, at [t][j]; a tile
+// without a usable point gets an empty time range.  One warp per (tile, leg).
+template <int TZ, int TX>
+__global__ void __launch_bounds__(256) k_leg_bounds(const double2 *TP, const float2 *XW, int nlegs, int nz, int nx,
+                                                    int angle, float4 *out, int stride, int first)
+{
+    const int lane = threadIdx.x & 31, j = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (j >= nlegs) return;
+    const int tiles_z = (nz + TZ - 1) / TZ, tz = blockIdx.x % tiles_z, tx = blockIdx.x / tiles_z;
+    const size_t base = (size_t)j * nz * nx;
+    float pl = INFINITY, ph = -INFINITY, tl = INFINITY, th = -INFINITY;
+#pragma unroll
+    for (int q = 0; q < TZ * TX / 32; q++) {
+        const int p = q * 32 + lane, iz = tz * TZ + p % TZ, ix = tx * TX + p / TZ;
+        if (iz >= nz || ix >= nx) continue;
+        const size_t i = base + (size_t)ix * nz + iz;
+        const double2 v = __ldg(TP + i);
+        if (!(__ldg(&XW[i].y) > 0.0f) || (angle && isnan(v.y))) continue;  // no pair here
+        if (angle) {
+            pl = fminf(pl, __double2float_rd(v.y));
+            ph = fmaxf(ph, __double2float_ru(v.y));
+        }
+        tl = fminf(tl, __double2float_rd(v.x));  // NaN times drop out
+        th = fmaxf(th, __double2float_ru(v.x));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        pl = fminf(pl, __shfl_xor_sync(0xffffffffu, pl, o));
+        ph = fmaxf(ph, __shfl_xor_sync(0xffffffffu, ph, o));
+        tl = fminf(tl, __shfl_xor_sync(0xffffffffu, tl, o));
+        th = fmaxf(th, __shfl_xor_sync(0xffffffffu, th, o));
+    }
+    if (lane == 0) out[(size_t)blockIdx.x * stride + first + j] = make_float4(pl, ph, tl, th);
+}
+
+// whether a pair of legs may contribute somewhere in the tile
+__device__ __forceinline__ bool cull_keep(const SumArgs &a, float4 s, float4 r, float top)
+{
+    const float idt = (float)a.inv_dt, sft = (float)(a.tau - a.t0);
+    const float lo = (s.z + r.z + sft) * idt, hi = (s.w + r.w + sft) * idt;
+    // the centre sample lies in [0, top) (a whole sample of margin)
+    if (!(lo < top + 1.0f + 1e-6f * fabsf(lo)) || !(hi > -1.0f - 1e-6f * fabsf(hi))) return false;
+    if (a.mode >= 2) return true;
+    constexpr float kPi = 3.14159265f;
+    const float d0 = s.x - r.y, d1 = s.y - r.x;  // range of the directions' difference
+    const float m = fmaxf(0.0f, fmaxf(d0, -d1)), M = fmaxf(fabsf(d0), fabsf(d1));
+    // folded to [0, pi]: th = |d| or 2 pi - |d|
+    const float t0 = M <= kPi ? m : fmaxf(0.0f, fminf(m, 2.0f * kPi - M));
+    const float t1 = M <= kPi ? M : m >= kPi ? 2.0f * kPi - m : kPi;
+    const float u0 = t0 * (float)a.uk + (float)a.ub, u1 = t1 * (float)a.uk + (float)a.ub;
+    // half a bin for the nearest-bin rule, and a margin over the directions' rounding
+    const float pad = 0.52f + 2e-6f * (float)a.uk;
+    return u0 <= (float)a.utop + pad && u1 >= -pad;
+}
+
+// One warp per (tile, block of KB shots): the block's receivers in order, 32
+// at a time, an entry r << 4 | shots where some shot's pair may contribute.
+// Left out too: traces of weight 0, a ragged shot's missing receivers, and
+// reciprocal traces migrated with an earlier shot group (struct Fold).
+template <int KB>
+__global__ void __launch_bounds__(256) k_cull(const __grid_constant__ SumArgs a, const float4 *bs, const float4 *br,
+                                              int ns_stride, int nr_stride, int ntiles, unsigned *list, int *cnt)
+{
+    const int lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= (long long)ntiles * a.nblk) return;
+    const int tile = (int)(w / a.nblk), blk = (int)(w % a.nblk), sb = blk * KB;
+    const float4 *R = br + (size_t)tile * nr_stride;
+    float4 S[KB];
+    float top[KB];
+    int nr[KB];
+#pragma unroll
+    for (int k = 0; k < KB; k++) {
+        const bool live = sb + k < a.nsb;
+        S[k] = live ? __ldg(bs + (size_t)tile * ns_stride + sb + k) : make_float4(0.f, 0.f, INFINITY, -INFINITY);
+        top[k] = a.stop && live ? __ldg(a.stop + sb + k) : (float)a.top;
+        nr[k] = !live ? 0 : a.snh ? __ldg(a.snh + sb + k) : a.nh;
+    }
+    // receivers f_lo .. f_hi - 1 go with their reciprocals of earlier groups
+    int f_lo = 0, f_hi = 0;
+    if (a.fold.on) {
+        const int g = (a.shot0 + sb) / kFoldGroup;
+        if (g > a.fold.ga && g < a.fold.gb) {
+            f_lo = kFoldGroup * a.fold.ga + a.fold.off - a.rcv0;
+            f_hi = kFoldGroup * g + a.fold.off - a.rcv0;
+        }
+    }
+    unsigned *o = list + (size_t)w * a.nh;
+    int n = 0;
+    for (int r0 = 0; r0 < a.nh; r0 += 32) {
+        const int r = r0 + lane;
+        unsigned m = 0;
+        if (r < a.nh && !(r >= f_lo && r < f_hi)) {
+            float4 L;
+            if (a.shared_r) L = __ldg(R + r);
+#pragma unroll
+            for (int k = 0; k < KB; k++) {
+                if (r >= nr[k]) continue;
+                const size_t t = (size_t)(sb + k) * a.nh + r;
+                if (!a.unit_all && __ldg(a.trw + t) == 0.0f) continue;
+                if (!a.shared_r) L = __ldg(R + __ldg(a.rfi + t));
+                if (cull_keep(a, S[k], L, top[k])) m |= 1u << k;
+            }
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, m != 0);
+        if (m) o[n + __popc(b & ((1u << lane) - 1))] = (unsigned)r << 4 | m;
+        n += __popc(b);
+    }
+    if (lane == 0) cnt[w] = n;
+}
+
+// tile and shots per block of a launch of nb bins
+static void sum_shape(int tile, int nb, bool shared_r, int *tz, int *tx, int *kb);
+
+template <int TZ, int TX, int KB, bool SR, int MODE>
 static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 {
     constexpr int P = TZ * TX;
     const size_t sm = (size_t)nb * P * sizeof(float);
-    auto kern = k_sum<TZ, TX, KB, SR, MODE, FOLD, false>;
-    if (MODE <= 1 && a.unit_tw && nb == a.ng) kern = k_sum<TZ, TX, KB, SR, MODE, FOLD, MODE <= 1>;
+    auto kern = k_sum<TZ, TX, KB, SR, MODE, false>;
+    if (MODE <= 1 && a.unit_tw && nb == a.ng) kern = k_sum<TZ, TX, KB, SR, MODE, MODE <= 1>;
     // all of the unified L1/shared memory as shared: the accumulators of as
     // many CTAs as the registers allow (the driver's own choice held 8x8
     // tiles to 10 CTAs per SM)
@@ -1456,11 +1566,6 @@ static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 template <int TZ, int TX, int KB>
 static int launch_sum_mode(const SumArgs &a, int nb, cudaStream_t st)
 {
-    if (a.shared_r && a.fold.on) {
-        if (a.mode == 0) return launch_sum_t<TZ, TX, KB, true, 0, true>(a, nb, st);
-        if (a.mode == 1) return launch_sum_t<TZ, TX, KB, true, 1, true>(a, nb, st);
-        return launch_sum_t<TZ, TX, KB, true, 2, true>(a, nb, st);
-    }
     if (a.shared_r) {
         if (a.mode == 0) return launch_sum_t<TZ, TX, KB, true, 0>(a, nb, st);
         if (a.mode == 1) return launch_sum_t<TZ, TX, KB, true, 1>(a, nb, st);
@@ -1490,46 +1595,93 @@ static int launch_sum_mode(const SumArgs &a, int nb, cudaStream_t st)
 // most 384 bins.
 const int kSumTileShape[kSumTiles][3] = {{0, 0, 0}, {16, 8, 4}, {8, 8, 4}, {8, 16, 4}, {16, 8, 2}};
 
-int launch_sum(const SumArgs &args, cudaStream_t st, int *launches)
+static void sum_shape(int tile, int nb, bool shared_r, int *tz, int *tx, int *kb)
 {
+    const bool fits128 = (size_t)nb * 128 * 4 <= 200 * 1024;  // every variant but 8x8 holds 128 points
+    if (tile == 2 || (tile >= 1 && tile <= 4 && fits128)) {
+        *tz = kSumTileShape[tile][0];
+        *tx = kSumTileShape[tile][1];
+        *kb = kSumTileShape[tile][2];
+    } else {
+        const bool fits = (size_t)nb * KCIG_TZ * KCIG_TX * 4 <= 200 * 1024;
+        *tz = fits ? KCIG_TZ : 8;
+        *tx = fits ? KCIG_TX : 8;
+        *kb = KCIG_KB;
+    }
+    if (!shared_r) *kb = KCIG_KB_UNSHARED;
+}
+
+constexpr int kMaxBins = 384;  // of one launch
+
+// the culling scratch of a launch: the legs' bounds, the counts and the lists
+size_t sum_cull_bytes(int nz, int nx, int nsb, int nh, int nrl, int ng, int tile, bool shared_r)
+{
+    size_t most = 0;
+    for (int nb : {std::min(ng, kMaxBins), (ng - 1) % kMaxBins + 1}) {
+        int tz, tx, kb;
+        sum_shape(tile, nb, shared_r, &tz, &tx, &kb);
+        const size_t tiles = (size_t)((nz + tz - 1) / tz) * ((nx + tx - 1) / tx), nblk = (nsb + kb - 1) / kb;
+        most = std::max(most, tiles * ((size_t)(nsb + nrl) * sizeof(float4) + nblk * (4 + (size_t)nh * 4)) + 64);
+    }
+    return most;
+}
+
+template <int TZ, int TX>
+static int launch_bounds_t(const SumArgs &a, const double2 *TP, const float2 *XW, int n, float4 *out, int tiles,
+                           int stride, int first, cudaStream_t st)
+{
+    for (int j0 = 0; j0 < n; j0 += 8 * 65535) {
+        const int nj = std::min(n - j0, 8 * 65535);
+        const size_t o = (size_t)j0 * a.nz * a.nx;
+        k_leg_bounds<TZ, TX><<<dim3(tiles, (nj + 7) / 8), 256, 0, st>>>(TP + o, XW + o, nj, a.nz, a.nx, a.mode < 2, out,
+                                                                       stride, first + j0);
+    }
+    KCIG_CUDA(cudaGetLastError());
+    return KCIG_OK;
+}
+
+int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
+{
+    static_assert((KCIG_KB == 4 || KCIG_KB == 2) && (KCIG_KB_UNSHARED == 2 || KCIG_KB_UNSHARED == 4), "k_cull's block sizes");
     SumArgs a0 = args;
     a0.uk = a0.deg * a0.uinv;
     a0.ub = -(a0.ug0 * a0.uinv);
     a0.utop = (double)(a0.ng - 1);
     a0.uhi = a0.utop + 1.0e-5;
     a0.top = (double)(a0.nt - 1);
-    if (a0.fold.on) {
-        // receivers before the first folded group's: no trace of theirs has a
-        // reciprocal among the shots, they go as an unfolded summation first
-        const int lead = min(a0.nh, kFoldGroup * a0.fold.ga + a0.fold.off - a0.rcv0);
-        if (lead > 0) {
-            SumArgs a = a0;
-            a.fold.on = 0;
-            a.nh = lead;
-            KCIG_TRY(launch_sum(a, st, launches));
-            if (lead == a0.nh) return KCIG_OK;
-            a = a0;
-            const size_t nzx = (size_t)a.nz * a.nx;
-            a.rcv0 += lead;
-            a.nh -= lead;
-            a.RTP += lead * nzx;
-            a.RXW += lead * nzx;
-            a.D += (size_t)lead * a.nt;
-            a.trw += lead;
-            a.rfi += lead;
-            a.igo += lead;
-            a.zero_init = 0;
-            return launch_sum(a, st, launches);
-        }
-    }
-    const int maxb = 384;
-    for (int g = 0; g < a0.ng; g += maxb) {
+    for (int g = 0; g < a0.ng; g += kMaxBins) {
         SumArgs a = a0;
         a.gchunk0 = g;
-        a.gchunk1 = min(a0.ng, g + maxb);
+        a.gchunk1 = min(a0.ng, g + kMaxBins);
         const int nb = a.gchunk1 - a.gchunk0;
+        int tz, tx, kb;
+        sum_shape(a.tile, nb, a.shared_r != 0, &tz, &tx, &kb);
+        a.nblk = (a.nsb + kb - 1) / kb;
+        // the lists of this tile shape: legs' bounds, then the receivers per
+        // tile and block.  Shots whose fields are a receiver's take its bounds.
+        const int tiles = ((a.nz + tz - 1) / tz) * ((a.nx + tx - 1) / tx);
+        const size_t nzx = (size_t)a.nz * a.nx;
+        const ptrdiff_t off = (a.STP - a.RTP) / (ptrdiff_t)nzx;
+        const bool alias = a.shared_r && a.STP >= a.RTP && off + a.nsb <= a.nrl;
+        float4 *br = reinterpret_cast<float4 *>(a.cull), *bs = alias ? br + off : br + (size_t)tiles * a.nrl;
+        const int ss = alias ? a.nrl : a.nsb;
+        int *cnt = reinterpret_cast<int *>(br + (size_t)tiles * (a.nrl + (alias ? 0 : a.nsb)));
+        unsigned *list = reinterpret_cast<unsigned *>(cnt) + (size_t)tiles * a.nblk;
+        auto bounds = [&](const double2 *TP, const float2 *XW, int n, float4 *out, int stride) -> int {
+            if (tz == 16) return launch_bounds_t<16, 8>(a, TP, XW, n, out, tiles, stride, 0, st);
+            if (tx == 16) return launch_bounds_t<8, 16>(a, TP, XW, n, out, tiles, stride, 0, st);
+            return launch_bounds_t<8, 8>(a, TP, XW, n, out, tiles, stride, 0, st);
+        };
+        KCIG_TRY(bounds(a.RTP, a.RXW, a.nrl, br, a.nrl));
+        if (!alias) KCIG_TRY(bounds(a.STP, a.SXW, a.nsb, bs, ss));
+        const unsigned grid = (unsigned)(((long long)tiles * a.nblk + 7) / 8);
+        if (kb == 4) k_cull<4><<<grid, 256, 0, st>>>(a, bs, br, ss, a.nrl, tiles, list, cnt);
+        else k_cull<2><<<grid, 256, 0, st>>>(a, bs, br, ss, a.nrl, tiles, list, cnt);
+        KCIG_CUDA(cudaGetLastError());
+        a.cnt = cnt;
+        a.list = list;
         int rc;
-        const bool fits128 = (size_t)nb * 128 * 4 <= 200 * 1024;  // every variant but 8x8 holds 128 points
+        const bool fits128 = (size_t)nb * 128 * 4 <= 200 * 1024;
         if (a.tile == 1 && fits128) rc = launch_sum_mode<16, 8, 4>(a, nb, st);
         else if (a.tile == 2) rc = launch_sum_mode<8, 8, 4>(a, nb, st);
         else if (a.tile == 3 && fits128) rc = launch_sum_mode<8, 16, 4>(a, nb, st);
@@ -1538,6 +1690,7 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches)
         else rc = launch_sum_mode<8, 8, KCIG_KB>(a, nb, st);
         if (rc) return rc;
         if (launches) (*launches)++;
+        if (aux) *aux += alias ? 2 : 3;
     }
     if (a0.nsplit > 1) {
         const size_t n = (size_t)a0.ng * a0.nz * a0.nx;

@@ -59,6 +59,7 @@ struct kcig_plan {
     DevBuf own_stab, own_sder, own_rtab, own_rder, own_sgx, own_sgz, own_rgx, own_rgz;
     DevBuf d_data, d_image, d_rT, d_rF, d_sT, d_sF, d_work, d_D, d_legs, d_tr;
     DevBuf d_part;  // partial images of a split summation (small grids)
+    DevBuf d_cull;  // the summation's lists of pairs that may reach a tile
     DevBuf d_status;  // flag of the leg-field kernels' bounded waits (k_leg_tile)
     // tables left in host memory (KCIG_MEM_HOST_STREAM): the slices of each
     // leg batch are copied into d_stage
@@ -463,7 +464,7 @@ extern "C" int kcig_plan_destroy(kcig_plan *P)
     DevBuf *bufs[] = {&P->own_stab, &P->own_sder, &P->own_rtab, &P->own_rder, &P->own_sgx, &P->own_sgz,
                       &P->own_rgx,  &P->own_rgz,  &P->d_data,   &P->d_image,  &P->d_rT,   &P->d_rF,
                       &P->d_sT,     &P->d_sF,   &P->d_work,   &P->d_D,      &P->d_legs, &P->d_tr,
-                      &P->d_part,   &P->d_stage};
+                      &P->d_part,   &P->d_stage, &P->d_cull};
     for (DevBuf *b : bufs) b->release();
     release_shots(P);
     if (P->own_st) cudaStreamDestroy(P->own_st);
@@ -758,9 +759,13 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     if (shared_r && (unsigned long long)nhc * leg_bytes > budget / 2)
         nhc = (int)std::max<unsigned long long>(1, (budget / 2) / leg_bytes);
     const size_t work_bytes = angle ? (size_t)std::min<size_t>(64, (256ull << 20) / (nzx * 32) + 1) * 4 * nzx * 8 : 0;
+    // culling scratch: of eight shots beside the receivers, and what eight more add
+    const size_t cull8 = sum_cull_bytes(g.nz, g.nx, 8, nhc, shared_r ? nhc : 8 * nhc, P->ng, P->tile, shared_r);
+    const size_t cull16 = sum_cull_bytes(g.nz, g.nx, 16, nhc, shared_r ? nhc : 16 * nhc, P->ng, P->tile, shared_r);
     const size_t per_shot = leg_bytes + (size_t)nhc * g.nt * sizeof(double2) + (size_t)nhc * 32 +
-                            (shared_r ? 0 : (size_t)nhc * leg_bytes);
-    const unsigned long long fixed = (shared_r ? (unsigned long long)nhc * leg_bytes : 0) + work_bytes;
+                            (shared_r ? 0 : (size_t)nhc * leg_bytes) + (cull16 - cull8) / 8;
+    const unsigned long long fixed =
+        (shared_r ? (unsigned long long)nhc * leg_bytes : 0) + work_bytes + (cull8 - (cull16 - cull8));
     long long room = (long long)budget - (long long)fixed;
     int nsb = (int)std::max<long long>(1, room / (long long)per_shot);
     nsb = std::min(nsb, ns);
@@ -917,7 +922,10 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.fold = fold;
             sa.shot0 = s0;
             sa.rcv0 = r0;
-            sa.trs = nhb;
+            sa.nrl = shared_r ? nhb : (int)rl.size();
+            rc = P->d_cull.ensure(sum_cull_bytes(g.nz, g.nx, nsh, nhb, sa.nrl, P->ng, P->tile, shared_r));
+            if (rc) break;
+            sa.cull = P->d_cull.p;
             sa.RTP = P->d_rT.as<double2>();
             sa.RXW = P->d_rF.as<float2>();
             sa.D = P->d_D.as<double2>();
@@ -934,7 +942,9 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.ng = P->ng;
             sa.mode = p.tool == 1 ? 3 : (angle ? (p.angle_interp ? 0 : 1) : 2);
             // a uniform flag spares the pair loop a dependent load per pair
-            sa.unit_tw = std::all_of(h_trw.begin(), h_trw.begin() + nb, [](float v) { return v == 1.0f; }) ? 1 : 0;
+            sa.unit_all = std::all_of(h_trw.begin(), h_trw.begin() + nb, [](float v) { return v == 1.0f; }) ? 1 : 0;
+            sa.unit_tw = sa.unit_all ||
+                         std::all_of(h_trw.begin(), h_trw.begin() + nb, [](float v) { return v == 1.0f || v == 0.0f; });
             sa.tile = P->tile;
             sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, shared_r);
             if (sa.nsplit > 1) {
@@ -967,7 +977,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             evs.push_back(e1);
             cudaEventRecord(e0, st);
             int nl = 0;
-            rc = launch_sum(sa, st, &nl);
+            rc = launch_sum(sa, st, &nl, &P->all_launches);
             cudaEventRecord(e1, st);
             if (rc) break;
             P->sum_launches += nl;
@@ -1345,7 +1355,9 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.nx = g.nx;
     sa.nt = S->ntmax;
     sa.nsb = B.ns;
-    sa.nh = sa.trs = B.nhb;
+    sa.nh = B.nhb;
+    sa.nrl = B.nrl;
+    sa.cull = P->d_cull.p;  // sized by kcig_shots_prepare and the autotuner
     sa.ng = P->ng;
     sa.mode = angle ? (p.angle_interp ? 0 : 1) : 2;
     sa.unit_tw = B.unit_tw;
@@ -1390,7 +1402,7 @@ int run_prepared(kcig_plan *P, float *d_img, cudaStream_t st, cudaEvent_t *ev = 
         if (ev) cudaEventRecord(ev[4 * b + 2], st);
         const SumArgs sa = batch_sum_args(P, b, d_img);
         int nl = 0;
-        KCIG_TRY(launch_sum(sa, st, &nl));
+        KCIG_TRY(launch_sum(sa, st, &nl, &P->all_launches));
         if (ev) cudaEventRecord(ev[4 * b + 3], st);
         P->sum_launches += nl;
         P->all_launches += nl + (sa.nsplit > 1 ? 1 : 0);
@@ -1476,7 +1488,8 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
             }
             const int ns1 = i1 - i0 + 1, nh1 = std::max(nhb, sh.nh);
             const size_t need = (size_t)(ns1 + seen.size() + add.size()) * leg_bytes +
-                                (size_t)ns1 * nh1 * ((size_t)ntmax * sizeof(double2) + 48) + work_bytes;
+                                (size_t)ns1 * nh1 * ((size_t)ntmax * sizeof(double2) + 48) + work_bytes +
+                                sum_cull_bytes(g.nz, g.nx, ns1, nh1, (int)(seen.size() + add.size()), P->ng, P->tile, false);
             if (i1 > i0 && need > budget) break;
             for (auto &kv : add) seen.emplace(kv.first, 0);
             nhb = nh1;
@@ -1512,7 +1525,6 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
                     h_rfi.push_back(0);
                     h_igo.push_back(0);
                     h_tnt.push_back(0);
-                    unit = false;
                     continue;
                 }
                 const double hx = sh.h ? (double)sh.h[r] : (double)sh.h0 + (double)r * (double)dhf;
@@ -1554,7 +1566,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
                     if (b < 0) w = 0.0;
                     ig = b < 0 ? 0 : b;
                 }
-                if (w != 1.0) unit = false;
+                if (w != 1.0 && w != 0.0) unit = false;
                 h_msx.push_back((double)sh.sx);
                 h_mrx.push_back(rpos);
                 h_toff.push_back((long long)(base[i0 + k] + (size_t)r * sh.nt));
@@ -1589,6 +1601,10 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
     int max_split = 1;
     for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, false));
     if (!rc && max_split > 1) rc = P->d_part.ensure((size_t)max_split * P->ng * nzx * sizeof(float));
+    size_t cull = 0;
+    for (const ShotBatch &B : S->batches)
+        cull = std::max(cull, sum_cull_bytes(g.nz, g.nx, B.ns, B.nhb, B.nrl, P->ng, P->tile, false));
+    if (!rc) rc = P->d_cull.ensure(cull);
     struct Cp { void *dst; const void *src; size_t bytes; } cps[] = {
         {S->legs.p, hlegs.data(), hlegs.size() * sizeof(LegInterp)},
         {S->trf.as<double>(), h_msx.data(), ntr * 8},
@@ -1732,6 +1748,12 @@ extern "C" int kcig_plan_autotune(kcig_plan *P, int *choice, float *ms)
     KCIG_TRY(P->d_image.ensure((size_t)P->ng * nzx * sizeof(float)));
     cudaStream_t st = P->st;
     KCIG_TRY(batch_inputs(P, 0, st));
+    // every variant's lists, for every batch: the chosen one stays
+    size_t cull = 0;
+    for (const ShotBatch &B : P->shots->batches)
+        for (int t = 0; t < kSumTiles; t++)
+            cull = std::max(cull, sum_cull_bytes(P->g.nz, P->g.nx, B.ns, B.nhb, B.nrl, P->ng, t, false));
+    KCIG_TRY(P->d_cull.ensure(cull));
     SumArgs sa = batch_sum_args(P, 0, P->d_image.as<float>());
     cudaEvent_t e0, e1;
     KCIG_CUDA(cudaEventCreate(&e0));
