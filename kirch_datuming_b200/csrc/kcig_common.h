@@ -91,6 +91,9 @@ int launch_leg_grad(const FieldArgs &a, LegFields out, double *work, cudaStream_
 // Whether launch_leg_grad uses the work planes (gradient volumes, or a halo
 // too wide for the fused kernel): 4 * nzx doubles per leg.
 bool leg_grad_needs_work(const FieldArgs &a);
+// Whether launch_leg_fields runs as one pass from the tables (any number of
+// legs in a launch, no work planes).
+bool leg_tile_applies(const FieldArgs &a);
 
 // Leg fields from a traveltime surrogate (kcig_mlp.cu): one launch for all
 // `nlegs` legs (only .pos and .scale of each are read).  mode 0: the
@@ -175,6 +178,7 @@ struct SumArgs {
     void *cull;            // scratch of sum_cull_bytes
     int nrl;               // receiver legs (RTP, RXW)
     int unit_all;          // every trace weight is 1, none is 0 (unit_tw: every one that is not 0)
+    int parts;             // set by launch_sum: parts of a block's list (rows of CTAs beyond the blocks)
     int nblk;              // set by launch_sum: blocks of shots, and per tile and block the
     const int *cnt;        // [tiles][nblk] number of receivers with a pair that may reach the tile
     const unsigned *list;  // [tiles][nblk][nh] and those receivers: r << 4 | shots of the block
@@ -207,9 +211,9 @@ int launch_doubint_f32(const double *in, float *out, int ntr, int nt, cudaStream
 // Gives back the memory kcig_eikods keeps between calls on the current device.
 int eik_release_pool();
 
-// How many shot splits a summation over nsb shots on an nz x nx image needs
-// to give the GPU at least two waves of CTAs (1: none).
-int sum_nsplit(int nz, int nx, int nsb, bool shared_r);
+// How many rows of CTAs (partial images) a summation over nsb shots of nh
+// receivers on an nz x nx image is split into to fill the GPU (1: none).
+int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r);
 constexpr int kSumTiles = 5;
 extern const int kSumTileShape[kSumTiles][3];
 

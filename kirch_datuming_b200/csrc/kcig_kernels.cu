@@ -977,7 +977,7 @@ bool leg_grad_needs_work(const FieldArgs &a)
 // between two positions, or a clamped end) with the angle on and no gradient
 // volumes; the partial-shift interpolation, gradient volumes, the kirchmig2d
 // cone flags and halos wider than its shared memory take the two-stage path.
-static bool leg_tile_applies(const FieldArgs &a)
+bool leg_tile_applies(const FieldArgs &a)
 {
     if (!a.angle || a.use_grad || a.cone || a.type_p) return false;
     const int r = a.radius < 1 ? 1 : a.radius, W = kGradTile + 2 * (r + 2 * a.smooth);
@@ -1068,7 +1068,7 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 
 // PLAIN: every trace weight of the launch is 1 and it holds all angle bins
 // (one chunk), so neither a weight nor a bin's range is tested per pair.
-template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool PLAIN>
+template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool PLAIN, bool PARTS>
 __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_MINB_UNSHARED) * 128 / (TZ * TX))
     k_sum(const __grid_constant__ SumArgs a)
 {
@@ -1110,13 +1110,19 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     // shot (receivers not shared), so that KB independent (shot, receiver)
     // gather chains are in flight per thread either way
     constexpr int KR = SHARED_R ? 1 : KB;
-    for (int blk = blockIdx.y; blk < a.nblk; blk += gridDim.y) {
+    // (rows beyond the blocks: each block's list in as many parts, PARTS)
+    for (int blk = PARTS ? blockIdx.y / a.parts : blockIdx.y; blk < a.nblk; blk += PARTS ? a.nblk : gridDim.y) {
         // the block's receivers with a pair that may reach this tile, in
         // order, each with the shots it may do so with (k_cull)
         const size_t lb = (size_t)blockIdx.x * a.nblk + blk;
-        const int cnt = __ldg(a.cnt + lb);
-        if (cnt == 0) continue;
+        int cnt = __ldg(a.cnt + lb);
         const unsigned *lst = a.list + lb * a.nh;
+        if (PARTS) {
+            const int part = blockIdx.y % a.parts, lo = cnt * part / a.parts;
+            cnt = cnt * (part + 1) / a.parts - lo;
+            lst += lo;
+        }
+        if (cnt == 0) continue;
         const int sb = blk * KB;
         double2 sTP[KB];
         float2 sXW[KB];
@@ -1429,11 +1435,17 @@ __global__ void k_sum_reduce(float *image, const float *partial, int nsplit, siz
 // {direction lo, hi, time lo, hi} of leg j over tile t, at [t][j]; a tile
 // without a usable point gets an empty time range.  One warp per (tile, leg).
 template <int TZ, int TX>
-__global__ void __launch_bounds__(256) k_leg_bounds(const double2 *TP, const float2 *XW, int nlegs, int nz, int nx,
-                                                    int angle, float4 *out, int stride, int first)
+__global__ void __launch_bounds__(256) k_leg_bounds(const double2 *RTP, const float2 *RXW, int nr, const double2 *STP,
+                                                    const float2 *SXW, int nlegs, int nz, int nx, int angle,
+                                                    float4 *out, int leg0)
 {
-    const int lane = threadIdx.x & 31, j = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (j >= nlegs) return;
+    const int lane = threadIdx.x & 31, jj = leg0 + blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (jj >= nlegs) return;
+    // receivers' legs first, then the sources' own
+    const bool rcv = jj < nr;
+    const int j = rcv ? jj : jj - nr;
+    const double2 *TP = rcv ? RTP : STP;
+    const float2 *XW = rcv ? RXW : SXW;
     const int tiles_z = (nz + TZ - 1) / TZ, tz = blockIdx.x % tiles_z, tx = blockIdx.x / tiles_z;
     const size_t base = (size_t)j * nz * nx;
     float pl = INFINITY, ph = -INFINITY, tl = INFINITY, th = -INFINITY;
@@ -1458,7 +1470,7 @@ __global__ void __launch_bounds__(256) k_leg_bounds(const double2 *TP, const flo
         tl = fminf(tl, __shfl_xor_sync(0xffffffffu, tl, o));
         th = fmaxf(th, __shfl_xor_sync(0xffffffffu, th, o));
     }
-    if (lane == 0) out[(size_t)blockIdx.x * stride + first + j] = make_float4(pl, ph, tl, th);
+    if (lane == 0) out[(size_t)blockIdx.x * nlegs + jj] = make_float4(pl, ph, tl, th);
 }
 
 // whether a pair of legs may contribute somewhere in the tile
@@ -1487,20 +1499,20 @@ __device__ __forceinline__ bool cull_keep(const SumArgs &a, float4 s, float4 r, 
 // reciprocal traces migrated with an earlier shot group (struct Fold).
 template <int KB>
 __global__ void __launch_bounds__(256) k_cull(const __grid_constant__ SumArgs a, const float4 *bs, const float4 *br,
-                                              int ns_stride, int nr_stride, int ntiles, unsigned *list, int *cnt)
+                                              int nlegs, int ntiles, unsigned *list, int *cnt)
 {
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (w >= (long long)ntiles * a.nblk) return;
     const int tile = (int)(w / a.nblk), blk = (int)(w % a.nblk), sb = blk * KB;
-    const float4 *R = br + (size_t)tile * nr_stride;
+    const float4 *R = br + (size_t)tile * nlegs;
     float4 S[KB];
     float top[KB];
     int nr[KB];
 #pragma unroll
     for (int k = 0; k < KB; k++) {
         const bool live = sb + k < a.nsb;
-        S[k] = live ? __ldg(bs + (size_t)tile * ns_stride + sb + k) : make_float4(0.f, 0.f, INFINITY, -INFINITY);
+        S[k] = live ? __ldg(bs + (size_t)tile * nlegs + sb + k) : make_float4(0.f, 0.f, INFINITY, -INFINITY);
         top[k] = a.stop && live ? __ldg(a.stop + sb + k) : (float)a.top;
         nr[k] = !live ? 0 : a.snh ? __ldg(a.snh + sb + k) : a.nh;
     }
@@ -1545,8 +1557,9 @@ static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 {
     constexpr int P = TZ * TX;
     const size_t sm = (size_t)nb * P * sizeof(float);
-    auto kern = k_sum<TZ, TX, KB, SR, MODE, false>;
-    if (MODE <= 1 && a.unit_tw && nb == a.ng) kern = k_sum<TZ, TX, KB, SR, MODE, MODE <= 1>;
+    const bool plain = MODE <= 1 && a.unit_tw && nb == a.ng;
+    auto kern = plain ? k_sum<TZ, TX, KB, SR, MODE, MODE <= 1, false> : k_sum<TZ, TX, KB, SR, MODE, false, false>;
+    if (a.parts > 1) kern = plain ? k_sum<TZ, TX, KB, SR, MODE, MODE <= 1, true> : k_sum<TZ, TX, KB, SR, MODE, false, true>;
     // all of the unified L1/shared memory as shared: the accumulators of as
     // many CTAs as the registers allow (the driver's own choice held 8x8
     // tiles to 10 CTAs per SM)
@@ -1627,15 +1640,11 @@ size_t sum_cull_bytes(int nz, int nx, int nsb, int nh, int nrl, int ng, int tile
 }
 
 template <int TZ, int TX>
-static int launch_bounds_t(const SumArgs &a, const double2 *TP, const float2 *XW, int n, float4 *out, int tiles,
-                           int stride, int first, cudaStream_t st)
+static int launch_bounds_t(const SumArgs &a, int nlegs, float4 *out, int tiles, cudaStream_t st)
 {
-    for (int j0 = 0; j0 < n; j0 += 8 * 65535) {
-        const int nj = std::min(n - j0, 8 * 65535);
-        const size_t o = (size_t)j0 * a.nz * a.nx;
-        k_leg_bounds<TZ, TX><<<dim3(tiles, (nj + 7) / 8), 256, 0, st>>>(TP + o, XW + o, nj, a.nz, a.nx, a.mode < 2, out,
-                                                                       stride, first + j0);
-    }
+    for (int j0 = 0; j0 < nlegs; j0 += 8 * 65535)
+        k_leg_bounds<TZ, TX><<<dim3(tiles, std::min(65535, (nlegs - j0 + 7) / 8)), 256, 0, st>>>(
+            a.RTP, a.RXW, a.nrl, a.STP, a.SXW, nlegs, a.nz, a.nx, a.mode < 2, out, j0);
     KCIG_CUDA(cudaGetLastError());
     return KCIG_OK;
 }
@@ -1663,23 +1672,20 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         const size_t nzx = (size_t)a.nz * a.nx;
         const ptrdiff_t off = (a.STP - a.RTP) / (ptrdiff_t)nzx;
         const bool alias = a.shared_r && a.STP >= a.RTP && off + a.nsb <= a.nrl;
-        float4 *br = reinterpret_cast<float4 *>(a.cull), *bs = alias ? br + off : br + (size_t)tiles * a.nrl;
-        const int ss = alias ? a.nrl : a.nsb;
-        int *cnt = reinterpret_cast<int *>(br + (size_t)tiles * (a.nrl + (alias ? 0 : a.nsb)));
+        const int nlegs = a.nrl + (alias ? 0 : a.nsb);
+        float4 *br = reinterpret_cast<float4 *>(a.cull), *bs = br + (alias ? off : a.nrl);
+        int *cnt = reinterpret_cast<int *>(br + (size_t)tiles * nlegs);
         unsigned *list = reinterpret_cast<unsigned *>(cnt) + (size_t)tiles * a.nblk;
-        auto bounds = [&](const double2 *TP, const float2 *XW, int n, float4 *out, int stride) -> int {
-            if (tz == 16) return launch_bounds_t<16, 8>(a, TP, XW, n, out, tiles, stride, 0, st);
-            if (tx == 16) return launch_bounds_t<8, 16>(a, TP, XW, n, out, tiles, stride, 0, st);
-            return launch_bounds_t<8, 8>(a, TP, XW, n, out, tiles, stride, 0, st);
-        };
-        KCIG_TRY(bounds(a.RTP, a.RXW, a.nrl, br, a.nrl));
-        if (!alias) KCIG_TRY(bounds(a.STP, a.SXW, a.nsb, bs, ss));
+        if (tz == 16) KCIG_TRY((launch_bounds_t<16, 8>(a, nlegs, br, tiles, st)));
+        else if (tx == 16) KCIG_TRY((launch_bounds_t<8, 16>(a, nlegs, br, tiles, st)));
+        else KCIG_TRY((launch_bounds_t<8, 8>(a, nlegs, br, tiles, st)));
         const unsigned grid = (unsigned)(((long long)tiles * a.nblk + 7) / 8);
-        if (kb == 4) k_cull<4><<<grid, 256, 0, st>>>(a, bs, br, ss, a.nrl, tiles, list, cnt);
-        else k_cull<2><<<grid, 256, 0, st>>>(a, bs, br, ss, a.nrl, tiles, list, cnt);
+        if (kb == 4) k_cull<4><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
+        else k_cull<2><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
         KCIG_CUDA(cudaGetLastError());
         a.cnt = cnt;
         a.list = list;
+        a.parts = a.nsplit > a.nblk ? a.nsplit / a.nblk : 1;
         int rc;
         const bool fits128 = (size_t)nb * 128 * 4 <= 200 * 1024;
         if (a.tile == 1 && fits128) rc = launch_sum_mode<16, 8, 4>(a, nb, st);
@@ -1690,7 +1696,7 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         else rc = launch_sum_mode<8, 8, KCIG_KB>(a, nb, st);
         if (rc) return rc;
         if (launches) (*launches)++;
-        if (aux) *aux += alias ? 2 : 3;
+        if (aux) *aux += 2;
     }
     if (a0.nsplit > 1) {
         const size_t n = (size_t)a0.ng * a0.nz * a0.nx;
@@ -1715,7 +1721,7 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
 #define KCIG_SPLIT_WAVES 8
 #endif
 
-int sum_nsplit(int nz, int nx, int nsb, bool shared_r)
+int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
 {
     static int sms = 0;
     if (!sms) {
@@ -1726,6 +1732,13 @@ int sum_nsplit(int nz, int nx, int nsb, bool shared_r)
     const long long tiles = (long long)((nz + 15) / 16) * ((nx + 7) / 8);
     const long long slots = (long long)sms * KCIG_SUM_MINB;  // resident CTAs of one wave
     const int blocks = shared_r ? (nsb + KCIG_KB - 1) / KCIG_KB : (nsb + KCIG_KB_UNSHARED - 1) / KCIG_KB_UNSHARED;
+    // a grid whose blocks, one a row, leave half the slots empty: the blocks'
+    // receiver lists in parts, of four receivers or more (the test line of 33
+    // tiles, 2 blocks and 21 receivers: k_sum 43 -> 17 us in five parts)
+    if (tiles * blocks * 2 <= slots) {
+        const long long parts = std::min<long long>(8, std::min<long long>(slots / (tiles * blocks), nh / 4));
+        return blocks * (int)std::max<long long>(1, parts);
+    }
     if (tiles >= (long long)KCIG_SPLIT_BELOW * slots) {
         // fill(n): the waves of n parts over whole waves
         auto fill = [&](int n) {

@@ -324,33 +324,37 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
     }
     if (P->stream_tables && !tab)
         return set_error(KCIG_ERR_UNSUPPORTED, "tables kept in host memory need the host-side leg path");
-    const int FB = field_batch(P, (size_t)n);
-    if (angle) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
+    FieldArgs a;
+    memset(&a, 0, sizeof a);
+    a.tab = tab ? tab : (is_source ? P->stab : P->rtab);
+    a.der = der ? der : (is_source ? P->sder : P->rder);
+    a.gxv = is_source ? P->sgx : P->rgx;
+    a.gzv = is_source ? P->sgz : P->rgz;
+    a.nz = g.nz;
+    a.nx = g.nx;
+    a.dz = g.dz;
+    a.dx = g.dx;
+    a.x0 = g.x0;
+    a.radius = P->p.angle_grad_radius;
+    a.smooth = P->p.angle_smooth;
+    a.angle = angle;
+    a.use_grad = P->sgx != nullptr;
+    a.aper = P->p.aperture;
+    a.aper_taper = P->p.aperture_taper;
+    a.rmin = P->p.aperture_rmin;
+    a.rtaper = P->p.aperture_rtaper;
+    a.apb = aperture_bounds(a.aper, a.aper_taper);
+    a.cone = P->p.tool == 1;
+    a.status = P->d_status.as<int>();
+    a.type_p = P->p.interp_type == 'p';
+    // the one-pass kernel takes every leg in one launch; the staged kernels go
+    // in batches of their work planes
+    const bool one = leg_tile_applies(a);
+    const int FB = one ? std::min(n, 65535) : field_batch(P, (size_t)n);
+    if (angle && !one) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
     for (int j0 = 0; j0 < n; j0 += FB) {
-        FieldArgs a;
-        a.tab = tab ? tab : (is_source ? P->stab : P->rtab);
-        a.der = der ? der : (is_source ? P->sder : P->rder);
-        a.gxv = is_source ? P->sgx : P->rgx;
-        a.gzv = is_source ? P->sgz : P->rgz;
         a.legs = d_legs + j0;
         a.n = std::min(FB, n - j0);
-        a.nz = g.nz;
-        a.nx = g.nx;
-        a.dz = g.dz;
-        a.dx = g.dx;
-        a.x0 = g.x0;
-        a.radius = P->p.angle_grad_radius;
-        a.smooth = P->p.angle_smooth;
-        a.angle = angle;
-        a.use_grad = P->sgx != nullptr;
-        a.aper = P->p.aperture;
-        a.aper_taper = P->p.aperture_taper;
-        a.rmin = P->p.aperture_rmin;
-        a.rtaper = P->p.aperture_rtaper;
-        a.apb = aperture_bounds(a.aper, a.aper_taper);
-        a.cone = P->p.tool == 1;
-        a.status = P->d_status.as<int>();
-        a.type_p = P->p.interp_type == 'p';
         LegFields out{TP + (size_t)j0 * nzx, XW + (size_t)j0 * nzx};
         int nl = 0;
         KCIG_TRY(launch_leg_fields(a, out, P->d_work.as<double>(), P->st, &nl));
@@ -776,14 +780,19 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     // every shot's fields are among the receivers' when those are all resident
     const bool alias_src = all_on_receivers && nhc == g.nh;
 
+    // one batch, both sides from the same tables: the sources' legs follow the
+    // receivers' in one buffer and one launch (two launches of a small grid
+    // leave it half empty)
+    const bool joint = shared_r && !alias_src && nhc == g.nh && nsb == ns && same_sides(P) && !P->stream_tables &&
+                       !P->sg_src;
     if (shared_r) {
-        KCIG_TRY(P->d_rT.ensure((size_t)nhc * nzx * sizeof(double2)));
-        KCIG_TRY(P->d_rF.ensure((size_t)nhc * nzx * sizeof(float2)));
+        KCIG_TRY(P->d_rT.ensure((size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(double2)));
+        KCIG_TRY(P->d_rF.ensure((size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(float2)));
     } else {
         KCIG_TRY(P->d_rT.ensure((size_t)nsb * g.nh * nzx * sizeof(double2)));
         KCIG_TRY(P->d_rF.ensure((size_t)nsb * g.nh * nzx * sizeof(float2)));
     }
-    if (!alias_src) {
+    if (!alias_src && !joint) {
         KCIG_TRY(P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2)));
         KCIG_TRY(P->d_sF.ensure((size_t)nsb * nzx * sizeof(float2)));
     }
@@ -819,7 +828,8 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     for (int r0 = 0; r0 < g.nh && rc == KCIG_OK; r0 += nhc) {
         const int nhb = std::min(nhc, g.nh - r0);
         if (shared_r) {
-            const std::vector<LegInterp> rl(rlegs.begin() + r0, rlegs.begin() + r0 + nhb);
+            std::vector<LegInterp> rl(rlegs.begin() + r0, rlegs.begin() + r0 + nhb);
+            if (joint) rl.insert(rl.end(), slegs.begin(), slegs.end());
             rc = fields(0, rl, P->d_rT.as<double2>(), P->d_rF.as<float2>());
             if (rc) break;
         }
@@ -827,9 +837,10 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             const int nsh = std::min(nsb, ns - s0);
             const double2 *sT = P->d_sT.as<double2>();
             const float2 *sF = P->d_sF.as<float2>();
-            if (alias_src) {
-                sT = P->d_rT.as<double2>() + (size_t)(s0 + fold.off) * nzx;
-                sF = P->d_rF.as<float2>() + (size_t)(s0 + fold.off) * nzx;
+            if (alias_src || joint) {
+                const int leg0 = joint ? nhc : s0 + fold.off;
+                sT = P->d_rT.as<double2>() + (size_t)leg0 * nzx;
+                sF = P->d_rF.as<float2>() + (size_t)leg0 * nzx;
             } else {
                 std::vector<LegInterp> sl(slegs.begin() + s0, slegs.begin() + s0 + nsh);
                 rc = fields(1, sl, P->d_sT.as<double2>(), P->d_sF.as<float2>());
@@ -946,7 +957,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.unit_tw = sa.unit_all ||
                          std::all_of(h_trw.begin(), h_trw.begin() + nb, [](float v) { return v == 1.0f || v == 0.0f; });
             sa.tile = P->tile;
-            sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, shared_r);
+            sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, nhb, shared_r);
             if (sa.nsplit > 1) {
                 rc = P->d_part.ensure((size_t)sa.nsplit * P->ng * nzx * sizeof(float));
                 if (rc) break;
@@ -1347,7 +1358,7 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.stop = S->stop.as<float>() + B.shot0;
     sa.snh = S->snh.as<int>() + B.shot0;
     sa.tile = P->tile;
-    sa.nsplit = sum_nsplit(g.nz, g.nx, B.ns, false);
+    sa.nsplit = sum_nsplit(g.nz, g.nx, B.ns, B.nhb, false);
     if (sa.nsplit > 1) sa.partial = P->d_part.as<float>();  // sized by kcig_shots_prepare
     sa.image = d_img;
     sa.zero_init = b == 0 ? 1 : 0;
@@ -1599,7 +1610,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
     if (!rc && angle && !(P->sg_src && P->sg_rcv))
         rc = P->d_work.ensure((size_t)field_batch(P, std::max(max_s, max_r)) * 4 * nzx * sizeof(double));
     int max_split = 1;
-    for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, false));
+    for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, B.nhb, false));
     if (!rc && max_split > 1) rc = P->d_part.ensure((size_t)max_split * P->ng * nzx * sizeof(float));
     size_t cull = 0;
     for (const ShotBatch &B : S->batches)
