@@ -77,7 +77,22 @@ struct FieldArgs {
     int cone;  // kirchmig2d: the w field holds the leg's two cone flags (see k_leg_interp)
     int *status;  // device flag a kernel sets when a bounded wait gives up (may be null)
     int type_p;   // the legs use the partial-shift interpolation ('p')
+    // one-pass kernel: [n][tiles] whether any pair of the leg may end within
+    // the record in that block of points (null: all of them)
+    const unsigned char *need;
 };
+
+// Which blocks of points of which legs are needed: receivers' legs 0 .. nr - 1,
+// the sources' among them from src0 (src0 + ns <= nr) or after them (src0 =
+// nr).  A pair's centre time may not pass `end`.
+struct NeedArgs {
+    int nr, src0, ns;
+    double end;
+};
+// tmin: scratch of n * leg_tiles floats, need: n * leg_tiles bytes
+int launch_leg_need(const FieldArgs &a, const NeedArgs &q, float *tmin, unsigned char *need, cudaStream_t st);
+int leg_tiles(int nz, int nx);  // blocks of points of a leg
+
 
 // Workspace for the gradient pipeline: 4 double planes per position.
 int launch_leg_fields(const FieldArgs &a, LegFields out, double *work, cudaStream_t st, int *launches = nullptr);
@@ -176,6 +191,7 @@ struct SumArgs {
     int shot0, rcv0;       // first shot and receiver of the batch in the call
     double uk, ub, utop, uhi, top;  // set by launch_sum: u = theta uk + ub, ng - 1 (+ 1e-5), nt - 1
     void *cull;            // scratch of sum_cull_bytes
+    const unsigned char *need_r, *need_s;  // [legs][leg_tiles] blocks whose fields exist, or null (all)
     int nrl;               // receiver legs (RTP, RXW)
     int unit_all;          // every trace weight is 1, none is 0 (unit_tw: every one that is not 0)
     int parts;             // set by launch_sum: parts of a block's list (rows of CTAs beyond the blocks)

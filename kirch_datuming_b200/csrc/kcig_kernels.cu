@@ -788,6 +788,7 @@ __global__ void __launch_bounds__(256, 3) k_leg_tile(FieldArgs a, LegFields out)
     const int r = a.radius < 1 ? 1 : a.radius, s = a.smooth;
     const int H = r + 2 * s, W = kGradTile + 2 * H, SW = leg_tile_pitch(W);
     const int tiles_z = (nz + kGradTile - 1) / kGradTile;
+    if (a.need && !a.need[(size_t)blockIdx.y * gridDim.x + blockIdx.x]) return;
     const int gz0 = (int)(blockIdx.x % tiles_z) * kGradTile - H, gx0 = (int)(blockIdx.x / tiles_z) * kGradTile - H;
     const int zlo = max(0, -gz0), zhi = min(W, nz - gz0), xlo = max(0, -gx0), xhi = min(W, nx - gx0);
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
@@ -914,6 +915,87 @@ __global__ void __launch_bounds__(256, 3) k_leg_tile(FieldArgs a, LegFields out)
                                                                      : atan2(vz, vx);
             TPo[(size_t)(gx0 + lx) * nz + (gz0 + lz)].y = phi;
         }
+}
+
+int leg_tiles(int nz, int nx) { return ((nz + kGradTile - 1) / kGradTile) * ((nx + kGradTile - 1) / kGradTile); }
+
+// Least traveltime of every leg over every block of points (the values
+// k_leg_tile forms: the same interpolation), rounded down.
+__global__ void __launch_bounds__(256) k_leg_tmin(FieldArgs a, float *tmin)
+{
+    __shared__ float part[8];
+    const size_t nzx = (size_t)a.nz * a.nx;
+    const int tiles_z = (a.nz + kGradTile - 1) / kGradTile;
+    const int iz = (int)(blockIdx.x % tiles_z) * kGradTile + (int)threadIdx.x;
+    const int x0 = (int)(blockIdx.x / tiles_z) * kGradTile;
+    const LegInterp &L = a.legs[blockIdx.y];
+    const int i0 = L.i0, i1 = L.i1;
+    const double c0 = L.c[0], c1 = L.c[1], c2 = L.c[2], c3 = L.c[3];
+    float m = INFINITY;
+    if (iz < a.nz) {
+#pragma unroll
+        for (int q = 0; q < kGradTile / 8; q++) {
+            const int ix = x0 + (int)threadIdx.y + 8 * q;
+            if (ix >= a.nx) break;
+            const size_t i = (size_t)ix * a.nz + iz;
+            double T = a.tab[(size_t)i0 * nzx + i];
+            if (i1 >= 0)
+                T = c0 * T + c1 * a.der[(size_t)i0 * nzx + i] + c2 * a.tab[(size_t)i1 * nzx + i] +
+                    c3 * a.der[(size_t)i1 * nzx + i];
+            m = fminf(m, __double2float_rd(T));  // NaN times drop out
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) part[threadIdx.y] = m;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int w = 1; w < 8; w++) m = fminf(m, part[w]);
+        tmin[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = m;
+    }
+}
+
+// A leg is needed in a block of points if its least time there and the other
+// side's least end within the record: most legs of a survey much longer than
+// its records reach are not (struct NeedArgs).  One CTA per block of points.
+__global__ void __launch_bounds__(256) k_leg_need(const float *tmin, unsigned char *need, NeedArgs q, int n)
+{
+    __shared__ float mr[8], ms[8];
+    const int tiles = gridDim.x, t = blockIdx.x, warp = threadIdx.x >> 5;
+    float r = INFINITY, s = INFINITY;
+    for (int j = threadIdx.x; j < n; j += 256) {
+        const float v = tmin[(size_t)j * tiles + t];
+        if (j < q.nr) r = fminf(r, v);
+        if (j >= q.src0 && j < q.src0 + q.ns) s = fminf(s, v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        r = fminf(r, __shfl_xor_sync(0xffffffffu, r, o));
+        s = fminf(s, __shfl_xor_sync(0xffffffffu, s, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        mr[warp] = r;
+        ms[warp] = s;
+    }
+    __syncthreads();
+    for (int w = 0; w < 8; w++) {
+        r = w ? fminf(r, mr[w]) : mr[0];
+        s = w ? fminf(s, ms[w]) : ms[0];
+    }
+    for (int j = threadIdx.x; j < n; j += 256) {
+        const double v = tmin[(size_t)j * tiles + t];
+        const bool as_r = j < q.nr && v + (double)s <= q.end, as_s = j >= q.src0 && j < q.src0 + q.ns && v + (double)r <= q.end;
+        need[(size_t)j * tiles + t] = as_r || as_s;
+    }
+}
+
+int launch_leg_need(const FieldArgs &a, const NeedArgs &q, float *tmin, unsigned char *need, cudaStream_t st)
+{
+    const int tiles = leg_tiles(a.nz, a.nx);
+    k_leg_tmin<<<dim3(tiles, a.n), dim3(32, 8), 0, st>>>(a, tmin);
+    k_leg_need<<<tiles, 256, 0, st>>>(tmin, need, q, a.n);
+    KCIG_CUDA(cudaGetLastError());
+    return KCIG_OK;
 }
 
 int launch_leg_interp(const FieldArgs &a, LegFields out, double *work, cudaStream_t st, int *launches)
@@ -1437,7 +1519,8 @@ __global__ void k_sum_reduce(float *image, const float *partial, int nsplit, siz
 template <int TZ, int TX>
 __global__ void __launch_bounds__(256) k_leg_bounds(const double2 *RTP, const float2 *RXW, int nr, const double2 *STP,
                                                     const float2 *SXW, int nlegs, int nz, int nx, int angle,
-                                                    float4 *out, int leg0)
+                                                    float4 *out, int leg0, const unsigned char *need_r,
+                                                    const unsigned char *need_s)
 {
     const int lane = threadIdx.x & 31, jj = leg0 + blockIdx.y * 8 + (threadIdx.x >> 5);
     if (jj >= nlegs) return;
@@ -1447,6 +1530,14 @@ __global__ void __launch_bounds__(256) k_leg_bounds(const double2 *RTP, const fl
     const double2 *TP = rcv ? RTP : STP;
     const float2 *XW = rcv ? RXW : SXW;
     const int tiles_z = (nz + TZ - 1) / TZ, tz = blockIdx.x % tiles_z, tx = blockIdx.x / tiles_z;
+    if (const unsigned char *need = rcv ? need_r : need_s) {  // the leg's fields may not exist here
+        const int nbz = (nz + kGradTile - 1) / kGradTile, nb = nbz * ((nx + kGradTile - 1) / kGradTile);
+        if (!need[(size_t)j * nb + tz * TZ / kGradTile + tx * TX / kGradTile * nbz]) {
+            if (lane == 0)
+                out[(size_t)blockIdx.x * nlegs + jj] = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+            return;
+        }
+    }
     const size_t base = (size_t)j * nz * nx;
     float pl = INFINITY, ph = -INFINITY, tl = INFINITY, th = -INFINITY;
 #pragma unroll
@@ -1644,7 +1735,7 @@ static int launch_bounds_t(const SumArgs &a, int nlegs, float4 *out, int tiles, 
 {
     for (int j0 = 0; j0 < nlegs; j0 += 8 * 65535)
         k_leg_bounds<TZ, TX><<<dim3(tiles, std::min(65535, (nlegs - j0 + 7) / 8)), 256, 0, st>>>(
-            a.RTP, a.RXW, a.nrl, a.STP, a.SXW, nlegs, a.nz, a.nx, a.mode < 2, out, j0);
+            a.RTP, a.RXW, a.nrl, a.STP, a.SXW, nlegs, a.nz, a.nx, a.mode < 2, out, j0, a.need_r, a.need_s);
     KCIG_CUDA(cudaGetLastError());
     return KCIG_OK;
 }

@@ -59,6 +59,9 @@ struct kcig_plan {
     DevBuf own_stab, own_sder, own_rtab, own_rder, own_sgx, own_sgz, own_rgx, own_rgz;
     DevBuf d_data, d_image, d_rT, d_rF, d_sT, d_sF, d_work, d_D, d_legs, d_tr;
     DevBuf d_part;  // partial images of a split summation (small grids)
+    DevBuf d_need;  // which blocks of points of which legs are needed, and their least times
+    NeedArgs need_args = {0, 0, 0, 0.0};  // of the legs computed next (nr = 0: all needed)
+    const unsigned char *need = nullptr;  // the last legs' flags (null: all their fields exist)
     DevBuf d_cull;  // the summation's lists of pairs that may reach a tile
     DevBuf d_status;  // flag of the leg-field kernels' bounded waits (k_leg_tile)
     // tables left in host memory (KCIG_MEM_HOST_STREAM): the slices of each
@@ -352,6 +355,17 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
     const bool one = leg_tile_applies(a);
     const int FB = one ? std::min(n, 65535) : field_batch(P, (size_t)n);
     if (angle && !one) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
+    P->need = nullptr;
+    if (P->need_args.nr > 0 && one && n <= FB) {
+        const size_t cells = (size_t)n * leg_tiles(g.nz, g.nx);
+        KCIG_TRY(P->d_need.ensure(cells * (sizeof(float) + 1)));
+        unsigned char *need = P->d_need.as<unsigned char>() + cells * sizeof(float);
+        a.legs = d_legs;
+        a.n = n;
+        KCIG_TRY(launch_leg_need(a, P->need_args, P->d_need.as<float>(), need, P->st));
+        P->all_launches += 2;
+        P->need = a.need = need;
+    }
     for (int j0 = 0; j0 < n; j0 += FB) {
         a.legs = d_legs + j0;
         a.n = std::min(FB, n - j0);
@@ -468,7 +482,7 @@ extern "C" int kcig_plan_destroy(kcig_plan *P)
     DevBuf *bufs[] = {&P->own_stab, &P->own_sder, &P->own_rtab, &P->own_rder, &P->own_sgx, &P->own_sgz,
                       &P->own_rgx,  &P->own_rgz,  &P->d_data,   &P->d_image,  &P->d_rT,   &P->d_rF,
                       &P->d_sT,     &P->d_sF,   &P->d_work,   &P->d_D,      &P->d_legs, &P->d_tr,
-                      &P->d_part,   &P->d_stage, &P->d_cull};
+                      &P->d_part,   &P->d_stage, &P->d_cull, &P->d_need};
     for (DevBuf *b : bufs) b->release();
     release_shots(P);
     if (P->own_st) cudaStreamDestroy(P->own_st);
@@ -819,6 +833,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
         cudaEventRecord(f1, st);
         return r;
     };
+    const unsigned char *need = nullptr;  // of the receivers' legs (and the sources' with them)
     bool first = true;
     std::vector<float> h_trw(trn);
     std::vector<int> h_rfi(trn), h_igo(trn);
@@ -830,8 +845,21 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
         if (shared_r) {
             std::vector<LegInterp> rl(rlegs.begin() + r0, rlegs.begin() + r0 + nhb);
             if (joint) rl.insert(rl.end(), slegs.begin(), slegs.end());
+            // both sides' legs at hand: blocks of points that no pair of a leg
+            // reaches within the record are left out (two samples of margin).
+            // Small grids compute them all: two launches cost more.
+            if ((joint || (alias_src && nsb == ns)) && !P->stream_tables && !P->sg_src &&
+                (size_t)rl.size() * nzx >= ((size_t)32 << 20)) {
+                P->need_args.nr = nhb;
+                P->need_args.src0 = joint ? nhb : fold.off;
+                P->need_args.ns = ns;
+                const double end = ((double)g.nt + 1.0) * (double)g.dt + (double)g.t0 - (double)p.tau;
+                P->need_args.end = end + 1e-6 * fabs(end);
+            }
             rc = fields(0, rl, P->d_rT.as<double2>(), P->d_rF.as<float2>());
+            P->need_args.nr = 0;
             if (rc) break;
+            need = P->need;
         }
         for (int s0 = 0; s0 < ns && rc == KCIG_OK; s0 += nsb) {
             const int nsh = std::min(nsb, ns - s0);
@@ -934,6 +962,8 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.shot0 = s0;
             sa.rcv0 = r0;
             sa.nrl = shared_r ? nhb : (int)rl.size();
+            sa.need_r = need;
+            if (need) sa.need_s = need + (size_t)(joint ? nhb : s0 + fold.off) * leg_tiles(g.nz, g.nx);
             rc = P->d_cull.ensure(sum_cull_bytes(g.nz, g.nx, nsh, nhb, sa.nrl, P->ng, P->tile, shared_r));
             if (rc) break;
             sa.cull = P->d_cull.p;
