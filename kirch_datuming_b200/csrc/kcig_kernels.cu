@@ -1823,13 +1823,6 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
     const long long tiles = (long long)((nz + 15) / 16) * ((nx + 7) / 8);
     const long long slots = (long long)sms * KCIG_SUM_MINB;  // resident CTAs of one wave
     const int blocks = shared_r ? (nsb + KCIG_KB - 1) / KCIG_KB : (nsb + KCIG_KB_UNSHARED - 1) / KCIG_KB_UNSHARED;
-    // a grid whose blocks, one a row, leave half the slots empty: the blocks'
-    // receiver lists in parts, of four receivers or more (the test line of 33
-    // tiles, 2 blocks and 21 receivers: k_sum 43 -> 17 us in five parts)
-    if (tiles * blocks * 2 <= slots) {
-        const long long parts = std::min<long long>(8, std::min<long long>(slots / (tiles * blocks), nh / 4));
-        return blocks * (int)std::max<long long>(1, parts);
-    }
     if (tiles >= (long long)KCIG_SPLIT_BELOW * slots) {
         // fill(n): the waves of n parts over whole waves
         auto fill = [&](int n) {
@@ -1848,18 +1841,31 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
         // v(z) 201 x 401 survey (663 tiles, 16 blocks): 16 parts of one block
         // each, 11 units, against 13 parts (the 8-wave aim) at 9 x 2 = 18 --
         // measured 4.80 -> 4.42 ms
-        long long best = 1, cost = -1;
-        for (long long n = 1; n <= std::min(blocks, 64); n++) {
-            const long long c = ((n * tiles + slots - 1) / slots) * ((blocks + n - 1) / n);
-            if (cost < 0 || 20 * c < 19 * cost) {
+        // Blocks one a row may go on in parts of their receiver lists, of four
+        // receivers or more: a row then lasts 1 / parts of a block (41 x 81
+        // points, 2 blocks of 21 receivers: k_sum 43 -> 17 us in five parts;
+        // 43 x 172 points, 9 blocks of 202: 721 -> 373 us in five); from three
+        // waves on the set-up of more rows costs what the last wave gains (the
+        // v(z) survey in 48 rows: 2.64 -> 3.02 ms)
+        long long best = 1;
+        double cost = -1.0;
+        auto offer = [&](long long rows, double length) {
+            const double c = (double)((rows * tiles + slots - 1) / slots) * length;
+            if (cost < 0.0 || 20.0 * c < 19.0 * cost) {
                 cost = c;
-                best = n;
+                best = rows;
             }
-        }
+        };
+        for (long long n = 1; n <= std::min(blocks, 64); n++) offer(n, (double)((blocks + n - 1) / n));
+        if (blocks * tiles < 3 * slots)
+            for (int p = 2; p <= std::min(8, nh / 4) && (long long)p * blocks <= 64; p++)
+                offer((long long)p * blocks, 1.0 / p);
         return (int)best;
     }
     const long long want = (long long)KCIG_SPLIT_WAVES * slots;
     long long ns = (want + tiles - 1) / tiles;
+    if (ns >= 2LL * blocks && nh >= 8)  // too few blocks: their lists in parts
+        return blocks * (int)std::max<long long>(1, std::min<long long>(std::min(8, nh / 4), std::min<long long>(ns, 64) / blocks));
     ns = std::min<long long>(ns, std::min(blocks, 64));
     return (int)std::max<long long>(1, ns);
 }
