@@ -220,8 +220,15 @@ struct SprayArgs {
     int mode;              // 0 angle two-bin, 1 angle nearest, 2 single bin
     double t0, inv_dt, tau, deg, ug0, uinv;
     float aal, oazmin, oazmax, oaztaper, ats, ate;
+    int nrl;               // receiver legs (RTP, RXW)
+    void *scratch;         // spray_scratch_bytes
+    // set by launch_spray
+    SumArgs cull;          // what the pair bounds read
+    int nlegs;
+    const float4 *bounds;  // [tiles][receivers' legs, shots' legs]
 };
 int launch_spray(const SprayArgs &a, cudaStream_t st);
+size_t spray_scratch_bytes(int nz, int nx, int nsb, int nrl);
 int launch_doubint_f32(const double *in, float *out, int ntr, int nt, cudaStream_t st);
 
 // Gives back the memory kcig_eikods keeps between calls on the current device.

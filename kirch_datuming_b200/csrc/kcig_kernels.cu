@@ -16,6 +16,7 @@
 // SERECKIRCH/src/tinterpsr.cpp (:37-188).
 #include <math.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <algorithm>
 #include <map>
@@ -1371,129 +1372,6 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     for (int b = 0; b < nb; b++) out[(size_t)(gc0 + b) * nzx + i] = acc[b * P + tid];
 }
 
-// ------------------------------------------------------- forward modelling --
-// kirchmig2d_cig adj=0 (:1300-1312, kirmig.cpp:59-68): one CTA per shot and
-// block of RB receivers, the RB traces accumulated in shared memory in FP64
-// (the trace is integrated twice afterwards, which would amplify FP32
-// accumulation error; threads sweep the image points, and neighbouring points
-// land on different samples), the same gates, weights and pick positions as
-// k_sum.
-template <int MODE, int RB>
-__global__ void __launch_bounds__(256) k_spray(const __grid_constant__ SprayArgs a)
-{
-    constexpr double kPiD = 3.141592653589793238463, kTwoPi = 6.283185307179586476925;
-    extern __shared__ double tr[];  // [RB][nt]
-    const int nrb = (a.nh + RB - 1) / RB;
-    const int k = blockIdx.x / nrb, r0 = (blockIdx.x % nrb) * RB;
-    const int nr = min(RB, a.nh - r0);
-    for (int q = threadIdx.x; q < RB * a.nt; q += blockDim.x) tr[q] = 0.0;
-    float tw[RB];
-    int ri[RB], ig[RB];
-#pragma unroll
-    for (int j = 0; j < RB; j++) {
-        const int trc = k * a.nh + r0 + j;
-        tw[j] = j < nr ? __ldg(a.trw + trc) : 0.0f;
-        ri[j] = j < nr ? __ldg(a.rfi + trc) : 0;
-        ig[j] = j < nr ? __ldg(a.igo + trc) : 0;
-    }
-    __syncthreads();
-    const int nzx = a.nz * a.nx;
-    const double top = (double)(a.nt - 1);
-    const double ulo = -1.0e-5, uhi = (double)(a.ng - 1) + 1.0e-5;
-    const double uk = a.deg * a.uinv, ub = a.ug0 * a.uinv;
-    for (int i = threadIdx.x; i < nzx; i += blockDim.x) {
-        const double2 sTP = __ldg(a.STP + (size_t)k * nzx + i);
-        const float2 sXW = __ldg(a.SXW + (size_t)k * nzx + i);
-        if (!(sXW.y > 0.0f)) continue;
-        const int iz = i % a.nz;
-        const float zf = (a.nz > 1) ? (float)iz / (float)(a.nz - 1) : 0.0f;
-        const float cutoff = a.oazmin + zf * (a.oazmax - a.oazmin);
-#pragma unroll
-        for (int j = 0; j < RB; j++) {
-            if (tw[j] == 0.0f) continue;
-            const double2 rTP = __ldg(a.RTP + (size_t)ri[j] * nzx + i);
-            const float2 rXW = __ldg(a.RXW + (size_t)ri[j] * nzx + i);
-            const float apw = sXW.y * rXW.y;
-            if (!(apw > 0.0f)) continue;
-            int b0 = 0;
-            float w0 = 1.0f, w1 = 0.0f, aw;
-            if (MODE == 2) {
-                b0 = ig[j];
-                aw = tw[j] * apw;
-            } else {
-                double th = fabs(sTP.y - rTP.y);
-                th = (th > kPiD) ? kTwoPi - th : th;
-                const double u = fma(th, uk, -ub);
-                double fl;
-                if (MODE == 0) {
-                    if (!(u >= ulo && u <= uhi)) continue;
-                    fl = floor(u);
-                } else {
-                    fl = floor(u + 0.5);
-                    if (!(fl >= 0.0 && fl < (double)a.ng)) continue;
-                }
-                const float ang = (float)(th * a.deg);
-                aw = taper_weight(ang, a.ats, a.ate) * depth_weight(ang, cutoff, a.oaztaper) * tw[j] * apw;
-                if (!(aw > 0.0f)) continue;
-                if (MODE == 0) {
-                    if (u <= 0.0) { b0 = 0; w0 = 1.0f; w1 = 0.0f; }
-                    else if (u >= (double)(a.ng - 1)) { b0 = a.ng - 1; w0 = 1.0f; w1 = 0.0f; }
-                    else {
-                        b0 = (int)fl;
-                        const double f1 = u - fl;
-                        w1 = (float)f1;
-                        w0 = (float)(1.0 - f1);
-                    }
-                } else {
-                    b0 = (int)fl;
-                }
-            }
-            const double ft0 = (sTP.x + rTP.x + a.tau - a.t0) * a.inv_dt;
-            const double sh = fma((double)(fmaxf(fabsf(sXW.x), fabsf(rXW.x)) * a.aal), a.inv_dt, 1.0);
-            const double ftm0 = ft0 - sh, ftp0 = ft0 + sh;
-            const double fl0 = floor(ft0), flm = floor(ftm0), flp = floor(ftp0);
-            if (!(fl0 >= 0.0 && fl0 < top && flm >= 0.0 && flm <= fl0 && flp >= fl0 && flp < top)) continue;
-            float val = w0 * __ldg(a.image + (size_t)b0 * nzx + i);
-            if (MODE == 0 && w1 > 0.0f) val += w1 * __ldg(a.image + (size_t)(b0 + 1) * nzx + i);
-            const float r1 = 1.0f / (1.0f + 2.0f * (float)sh);  // dt / (dt + tp - tm)
-            const double sv = (double)(r1 * r1 * (aw * val));
-            double *t = tr + j * a.nt;
-            const double f0 = ft0 - fl0, fm = ftm0 - flm, fp = ftp0 - flp;
-            atomicAdd(t + (int)fl0, 2.0 * (1.0 - f0) * sv);
-            atomicAdd(t + (int)fl0 + 1, 2.0 * f0 * sv);
-            atomicAdd(t + (int)flm, -(1.0 - fm) * sv);
-            atomicAdd(t + (int)flm + 1, -fm * sv);
-            atomicAdd(t + (int)flp, -(1.0 - fp) * sv);
-            atomicAdd(t + (int)flp + 1, -fp * sv);
-        }
-    }
-    __syncthreads();
-    for (int j = 0; j < nr; j++)
-        for (int q = threadIdx.x; q < a.nt; q += blockDim.x)
-            a.raw[((size_t)k * a.nh + r0 + j) * a.nt + q] = tr[j * a.nt + q];
-}
-
-int launch_spray(const SprayArgs &a, cudaStream_t st)
-{
-    if (a.nsb <= 0 || a.nh <= 0) return KCIG_OK;
-    constexpr int RB = 4;
-    const size_t sm = (size_t)RB * a.nt * sizeof(double);
-    if (sm > 200 * 1024) return set_error(KCIG_ERR_UNSUPPORTED, "nt=%d too long for forward modelling", a.nt);
-    const int grid = a.nsb * ((a.nh + RB - 1) / RB);
-    if (a.mode == 0) {
-        KCIG_TRY(set_dyn_smem((const void *)k_spray<0, RB>, (int)sm));
-        k_spray<0, RB><<<grid, 256, sm, st>>>(a);
-    } else if (a.mode == 1) {
-        KCIG_TRY(set_dyn_smem((const void *)k_spray<1, RB>, (int)sm));
-        k_spray<1, RB><<<grid, 256, sm, st>>>(a);
-    } else {
-        KCIG_TRY(set_dyn_smem((const void *)k_spray<2, RB>, (int)sm));
-        k_spray<2, RB><<<grid, 256, sm, st>>>(a);
-    }
-    KCIG_CUDA(cudaGetLastError());
-    return KCIG_OK;
-}
-
 // image (+)= the split rows' partial images, rows in order (deterministic)
 __global__ void k_sum_reduce(float *image, const float *partial, int nsplit, size_t n, int zero_init)
 {
@@ -1795,6 +1673,157 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         KCIG_CUDA(cudaGetLastError());  // (counted by the caller: `launches` counts k_sum launches)
     }
     return KCIG_OK;
+}
+
+// ------------------------------------------------------- forward modelling --
+// kirchmig2d_cig adj=0 (:1300-1312, kirmig.cpp:59-68): one CTA per trace, the
+// same gates, weights and pick positions as k_sum.  The trace accumulates in
+// shared memory in FP64 (it is integrated twice afterwards, which would amplify
+// FP32 accumulation error); a warp takes every so many-th group of 8 tiles,
+// skips the tiles that the pair cannot reach (the bounds of k_leg_bounds, as
+// the summation's lists) and sweeps the others' columns of 32 depths.
+//
+// A shared FP64 atomic add is a compare-and-swap loop, and six a pair bound the
+// sweep: warps in flight hide them.  With a CTA per trace an SM holds 48 warps
+// whatever the record's length (a CTA of four traces, 32 KB of 1001 samples and
+// 160 KB of 5000, left 16 to 8), and the near offsets' longer sweeps spread out.
+// 201 x 401 points, 16 x 101 traces, the whole call: 1001 samples 2.55 -> 1.52
+// ms, 301 of 4 ms 1.96 -> 0.83, 6001 of 0.5 ms 6.84 -> 2.66.  The bounds alone
+// gave 0.17 ms; four resident CTAs instead of six 1.68 ms; copies of the trace
+// per warp with plain adds where a column's samples are distinct 1.62 ms (a
+// third of the columns are not, and the copies cost the warps in flight).
+constexpr int kSprayTZ = 32, kSprayTX = 4, kSprayThreads = 256;
+
+template <int MODE>
+__global__ void __launch_bounds__(kSprayThreads, 6) k_spray(const __grid_constant__ SprayArgs a)
+{
+    extern __shared__ double tr[];  // [nt]
+    constexpr int TZ = kSprayTZ, TX = kSprayTX;
+    constexpr double kPiD = 3.141592653589793238463, kTwoPi = 6.283185307179586476925;
+    const int trc = blockIdx.x, k = trc / a.nh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kSprayThreads / 32;
+    for (int q = threadIdx.x; q < a.nt; q += blockDim.x) tr[q] = 0.0;
+    __syncthreads();
+    const float tw = __ldg(a.trw + trc);
+    if (tw != 0.0f) {
+        const int ri = __ldg(a.rfi + trc), ig = __ldg(a.igo + trc);
+        const size_t nzx = (size_t)a.nz * a.nx;
+        const double2 *STP = a.STP + k * nzx, *RTP = a.RTP + ri * nzx;
+        const float2 *SXW = a.SXW + k * nzx, *RXW = a.RXW + ri * nzx;
+        const double top = (double)(a.nt - 1);
+        const double ulo = -1.0e-5, uhi = a.cull.utop + 1.0e-5, uk = a.cull.uk, ub = a.cull.ub;
+        const int tiles_z = (a.nz + TZ - 1) / TZ, tiles = tiles_z * ((a.nx + TX - 1) / TX);
+        for (int t0 = warp * 8; t0 < tiles; t0 += warps * 8) {
+            bool keep = false;
+            if (lane < 8 && t0 + lane < tiles) {
+                const float4 *bt = a.bounds + (size_t)(t0 + lane) * a.nlegs;
+                keep = cull_keep(a.cull, __ldg(bt + a.nrl + k), __ldg(bt + ri), (float)top);
+            }
+            unsigned on = __ballot_sync(0xffffffffu, keep);
+            for (; on; on &= on - 1u) {
+                const int t = t0 + __ffs(on) - 1;
+                const int iz = t % tiles_z * TZ + lane, x0 = t / tiles_z * TX, ncol = min(TX, a.nx - x0);
+                if (iz >= a.nz) continue;
+                const float zf = (a.nz > 1) ? (float)iz / (float)(a.nz - 1) : 0.0f;
+                const float cutoff = a.oazmin + zf * (a.oazmax - a.oazmin);
+#pragma unroll 1
+                for (int c = 0; c < ncol; c++) {
+                    const int i = (x0 + c) * a.nz + iz;
+                    const double2 sTP = __ldg(STP + i), rTP = __ldg(RTP + i);
+                    const float2 sXW = __ldg(SXW + i), rXW = __ldg(RXW + i);
+                    const float apw = sXW.y * rXW.y;
+                    if (!(sXW.y > 0.0f && apw > 0.0f)) continue;
+                    int b0 = ig;
+                    float w0 = 1.0f, w1 = 0.0f, aw = tw * apw;
+                    if (MODE != 2) {
+                        double th = fabs(sTP.y - rTP.y);
+                        th = (th > kPiD) ? kTwoPi - th : th;
+                        const double u = fma(th, uk, ub);
+                        double fl;
+                        if (MODE == 0) {
+                            if (!(u >= ulo && u <= uhi)) continue;
+                            fl = floor(u);
+                        } else {
+                            fl = floor(u + 0.5);
+                            if (!(fl >= 0.0 && fl < (double)a.ng)) continue;
+                        }
+                        const float ang = (float)(th * a.deg);
+                        aw = taper_weight(ang, a.ats, a.ate) * depth_weight(ang, cutoff, a.oaztaper) * tw * apw;
+                        if (!(aw > 0.0f)) continue;
+                        b0 = (int)fl;
+                        if (MODE == 0) {
+                            if (u <= 0.0) b0 = 0;
+                            else if (u >= (double)(a.ng - 1)) b0 = a.ng - 1;
+                            else {
+                                const double f1 = u - fl;
+                                w1 = (float)f1;
+                                w0 = (float)(1.0 - f1);
+                            }
+                        }
+                    }
+                    const double ft0 = (sTP.x + rTP.x + a.tau - a.t0) * a.inv_dt;
+                    const double sh = fma((double)(fmaxf(fabsf(sXW.x), fabsf(rXW.x)) * a.aal), a.inv_dt, 1.0);
+                    const double ftm0 = ft0 - sh, ftp0 = ft0 + sh;
+                    const double fl0 = floor(ft0), flm = floor(ftm0), flp = floor(ftp0);
+                    if (!(fl0 >= 0.0 && fl0 < top && flm >= 0.0 && flm <= fl0 && flp >= fl0 && flp < top)) continue;
+                    float val = w0 * __ldg(a.image + (size_t)b0 * nzx + i);
+                    if (MODE == 0 && w1 > 0.0f) val += w1 * __ldg(a.image + (size_t)(b0 + 1) * nzx + i);
+                    const float r1 = 1.0f / (1.0f + 2.0f * (float)sh);  // dt / (dt + tp - tm)
+                    const double sv = (double)(r1 * r1 * (aw * val));
+                    const double f0 = ft0 - fl0, fm = ftm0 - flm, fp = ftp0 - flp;
+                    atomicAdd(tr + (int)fl0, 2.0 * (1.0 - f0) * sv);
+                    atomicAdd(tr + (int)fl0 + 1, 2.0 * f0 * sv);
+                    atomicAdd(tr + (int)flm, -(1.0 - fm) * sv);
+                    atomicAdd(tr + (int)flm + 1, -fm * sv);
+                    atomicAdd(tr + (int)flp, -(1.0 - fp) * sv);
+                    atomicAdd(tr + (int)flp + 1, -fp * sv);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < a.nt; q += blockDim.x) a.raw[(size_t)trc * a.nt + q] = tr[q];
+}
+
+int launch_spray(const SprayArgs &a0, cudaStream_t st)
+{
+    if (a0.nsb <= 0 || a0.nh <= 0) return KCIG_OK;
+    SprayArgs a = a0;
+    const size_t sm = a.nt * sizeof(double);
+    if (4 * sm > 200 * 1024) return set_error(KCIG_ERR_UNSUPPORTED, "nt=%d too long for forward modelling", a.nt);
+    // what the pair bounds read, and the legs' ranges over the tiles
+    memset(&a.cull, 0, sizeof a.cull);
+    a.cull.inv_dt = a.inv_dt;
+    a.cull.tau = a.tau;
+    a.cull.t0 = a.t0;
+    a.cull.mode = a.mode;
+    a.cull.uk = a.deg * a.uinv;
+    a.cull.ub = -(a.ug0 * a.uinv);
+    a.cull.utop = (double)(a.ng - 1);
+    a.nlegs = a.nrl + a.nsb;
+    const int tiles = ((a.nz + kSprayTZ - 1) / kSprayTZ) * ((a.nx + kSprayTX - 1) / kSprayTX);
+    float4 *bounds = reinterpret_cast<float4 *>(a.scratch);
+    SumArgs b = a.cull;
+    b.RTP = a.RTP;
+    b.RXW = a.RXW;
+    b.STP = a.STP;
+    b.SXW = a.SXW;
+    b.nrl = a.nrl;
+    b.nz = a.nz;
+    b.nx = a.nx;
+    KCIG_TRY((launch_bounds_t<kSprayTZ, kSprayTX>(b, a.nlegs, bounds, tiles, st)));
+    a.bounds = bounds;
+    const auto kern = a.mode == 0 ? k_spray<0> : a.mode == 1 ? k_spray<1> : k_spray<2>;
+    KCIG_TRY(set_dyn_smem((const void *)kern, (int)sm));
+    kern<<<a.nsb * a.nh, kSprayThreads, sm, st>>>(a);
+    KCIG_CUDA(cudaGetLastError());
+    return KCIG_OK;
+}
+
+size_t spray_scratch_bytes(int nz, int nx, int nsb, int nrl)
+{
+    return (size_t)((nz + kSprayTZ - 1) / kSprayTZ) * ((nx + kSprayTX - 1) / kSprayTX) * (size_t)(nsb + nrl) *
+           sizeof(float4);
 }
 
 // A summation is split over shots into partial images when its tiles fill

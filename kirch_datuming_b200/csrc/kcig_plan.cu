@@ -1167,7 +1167,8 @@ extern "C" int kcig_model(kcig_plan *P, const float *image, float *data, int mem
     }
     // batches of shots: source and receiver legs, raw traces
     const size_t leg_bytes = nzx * (sizeof(double2) + sizeof(float2));
-    const size_t per_shot = leg_bytes * (1 + (size_t)g.nh) + (size_t)g.nh * g.nt * sizeof(double) + (size_t)g.nh * 16;
+    const size_t per_shot = leg_bytes * (1 + (size_t)g.nh) + (size_t)g.nh * g.nt * sizeof(double) + (size_t)g.nh * 16 +
+                            spray_scratch_bytes(g.nz, g.nx, 1, g.nh);
     int nsb = (int)std::max<long long>(1, (long long)(P->budget / 2) / (long long)per_shot);
     nsb = std::min(nsb, g.ns);
     int rc = P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2));
@@ -1253,6 +1254,10 @@ extern "C" int kcig_model(kcig_plan *P, const float *image, float *data, int mem
         sa.rfi = d_rfi;
         sa.igo = d_igo;
         sa.image = d_img;
+        sa.nrl = (int)rl.size();
+        rc = P->d_cull.ensure(spray_scratch_bytes(g.nz, g.nx, nsh, sa.nrl));
+        if (rc) break;
+        sa.scratch = P->d_cull.p;
         sa.raw = P->d_D.as<double>();
         sa.nz = g.nz;
         sa.nx = g.nx;
@@ -1275,7 +1280,7 @@ extern "C" int kcig_model(kcig_plan *P, const float *image, float *data, int mem
         sa.ate = p.angle_taper_end;
         rc = launch_spray(sa, st);
         if (!rc) rc = launch_doubint_f32(P->d_D.as<double>(), d_dat + (size_t)s0 * g.nh * g.nt, (int)nb, g.nt, st);
-        P->all_launches += 2;
+        P->all_launches += 3;
         P->sum_launches += 1;
         if (!rc) {  // the host tables are reused by the next batch
             cudaError_t e = cudaStreamSynchronize(st);
