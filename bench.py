@@ -138,41 +138,6 @@ def measured_peaks(kind: str = "hbm"):
         return fallback, "of fallback"
 
 
-def profiled_traffic():
-    """DRAM bytes per pair of the summation kernel from the committed ncu
-    summary (profiles/k_sum_traffic.json), or None."""
-    try:
-        with open(os.path.join(ROOT, "profiles", "k_sum_traffic.json")) as f:
-            return float(json.load(f)["dram_bytes_per_pair"])
-    except Exception:
-        return None
-
-
-def issue_ceiling(pairs_per_s: float, sm_mhz):
-    """The summation's instruction-issue ceiling next to its HBM roofline:
-    148 SMs x 4 schedulers x one warp instruction per cycle, divided by the
-    thread instructions per pair of the committed ncu summary; with that
-    summary's L2 hit rate.  None without the summary."""
-    try:
-        with open(os.path.join(ROOT, "profiles", "k_sum_traffic.json")) as f:
-            p = json.load(f)
-        ipp = float(p["thread_instructions_per_pair"])
-        mhz = float(sm_mhz) if sm_mhz else 1965.0
-        ceiling = 148 * 4 * 32 * mhz * 1e6 / ipp / 1e9
-        return {"thread_instructions_per_pair": ipp, "sm_mhz": mhz, "ceiling_gpairs": ceiling,
-                "frac": pairs_per_s / 1e9 / ceiling, "issue_active_pct_ncu": p.get("issue_active_pct"),
-                "l2_sector_hit_rate_pct_ncu": p.get("l2_sector_hit_rate_pct")}
-    except Exception:
-        return None
-
-
-# ----------------------------------------------------------- reference (CPU) --
-REF_BIN = os.path.join(ROOT, "oracle", "_ref", "kirchmig2d_cig")
-REF_EIK = os.path.join(ROOT, "oracle", "_ref", "eikods2d")
-SAMPLE_SHOT = 200          # shot at 8.0 km
-SAMPLE_RCV = (176, 48)     # 48 receivers, 7.04 .. 8.92 km
-
-
 def prepare_sample(wd: str, threads: int, tables=None):
     """Write the inputs of a bounded sample of the workload: one shot x 48
     receivers over the full 601x1601 image (4.62e7 pairs).  Tables are cut
@@ -592,7 +557,7 @@ def stitch_section(steps: int, warmup: int, threads: int):
     res = {"workload": STITCH_WORKLOAD, "device_ms": t_all, "samples_out": n1 * n2 * n3,
            "roofline": {"bound": "hbm", "achieved": algo_all / (t_all / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                         "frac": algo_all / (t_all / 1e3) / 1e9 / peak, "peak_source": peak_src,
-                        "kernel": "k_stitch_all",
+                        "kernel": "k_stitch_rows",
                         "note": "one kcig_stitch_windows call: the weight upload, one kernel, the counters' "
                                 "read-back and the synchronisation"},
            "one_pass_equals_window_calls": same_all,
@@ -1211,7 +1176,6 @@ def main():
     peak, peak_src = measured_peaks()
     pairs_rank = count * NPOS * NZ * NX  # the summation kernel's own share
     achieved = pairs_rank * B_PAIR / (ksum_ms / 1e3) / 1e9
-    tpp = profiled_traffic()
     line = {
         "metric": metric, "value": pairs / (ms / 1e3) / 1e9, "unit": "Gpairs/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
@@ -1224,11 +1188,10 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_src, "kernel": "k_sum", "kernel_ms": ksum_ms,
                      "algorithmic_bytes_per_pair": B_PAIR,
-                     "traffic": (tpp * pairs_rank) if tpp is not None else None,
-                     "issue": issue_ceiling(pairs_rank / (ksum_ms / 1e3), (clk or {}).get("sm_mhz")),
-                     "note": "16 B/pair counts the receiver leg's fields once per pair; k_sum loads each "
-                             "receiver leg once per block of 4 shots, so its DRAM traffic (ncu, 'traffic') is "
-                             "below the algorithmic bytes and frac can pass 1: the kernel is issue-bound"},
+                     "traffic": None,
+                     "note": "16 B/pair counts the receiver leg's fields once for every pair of the survey; pairs "
+                             "that cannot contribute are left out by bounds and reciprocal pairs are taken once, "
+                             "so frac passes 1: the pairs computed are bound by L1 wavefronts of their gathers"},
         "e2e": {"value": pairs / (e2e_ms / 1e3) / 1e9, "unit": "Gpairs/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms},
         "streamed_tables": None if stream_ms is None else {

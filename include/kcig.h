@@ -226,8 +226,10 @@ typedef struct kcig_eikods_opts {
  * first derivatives with respect to the source position; both or neither),
  * gradz/gradx (the branch-aware upwind gradients of eikods2d.cpp:30-68), all
  * [nshot][nx][nz] (device), and iters [nshot] (host): the sweeps each source
- * took.  nz in 3..1400, nx >= 3; the call allocates 4 bytes of scratch per
- * output sample.  The same local problem as the marching code, solved by
+ * took.  nz in 3..1400, nx >= 3.  Scratch comes from a memory pool
+ * of the library: the working values of the sources in flight (32 MB each on
+ * 601 x 1601; fewer at a time where memory is short), of which the pool keeps
+ * up to a sixteenth of the device until kcig_datum_release.  The same local problem as the marching code, solved by
  * sweeps to the fixed point: identical results for order 1, within ~2.5e-4 s
  * for order 2 (whose marching result depends on the heap's acceptance
  * order).  KCIG_ERR_DEVICE if a source has no fixed point within max_iter. */

@@ -154,7 +154,7 @@ static int prelude_block(int nt, int *warps)
 // so every running sum is FP64 and every shared-memory access is one
 // consecutive row (no bank conflicts).  Causal sum, then anticausal sum
 // (kirmig.cpp:8-24), then the optional centred difference (:381-394); the
-// {D[i], D[i+1]-D[i]} pairs leave with coalesced 16-byte stores.
+// segment lines {D[i] - i dD[i], dD[i]} leave with coalesced 16-byte stores.
 __device__ __forceinline__ double warp_incl_scan(double v)
 {
     const int lane = threadIdx.x & 31;
@@ -1127,7 +1127,7 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 // (kirchmig2d_cig.cpp:1206-1339), cheapest rejections first: trace weight,
 // aperture gate, opening angle as the folded difference of the two legs'
 // gradient directions (exact in FP64, no per-pair arc tangent) and its bin
-// range, the angle tapers, then the antialiased pick from {D[i], D[i+1]-D[i]}
+// range, the angle tapers, then the antialiased pick from {D[i] - i dD[i], dD[i]}
 // with its time-to-sample mapping and six-term sum in FP64.  Rejections are
 // mostly uniform across a warp (32 neighbouring image points), so skipping
 // them costs little.
@@ -1872,10 +1872,10 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
         // measured 4.80 -> 4.42 ms
         // Blocks one a row may go on in parts of their receiver lists, of four
         // receivers or more: a row then lasts 1 / parts of a block (41 x 81
-        // points, 2 blocks of 21 receivers: k_sum 43 -> 17 us in five parts;
-        // 43 x 172 points, 9 blocks of 202: 721 -> 373 us in five); from three
-        // waves on the set-up of more rows costs what the last wave gains (the
-        // v(z) survey in 48 rows: 2.64 -> 3.02 ms)
+        // points, 2 blocks of 21 receivers: the stage 62 -> 36 us in five parts;
+        // 43 x 172 points, 9 blocks of 202: 0.74 -> 0.39 ms); from three waves
+        // on the set-up of more rows costs more than the last wave gains (the
+        // v(z) survey with parts: 2.64 -> 3.02 ms)
         long long best = 1;
         double cost = -1.0;
         auto offer = [&](long long rows, double length) {
