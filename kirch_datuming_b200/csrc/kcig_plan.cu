@@ -1978,7 +1978,7 @@ extern "C" int kcig_leg_fields_noalloc(const kcig_params *p, const kcig_geometry
     leg_interp(&view, is_source, (float)pos, pos, &L);
     L.scale = 1.0f;
     KCIG_CUDA(cudaMemcpyAsync(d_leg, &L, sizeof L, cudaMemcpyHostToDevice, st));
-    FieldArgs a;
+    FieldArgs a{};  // no needed-blocks map
     a.tab = table;
     a.der = deriv;
     a.gxv = gradx;
