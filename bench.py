@@ -138,6 +138,13 @@ def measured_peaks(kind: str = "hbm"):
         return fallback, "of fallback"
 
 
+# ----------------------------------------------------------- reference (CPU) --
+REF_BIN = os.path.join(ROOT, "oracle", "_ref", "kirchmig2d_cig")
+REF_EIK = os.path.join(ROOT, "oracle", "_ref", "eikods2d")
+SAMPLE_SHOT = 200          # shot at 8.0 km
+SAMPLE_RCV = (176, 48)     # 48 receivers, 7.04 .. 8.92 km
+
+
 def prepare_sample(wd: str, threads: int, tables=None):
     """Write the inputs of a bounded sample of the workload: one shot x 48
     receivers over the full 601x1601 image (4.62e7 pairs).  Tables are cut
