@@ -272,6 +272,7 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
 {
     const kcig_geometry &g = P->g;
     const size_t nzx = (size_t)g.nz * g.nx;
+    P->need = nullptr;  // of these legs: all their fields, unless a map is made below
     if (n <= 0) return KCIG_OK;
     const int angle = P->p.cig && P->p.cig_is_angle;
     if (kcig_surrogate *sgt = is_source ? P->sg_src : P->sg_rcv) {
@@ -355,7 +356,6 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
     const bool one = leg_tile_applies(a);
     const int FB = one ? std::min(n, 65535) : field_batch(P, (size_t)n);
     if (angle && !one) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
-    P->need = nullptr;
     if (P->need_args.nr > 0 && one && n <= FB) {
         const size_t cells = (size_t)n * leg_tiles(g.nz, g.nx);
         KCIG_TRY(P->d_need.ensure(cells * (sizeof(float) + 1)));
@@ -856,10 +856,11 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
                 const double end = ((double)g.nt + 1.0) * (double)g.dt + (double)g.t0 - (double)p.tau;
                 P->need_args.end = end + 1e-6 * fabs(end);
             }
+            const bool mapped = P->need_args.nr > 0;
             rc = fields(0, rl, P->d_rT.as<double2>(), P->d_rF.as<float2>());
             P->need_args.nr = 0;
             if (rc) break;
-            need = P->need;
+            need = mapped ? P->need : nullptr;
         }
         for (int s0 = 0; s0 < ns && rc == KCIG_OK; s0 += nsb) {
             const int nsh = std::min(nsb, ns - s0);
