@@ -22,10 +22,12 @@ using namespace kcig;
 struct DevBuf {
     void *p = nullptr;
     size_t n = 0;
-    int ensure(size_t bytes)
+    // `retired`: a list that takes a buffer outgrown instead of its being freed
+    int ensure(size_t bytes, std::vector<void *> *retired = nullptr)
     {
         if (bytes <= n && p) return KCIG_OK;
-        if (p) cudaFree(p);
+        if (p && retired) retired->push_back(p);
+        else if (p) cudaFree(p);
         p = nullptr;
         n = 0;
         if (bytes == 0) return KCIG_OK;
@@ -83,6 +85,11 @@ struct kcig_plan {
     // first trace prelude waits for copy_ev
     cudaStream_t copy_st = nullptr;
     cudaEvent_t copy_ev = nullptr, order_ev = nullptr;
+    // A scratch buffer of at least `bytes`.  Every buffer that the launches of
+    // prepared shots read or write grows through here: a captured graph
+    // (kcig_migrate_prepared, kcig_graph_create) holds their addresses, so
+    // what it captured stays allocated until the shots are released.
+    int scratch(DevBuf &b, size_t bytes);
 };
 
 // Ragged shots on the device, batched (kcig_shots_prepare); the launch
@@ -102,7 +109,14 @@ struct ShotsPrepared {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     float *graph_image = nullptr;
+    bool captured = false;         // some graph holds addresses of the plan's scratch
+    std::vector<void *> retired;   // scratch outgrown since
 };
+
+int kcig_plan::scratch(DevBuf &b, size_t bytes)
+{
+    return b.ensure(bytes, shots && shots->captured ? &shots->retired : nullptr);
+}
 
 static void release_shots(kcig_plan *P)
 {
@@ -115,6 +129,7 @@ static void release_shots(kcig_plan *P)
     S->trf.release();
     S->stop.release();
     S->snh.release();
+    for (void *q : S->retired) cudaFree(q);
     delete S;
     P->shots = nullptr;
 }
@@ -314,7 +329,7 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
         P->all_launches += 1;
         if (fd_angle) {
             const int FB = leg_grad_needs_work(a) ? field_batch(P, (size_t)n) : n;
-            if (leg_grad_needs_work(a)) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
+            if (leg_grad_needs_work(a)) KCIG_TRY(P->scratch(P->d_work, (size_t)FB * 4 * nzx * sizeof(double)));
             for (int j0 = 0; j0 < n; j0 += FB) {
                 a.legs = d_legs + j0;
                 a.n = std::min(FB, n - j0);
@@ -355,7 +370,7 @@ int compute_fields_dev(kcig_plan *P, int is_source, const LegInterp *d_legs, int
     // in batches of their work planes
     const bool one = leg_tile_applies(a);
     const int FB = one ? std::min(n, 65535) : field_batch(P, (size_t)n);
-    if (angle && !one) KCIG_TRY(P->d_work.ensure((size_t)FB * 4 * nzx * sizeof(double)));
+    if (angle && !one) KCIG_TRY(P->scratch(P->d_work, (size_t)FB * 4 * nzx * sizeof(double)));
     if (P->need_args.nr > 0 && one && n <= FB) {
         const size_t cells = (size_t)n * leg_tiles(g.nz, g.nx);
         KCIG_TRY(P->d_need.ensure(cells * (sizeof(float) + 1)));
@@ -800,17 +815,17 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
     const bool joint = shared_r && !alias_src && nhc == g.nh && nsb == ns && same_sides(P) && !P->stream_tables &&
                        !P->sg_src;
     if (shared_r) {
-        KCIG_TRY(P->d_rT.ensure((size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(double2)));
-        KCIG_TRY(P->d_rF.ensure((size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(float2)));
+        KCIG_TRY(P->scratch(P->d_rT, (size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(double2)));
+        KCIG_TRY(P->scratch(P->d_rF, (size_t)(nhc + (joint ? ns : 0)) * nzx * sizeof(float2)));
     } else {
-        KCIG_TRY(P->d_rT.ensure((size_t)nsb * g.nh * nzx * sizeof(double2)));
-        KCIG_TRY(P->d_rF.ensure((size_t)nsb * g.nh * nzx * sizeof(float2)));
+        KCIG_TRY(P->scratch(P->d_rT, (size_t)nsb * g.nh * nzx * sizeof(double2)));
+        KCIG_TRY(P->scratch(P->d_rF, (size_t)nsb * g.nh * nzx * sizeof(float2)));
     }
     if (!alias_src && !joint) {
-        KCIG_TRY(P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2)));
-        KCIG_TRY(P->d_sF.ensure((size_t)nsb * nzx * sizeof(float2)));
+        KCIG_TRY(P->scratch(P->d_sT, (size_t)nsb * nzx * sizeof(double2)));
+        KCIG_TRY(P->scratch(P->d_sF, (size_t)nsb * nzx * sizeof(float2)));
     }
-    KCIG_TRY(P->d_D.ensure((size_t)nsb * nhc * g.nt * sizeof(double2)));
+    KCIG_TRY(P->scratch(P->d_D, (size_t)nsb * nhc * g.nt * sizeof(double2)));
     const size_t trn = (size_t)nsb * nhc;
     // one allocation: doubles first (8-byte aligned), then floats and ints
     KCIG_TRY(P->d_tr.ensure(trn * (2 * sizeof(double) + sizeof(float) + 2 * sizeof(int))));
@@ -965,7 +980,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.nrl = shared_r ? nhb : (int)rl.size();
             sa.need_r = need;
             if (need) sa.need_s = need + (size_t)(joint ? nhb : s0 + fold.off) * leg_tiles(g.nz, g.nx);
-            rc = P->d_cull.ensure(sum_cull_bytes(g.nz, g.nx, nsh, nhb, sa.nrl, P->ng, P->tile, shared_r));
+            rc = P->scratch(P->d_cull, sum_cull_bytes(g.nz, g.nx, nsh, nhb, sa.nrl, P->ng, P->tile, shared_r));
             if (rc) break;
             sa.cull = P->d_cull.p;
             sa.RTP = P->d_rT.as<double2>();
@@ -990,7 +1005,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.tile = P->tile;
             sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, nhb, shared_r);
             if (sa.nsplit > 1) {
-                rc = P->d_part.ensure((size_t)sa.nsplit * P->ng * nzx * sizeof(float));
+                rc = P->scratch(P->d_part, (size_t)sa.nsplit * P->ng * nzx * sizeof(float));
                 if (rc) break;
                 sa.partial = P->d_part.as<float>();
             }
@@ -1172,11 +1187,11 @@ extern "C" int kcig_model(kcig_plan *P, const float *image, float *data, int mem
                             spray_scratch_bytes(g.nz, g.nx, 1, g.nh);
     int nsb = (int)std::max<long long>(1, (long long)(P->budget / 2) / (long long)per_shot);
     nsb = std::min(nsb, g.ns);
-    int rc = P->d_sT.ensure((size_t)nsb * nzx * sizeof(double2));
-    if (!rc) rc = P->d_sF.ensure((size_t)nsb * nzx * sizeof(float2));
-    if (!rc) rc = P->d_rT.ensure((size_t)nsb * g.nh * nzx * sizeof(double2));
-    if (!rc) rc = P->d_rF.ensure((size_t)nsb * g.nh * nzx * sizeof(float2));
-    if (!rc) rc = P->d_D.ensure((size_t)nsb * g.nh * g.nt * sizeof(double));  // raw traces
+    int rc = P->scratch(P->d_sT, (size_t)nsb * nzx * sizeof(double2));
+    if (!rc) rc = P->scratch(P->d_sF, (size_t)nsb * nzx * sizeof(float2));
+    if (!rc) rc = P->scratch(P->d_rT, (size_t)nsb * g.nh * nzx * sizeof(double2));
+    if (!rc) rc = P->scratch(P->d_rF, (size_t)nsb * g.nh * nzx * sizeof(float2));
+    if (!rc) rc = P->scratch(P->d_D, (size_t)nsb * g.nh * g.nt * sizeof(double));  // raw traces
     if (!rc) rc = P->d_tr.ensure((size_t)nsb * g.nh * (sizeof(float) + 2 * sizeof(int)));
     if (rc) return rc;
     float *d_trw = P->d_tr.as<float>();
@@ -1256,7 +1271,7 @@ extern "C" int kcig_model(kcig_plan *P, const float *image, float *data, int mem
         sa.igo = d_igo;
         sa.image = d_img;
         sa.nrl = (int)rl.size();
-        rc = P->d_cull.ensure(spray_scratch_bytes(g.nz, g.nx, nsh, sa.nrl));
+        rc = P->scratch(P->d_cull, spray_scratch_bytes(g.nz, g.nx, nsh, sa.nrl));
         if (rc) break;
         sa.scratch = P->d_cull.p;
         sa.raw = P->d_D.as<double>();
@@ -1325,6 +1340,16 @@ TraceViews trace_views(const ShotsPrepared *S)
     v.igo = v.rfi + ntr;
     v.tnt = v.igo + ntr;
     return v;
+}
+
+// The lists of a batch in any tile variant: the autotuner times them all, and
+// the one it picks stays.
+size_t batch_cull_bytes(const kcig_plan *P, int ns, int nh, int nrl)
+{
+    size_t most = 0;
+    for (int t = 0; t < kSumTiles; t++)
+        most = std::max(most, sum_cull_bytes(P->g.nz, P->g.nx, ns, nh, nrl, P->ng, t, false));
+    return most;
 }
 
 // leg fields of batch b
@@ -1404,7 +1429,7 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.nsb = B.ns;
     sa.nh = B.nhb;
     sa.nrl = B.nrl;
-    sa.cull = P->d_cull.p;  // sized by kcig_shots_prepare and the autotuner
+    sa.cull = P->d_cull.p;  // sized by kcig_shots_prepare
     sa.ng = P->ng;
     sa.mode = angle ? (p.angle_interp ? 0 : 1) : 2;
     sa.unit_tw = B.unit_tw;
@@ -1638,20 +1663,19 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
     if (!rc) rc = S->trf.ensure(std::max<size_t>(ntr, 1) * (3 * 8 + 4 * 4));
     if (!rc) rc = S->stop.ensure(std::max<size_t>(h_stop.size(), 1) * sizeof(float));
     if (!rc) rc = S->snh.ensure(std::max<size_t>(h_snh.size(), 1) * sizeof(int));
-    if (!rc) rc = P->d_sT.ensure(std::max<size_t>(max_s, 1) * nzx * sizeof(double2));
-    if (!rc) rc = P->d_sF.ensure(std::max<size_t>(max_s, 1) * nzx * sizeof(float2));
-    if (!rc) rc = P->d_rT.ensure(std::max<size_t>(max_r, 1) * nzx * sizeof(double2));
-    if (!rc) rc = P->d_rF.ensure(std::max<size_t>(max_r, 1) * nzx * sizeof(float2));
-    if (!rc) rc = P->d_D.ensure(std::max<size_t>(max_d, 1) * (size_t)ntmax * sizeof(double2));
+    if (!rc) rc = P->scratch(P->d_sT, std::max<size_t>(max_s, 1) * nzx * sizeof(double2));
+    if (!rc) rc = P->scratch(P->d_sF, std::max<size_t>(max_s, 1) * nzx * sizeof(float2));
+    if (!rc) rc = P->scratch(P->d_rT, std::max<size_t>(max_r, 1) * nzx * sizeof(double2));
+    if (!rc) rc = P->scratch(P->d_rF, std::max<size_t>(max_r, 1) * nzx * sizeof(float2));
+    if (!rc) rc = P->scratch(P->d_D, std::max<size_t>(max_d, 1) * (size_t)ntmax * sizeof(double2));
     if (!rc && angle && !(P->sg_src && P->sg_rcv))
-        rc = P->d_work.ensure((size_t)field_batch(P, std::max(max_s, max_r)) * 4 * nzx * sizeof(double));
+        rc = P->scratch(P->d_work, (size_t)field_batch(P, std::max(max_s, max_r)) * 4 * nzx * sizeof(double));
     int max_split = 1;
     for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, B.nhb, false));
-    if (!rc && max_split > 1) rc = P->d_part.ensure((size_t)max_split * P->ng * nzx * sizeof(float));
+    if (!rc && max_split > 1) rc = P->scratch(P->d_part, (size_t)max_split * P->ng * nzx * sizeof(float));
     size_t cull = 0;
-    for (const ShotBatch &B : S->batches)
-        cull = std::max(cull, sum_cull_bytes(g.nz, g.nx, B.ns, B.nhb, B.nrl, P->ng, P->tile, false));
-    if (!rc) rc = P->d_cull.ensure(cull);
+    for (const ShotBatch &B : S->batches) cull = std::max(cull, batch_cull_bytes(P, B.ns, B.nhb, B.nrl));
+    if (!rc) rc = P->scratch(P->d_cull, cull);
     struct Cp { void *dst; const void *src; size_t bytes; } cps[] = {
         {S->legs.p, hlegs.data(), hlegs.size() * sizeof(LegInterp)},
         {S->trf.as<double>(), h_msx.data(), ntr * 8},
@@ -1733,6 +1757,7 @@ extern "C" int kcig_migrate_prepared(kcig_plan *P, float *image, int memory)
                 cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
                 if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamBeginCapture");
                 if (!rc) {
+                    S->captured = true;
                     const int rc2 = run_prepared(P, d_img, st);
                     cudaGraph_t gr = nullptr;
                     e = cudaStreamEndCapture(st, &gr);
@@ -1795,12 +1820,6 @@ extern "C" int kcig_plan_autotune(kcig_plan *P, int *choice, float *ms)
     KCIG_TRY(P->d_image.ensure((size_t)P->ng * nzx * sizeof(float)));
     cudaStream_t st = P->st;
     KCIG_TRY(batch_inputs(P, 0, st));
-    // every variant's lists, for every batch: the chosen one stays
-    size_t cull = 0;
-    for (const ShotBatch &B : P->shots->batches)
-        for (int t = 0; t < kSumTiles; t++)
-            cull = std::max(cull, sum_cull_bytes(P->g.nz, P->g.nx, B.ns, B.nhb, B.nrl, P->ng, t, false));
-    KCIG_TRY(P->d_cull.ensure(cull));
     SumArgs sa = batch_sum_args(P, 0, P->d_image.as<float>());
     cudaEvent_t e0, e1;
     KCIG_CUDA(cudaEventCreate(&e0));
@@ -1864,7 +1883,10 @@ extern "C" int kcig_graph_create(int n, kcig_plan *const *plans, float *const *i
         if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamBeginCapture");
         if (!rc) {
             int rc2 = KCIG_OK;
-            for (int i = 0; i < n && rc2 == KCIG_OK; i++) rc2 = run_prepared(plans[i], images[i], st);
+            for (int i = 0; i < n && rc2 == KCIG_OK; i++) {
+                plans[i]->shots->captured = true;
+                rc2 = run_prepared(plans[i], images[i], st);
+            }
             e = cudaStreamEndCapture(st, &G->graph);
             if (rc2) rc = rc2;
             else if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamEndCapture");

@@ -53,3 +53,50 @@ def test_surrogate_after_tables(ds):
     net.close()
     assert images[1].norm() > 0
     assert torch.equal(images[0], images[1])
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_graph_keeps_its_scratch(golden, own):
+    """A graph over prepared shots (kcig_graph, or the plan's own) replays the
+    same image after calls that need more scratch than the shots did: the
+    autotuner's larger lists, a migration and a modelling of the whole cube.
+    What they free, if anything, is overwritten before the replay."""
+    import torch
+    import _cases
+    kp, geom, axis, _, _ = _cases.case_setup(golden, "base")
+    kp.direct_mute = 0  # kcig_model takes none
+    tT, tD = (torch.from_numpy(a).cuda() for a in golden.tables())
+    cube = torch.from_numpy(golden.data("base")).cuda()
+    ns, nh, nt = cube.shape
+    dh = float(np.float32(geom["dh"]))
+    shot = dict(sx=float(np.float32(geom["s0"])), h0=float(np.float32(geom["h0"])), dh=dh, data=cube[0, :5].contiguous())
+    plan = kd.Plan(kp, kd.geometry(**geom))
+    plan.set_tables(tT, tD, tT, tD)
+    plan.prepare_shots([shot])
+    img, other, data = (torch.zeros(s, device="cuda") for s in ((axis[0], geom["nx"], geom["nz"]),) * 2 + (cube.shape,))
+    if own:
+        plan.set_graph(True)
+        plan.migrate_prepared(img)
+    else:
+        graph = kd.Graph([plan], [img])
+    replay = (lambda: plan.migrate_prepared(img)) if own else graph.launch
+    replay()
+    torch.cuda.synchronize()
+    want = img.clone()
+    assert want.norm() > 0
+    steps = [lambda: plan.migrate(cube, other), lambda: plan.model(want, data)]
+    if not own:  # the autotuner drops the plan's own graph
+        steps.insert(0, plan.autotune)
+    for step in steps:
+        step()
+        waste = [torch.full((n << 18,), float("nan"), device="cuda") for n in (1, 2, 4, 8, 16, 32, 64)]
+        torch.cuda.synchronize()
+        img.fill_(3.0)
+        replay()
+        torch.cuda.synchronize()
+        assert torch.equal(img, want)
+        del waste
+        torch.cuda.empty_cache()
+    if not own:
+        graph.close()
+    plan.close()
