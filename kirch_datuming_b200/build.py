@@ -32,7 +32,7 @@ DATUM_CLI = os.path.join(PKG, "bin", "kirchdat2d_freq")
 
 SOURCES = ["kcig_kernels.cu", "kcig_plan.cu", "kcig_eikods.cu", "kcig_mlp.cu", "kcig_params.cpp", "kcig_rsf.cpp", "kcig_cli.cpp",
            "kcig_eikods_cli.cpp", "kcig_stitch.cu", "kcig_stitch_cli.cpp", "kcig_datum.cu", "kcig_datum_cli.cpp"]
-HEADERS = ["kcig_common.h", "kcig_tc.h", "kcig_aperture.h", "kcig_par.h", "kcig_rsf.h"]
+HEADERS = ["kcig_common.h", "kcig_tc.h", "kcig_aperture.h", "kcig_div.h", "kcig_par.h", "kcig_rsf.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -46,6 +46,7 @@
 #include <vector>
 
 #include "kcig_common.h"
+#include "kcig_div.h"
 
 namespace kcig {
 namespace {
@@ -57,15 +58,6 @@ struct EikSource {
     int ic;                  // box centre (its slowness is the box's)
     float xs0, xs1, xs2;     // source minus origin: depth, lateral, third axis
 };
-
-// the same in FP32 for a = 0 or |a| >= 2^-80 (below, the remainder could underflow)
-__device__ __forceinline__ float div_by(float a, float b, float y)
-{
-    if (fabsf(a) < 8.27e-25f && a != 0.0f) return __fdiv_rn(a, b);
-    float q = __fmul_rn(a, y);
-    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
 
 // Reciprocals of the divisors of the local problem; [second order on axis 0]
 // [on axis 1] of the two-axis sum, [axis][second order] of one axis
@@ -88,7 +80,7 @@ struct EikArgs {
     int blk_shift, nblk;  // diagonals per skipping block (a power of two), blocks
     float d0, d1, d2;  // sampling: depth, lateral, third axis
     float rdx0, rdx1;  // 1 / d^2 rounded to float (neighbors.cpp:19-30)
-    float dd0, dd1, yd0, yd1;  // d^2 of both axes and its reciprocal
+    DivF dd0, dd1;     // d^2 of both axes
     EikRecip rc;
 };
 
@@ -120,19 +112,6 @@ template <int N>
 __device__ __forceinline__ void cp_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// a / b correctly rounded, y = RN(1 / b): Markstein's theorem (IBM J. Res.
-// Dev. 34, 1990) -- with q within an ulp of a / b and r = a - b q exact, q +
-// r y rounds to RN(a / b); the first correction brings q within an ulp.
-// The divisors of a point's update are few (sums of the axes' weights), so
-// their reciprocals come from the host, and the serial chain that bounds a
-// step shortens: five dependent operations for a general division's dozen.
-__device__ __forceinline__ double div_by(double a, double b, double y)
-{
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
 // neighbors.cpp:106-160 for one axis, with stencil() (:271-276): the
@@ -385,6 +364,8 @@ __device__ __forceinline__ bool eik_sweep(const EikArgs &a, const EikSource &sc,
                     const uint32_t tm = ((p - 1) & (kEikS - 1)) * q, tp = ((p + 1) & (kEikS - 1)) * q;
                     const float t0 = lds32(t + (p & (kEikS - 1)) * q);
                     double rhs = 0.0, den = 0.0;
+                    float e[2], el[2];  // of an axis without an upwind neighbour: not used
+                    bool up[2], quick = true;
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
                         const int ii = j == 0 ? iz : ix, len = j == 0 ? nz : nx;
@@ -394,13 +375,20 @@ __device__ __forceinline__ bool eik_sweep(const EikArgs &a, const EikSource &sc,
                         const float lb = __uint_as_float(j == 0 ? zp.x : xp.x);
                         const bool use_b = ii == 0 || (ii != len - 1 && ta > tb);
                         const float t1 = use_b ? tb : ta, l1 = use_b ? lb : la;
-                        const bool up = t1 < t0;
-                        const float dd = j == 0 ? a.dd0 : a.dd1, yd = j == 0 ? a.yd0 : a.yd1;
-                        const float e = up ? __fsub_rn(t0, t1) : 0.0f;
-                        const double term = (double)div_by(__fmul_rn(e, l1), dd, yd);
-                        const double dterm = (double)div_by(e, dd, yd);
-                        rhs = up ? __dadd_rn(rhs, term) : rhs;
-                        den = up ? __dadd_rn(den, dterm) : den;
+                        const DivF &dd = j == 0 ? a.dd0 : a.dd1;
+                        up[j] = t1 < t0;
+                        e[j] = up[j] ? __fsub_rn(t0, t1) : 1.0f;
+                        el[j] = __fmul_rn(e[j], l1);
+                        quick = quick && div_quick(e[j], dd) && (div_quick(el[j], dd) || el[j] == 0.0f);
+                    }
+                    // one test for the point's four divisions (never-reached times, infinite slopes)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        const DivF &dd = j == 0 ? a.dd0 : a.dd1;
+                        const double term = (double)(quick ? div_known(el[j], dd) : __fdiv_rn(el[j], dd.div));
+                        const double dterm = (double)(quick ? div_known(e[j], dd) : __fdiv_rn(e[j], dd.div));
+                        rhs = up[j] ? __dadd_rn(rhs, term) : rhs;
+                        den = up[j] ? __dadd_rn(den, dterm) : den;
                     }
                     nv = den != 0.0 ? __double2float_rn(__ddiv_rn(__dadd_rn(__dmul_rn(0.5, w_cur[qr]), rhs), den)) : 0.0f;
                     if (!(nv != __uint_as_float(lds64(r + o[2]).x))) continue;
@@ -829,10 +817,8 @@ extern "C" int kcig_eikods(const float *vel, int nz, int nx, float o1, float o2,
     a.d2 = d3;
     a.rdx0 = (float)(1. / (d1 * d1));
     a.rdx1 = (float)(1. / (d2 * d2));
-    a.dd0 = d1 * d1;
-    a.dd1 = d2 * d2;
-    a.yd0 = 1.0f / a.dd0;
-    a.yd1 = 1.0f / a.dd1;
+    a.dd0 = div_prepare(d1 * d1);
+    a.dd1 = div_prepare(d2 * d2);
     for (int i = 0; i < 2; i++) {
         const double w0 = (double)a.rdx0 * (i ? 2.25 : 1.0);
         a.rc.one[0][i] = 1.0 / w0;
