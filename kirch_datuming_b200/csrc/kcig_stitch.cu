@@ -304,12 +304,12 @@ __device__ __forceinline__ void stitch_round(const StitchRowsArgs &a, const Stit
         const float sx = __shfl_sync(0xffffffffu, sl, u);
         float v = __fmul_rn(va[u], __fmul_rn(w.sa, w.la ? sx : 1.0f));
         const bool ok = fabsf(v) <= 3.402823466e38f;
-        bad_a += !ok;
+        bad_a += !ok && (FULL || u < n);  // past the last column: 0 times a scale that may be infinite
         v = ok && w.a ? v : 0.0f;
         if (TWO && pb) {
             float x = __fmul_rn(vb[u], __fmul_rn(w.sb, w.lb ? sx : 1.0f));
             const bool fine = fabsf(x) <= 3.402823466e38f;
-            bad_b += !fine;
+            bad_b += !fine && (FULL || u < n);
             x = fine ? x : 0.0f;
             if (!w.keep) v = __fadd_rn(__fmul_rn(v, __fsub_rn(1.0f, w.w)), __fmul_rn(x, w.w));
         }
