@@ -39,10 +39,10 @@ struct StitchArgs {
 __global__ void __launch_bounds__(256) k_stitch_layer(const StitchArgs a)
 {
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int ncol = a.n2 * a.n3;  // < 2^31 (checked on the host)
+    const unsigned ncol = (unsigned)a.n2 * a.n3;  // < 2^31 (checked on the host); a stride past it stays below 2^32
     unsigned long long bad = 0;
-    for (int col = blockIdx.x * warps + (threadIdx.x >> 5); col < ncol; col += gridDim.x * warps) {
-        const int i2 = col % a.n2;
+    for (unsigned col = blockIdx.x * warps + (threadIdx.x >> 5); col < ncol; col += gridDim.x * warps) {
+        const int i2 = (int)(col % (unsigned)a.n2);
         const float sx = a.lateral ? a.lateral[i2] : 1.0f;
         const float scale = __fmul_rn(a.layer_scale, sx);
         const float *src = a.layer + (size_t)col * a.n1w;
@@ -206,9 +206,9 @@ __global__ void __launch_bounds__(256) k_stitch_all(const StitchAllArgs a)
     extern __shared__ float colbuf[];  // [warps][n1]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     float *buf = colbuf + (size_t)warp * a.n1;
-    const int ncol = a.n2 * a.n3;
-    for (int col = blockIdx.x * warps + warp; col < ncol; col += gridDim.x * warps) {
-        const int i2 = col % a.n2;
+    const unsigned ncol = (unsigned)a.n2 * a.n3;  // < 2^31; a stride past it stays below 2^32
+    for (unsigned col = blockIdx.x * warps + warp; col < ncol; col += gridDim.x * warps) {
+        const int i2 = (int)(col % (unsigned)a.n2);
         const float sx = a.lateral ? a.lateral[i2] : 1.0f;
         for (int r = lane; r < a.n1; r += 32) buf[r] = 0.0f;
         __syncwarp();
@@ -297,7 +297,7 @@ __device__ __forceinline__ void stitch_round(const StitchRowsArgs &a, const Stit
         for (int u = 0; u < U; u++) vb[u] = pb && (FULL || u < n) ? __ldcs(pb + (size_t)(unsigned)(u * w.nb)) : 0.0f;
     }
     // the columns' lateral scales: one load a round, column u's from lane u
-    const int il = (int)((unsigned)(i2 + (threadIdx.x & 31)) % (unsigned)a.n2);
+    const int il = (int)(((unsigned)i2 + (threadIdx.x & 31)) % (unsigned)a.n2);
     const float sl = a.lateral ? __ldg(a.lateral + il) : 1.0f;
 #pragma unroll
     for (int u = 0; u < U; u++) {
@@ -325,12 +325,12 @@ __device__ __forceinline__ void stitch_row(const StitchRowsArgs &a, const Stitch
     const float *pa = w.a ? w.a + (size_t)c0 * w.na : a.out, *pb = w.b ? w.b + (size_t)c0 * w.nb : nullptr;
     float *po = a.out + (size_t)c0 * a.n1 + r;
     int i2 = c0 % a.n2, bad_a = 0, bad_b = 0, c = c0;
-    for (; c + U <= c1; c += U) {
+    for (; c1 - c >= U; c += U) {
         stitch_round<TWO, U, true>(a, w, in, pa, pb, po, i2, U, bad_a, bad_b);
         pa += (size_t)U * w.na;
         if (TWO && pb) pb += (size_t)U * w.nb;
         po += (size_t)U * a.n1;
-        i2 = (int)((unsigned)(i2 + U) % (unsigned)a.n2);
+        i2 = (int)(((unsigned)i2 + U) % (unsigned)a.n2);
     }
     if (c < c1) stitch_round<TWO, U, false>(a, w, in, pa, pb, po, i2, c1 - c, bad_a, bad_b);
     if (bad_a && in && w.a) atomicAdd(a.nonfinite + w.ka, (unsigned long long)bad_a);
@@ -341,9 +341,11 @@ __global__ void __launch_bounds__(256, 4) k_stitch_rows(const StitchRowsArgs a)
 {
     const int nrb = (a.n1 + 31) / 32;
     const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int r = wid % nrb * 32 + (threadIdx.x & 31), c0 = wid / nrb * a.per;  // neighbouring warps: neighbouring rows
-    if (c0 >= a.ncol) return;
-    const int c1 = min(a.ncol, c0 + a.per);
+    const int r = wid % nrb * 32 + (threadIdx.x & 31);  // neighbouring warps: neighbouring rows
+    // the last block's warps start past the volume, possibly past 2^31
+    const unsigned u0 = (unsigned)(wid / nrb) * (unsigned)a.per;
+    if (u0 >= (unsigned)a.ncol) return;
+    const int c0 = (int)u0, c1 = (int)min((unsigned)a.ncol, u0 + (unsigned)a.per);
     StitchRow w = a.rows[min(r, a.n1 - 1)];
     if (r >= a.n1) w.b = nullptr;
     if (__any_sync(0xffffffffu, w.b != nullptr)) stitch_row<true, kStitchU / 2>(a, w, r < a.n1, r, c0, c1);

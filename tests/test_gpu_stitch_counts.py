@@ -26,3 +26,20 @@ def test_scales_not_finite(n2, n3, scale):
             prev = b
         assert counts == bad
         assert torch.equal(out, one)
+
+
+def test_most_columns_accepted():
+    """2^31 - 1 columns (17 GB with the window): the last ones are written by
+    each form of the stitching -- by rows, by columns (three windows on a row)
+    and window by window."""
+    import torch
+    n2 = 2 ** 31 - 1
+    vol = torch.empty((1, n2, 1), device="cuda").uniform_(1.0, 2.0)
+    out = torch.empty_like(vol)
+    for layers in ([vol], [vol, vol, vol]):
+        out.zero_()
+        assert kd.stitch_windows(out, layers, [(0, 0)] * len(layers), 0) == [0] * len(layers)
+        assert torch.equal(out, vol)
+    out.zero_()
+    assert kd.stitch_window(out, vol, 0, 0) == 0
+    assert torch.equal(out, vol)
