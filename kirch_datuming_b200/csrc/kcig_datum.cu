@@ -1780,11 +1780,13 @@ extern "C" int kcig_datum_freq(const kcig_datum_params *pp, const float *stable,
     const size_t op_r = h.rcv.size(), op_s = shared_op ? 0 : h.src.size();
     const size_t per_f = (interm ? 0 : (size_t)ntr * sizeof(float2)) + (op_r + op_s) * sizeof(float2);
     int chunk = (int)std::max<size_t>(1, std::min<size_t>(256, ((size_t)1536 << 20) / std::max<size_t>(per_f, 1)));
-    chunk = std::min(chunk, nw);
     // rows of the spectra in residue order when the operators come from FFTs:
     // a chunk is then a group of residues (Q rows each; the first Q / 2 + 1,
-    // the last Q / 2)
-    const int Q = op_points(K, nfft), M = Q ? nfft / Q : 0;
+    // the last Q / 2).  Spreads so wide that a residue's Q rows pass the
+    // chunk's memory keep Horner's rule, which takes any number of rows: FFTs
+    // halve the operators' time, but their GEMMs take ten times that.
+    const int Q0 = op_points(K, nfft), Q = chunk >= Q0 ? Q0 : 0, M = Q ? nfft / Q : 0;
+    chunk = std::min(chunk, nw);
     const int chunk_res = Q ? std::max(1, chunk / Q) : 0;
     struct Chunk {
         int f0, nf, a0, na;
