@@ -1561,7 +1561,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
             const int ns1 = i1 - i0 + 1, nh1 = std::max(nhb, sh.nh);
             const size_t need = (size_t)(ns1 + seen.size() + add.size()) * leg_bytes +
                                 (size_t)ns1 * nh1 * ((size_t)ntmax * sizeof(double2) + 48) + work_bytes +
-                                sum_cull_bytes(g.nz, g.nx, ns1, nh1, (int)(seen.size() + add.size()), P->ng, P->tile, false);
+                                batch_cull_bytes(P, ns1, nh1, (int)(seen.size() + add.size()));
             if (i1 > i0 && need > budget) break;
             for (auto &kv : add) seen.emplace(kv.first, 0);
             nhb = nh1;
