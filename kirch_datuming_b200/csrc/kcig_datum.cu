@@ -1226,6 +1226,7 @@ int ensure_buffers(DatumCache &c, const size_t *need)
         }
         if (bad < 0) return KCIG_OK;
         free_buffers(c);
+        KCIG_TRY(eik_release_pool());  // what the table calls keep
         if (attempt == 1)
             return set_error(KCIG_ERR_NOMEM, "kcig_datum_freq: cannot allocate %.3f GB for %s on the device",
                              need[bad] / 1e9, kSlotName[bad]);

@@ -676,7 +676,10 @@ struct DevBuf {
 // The calls' device memory comes from a stream-ordered pool of the library,
 // one per device, that keeps up to a sixteenth of the device between calls
 // (mapping and unmapping memory anew cost more than the solve on small
-// grids: ~16 ms per GB); eik_release_pool gives all of it back.
+// grids: ~16 ms per GB).  On a device with less than a 32nd free (5.7 GB) a call
+// gives back what it used (kEikKeep at most stays); the library's other
+// allocations take it back when they fail, and eik_release_pool at any time.
+constexpr uint64_t kEikKeep = 256ull << 20;
 std::mutex g_pool_mu;
 std::map<int, cudaMemPool_t> g_pools;
 
@@ -700,6 +703,40 @@ int eik_pool(cudaMemPool_t *out)
         it = g_pools.emplace(dev, pool).first;
     }
     *out = it->second;
+    return KCIG_OK;
+}
+
+// memory the pool holds and no call uses
+size_t eik_pool_idle(cudaMemPool_t pool)
+{
+    uint64_t held = 0, used = 0;
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held);
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    return held > used ? held - used : 0;
+}
+
+// Gives back what a call leaves in the pool where the device is `full`.
+// Declared before the call's buffers, so that they have been freed by then.
+struct PoolSettle {
+    cudaMemPool_t pool;
+    cudaStream_t st;
+    bool full = false;
+    ~PoolSettle()
+    {
+        if (!full || cudaStreamSynchronize(st) != cudaSuccess) return;
+        cudaMemPoolTrimTo(pool, kEikKeep);
+        cudaGetLastError();
+    }
+};
+
+// Whether the device is nearly full without what the pool holds idle; fr: what
+// is free with it.  (A query takes ~0.15 ms: calls below kEikKeep go without.)
+int eik_device_full(cudaMemPool_t pool, size_t *fr, bool *full)
+{
+    size_t tot = 0;
+    KCIG_CUDA(cudaMemGetInfo(fr, &tot));
+    *full = *fr < tot / 32;
+    *fr += eik_pool_idle(pool);
     return KCIG_OK;
 }
 
@@ -762,14 +799,15 @@ extern "C" int kcig_eikods(const float *vel, int nz, int nx, float o1, float o2,
     KCIG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     KCIG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     int slots = std::min(nshot, std::max(1, per_sm) * sms);
-    if (slots * slot > ((size_t)256 << 20)) {
-        size_t fr = 0, tot = 0;
-        KCIG_CUDA(cudaMemGetInfo(&fr, &tot));
+    cudaMemPool_t pool;
+    KCIG_TRY(eik_pool(&pool));
+    PoolSettle settle{pool, st};
+    if (slots * slot > kEikKeep) {
+        size_t fr = 0;
+        KCIG_TRY(eik_device_full(pool, &fr, &settle.full));
         slots = (int)std::max<size_t>(1, std::min<size_t>(slots, fr / 2 / slot));
     }
 
-    cudaMemPool_t pool;
-    KCIG_TRY(eik_pool(&pool));
     DevBuf bvv, bsk, bdw, bdp, bsrc, bstat, bit, bwork;
     bvv.st = bsk.st = bdw.st = bdp.st = bsrc.st = bstat.st = bit.st = bwork.st = st;
     KCIG_CUDA(cudaMallocFromPoolAsync(&bvv.p, nzx * sizeof(float), pool, st));
@@ -881,16 +919,15 @@ extern "C" int kcig_eikonal_tables(const float *vel, int nz, int nx, float dz, f
     o.l = 1;
     o.vel_is_slowness2 = 0;
     o.max_iter = iterations;
-    float *dl1 = nullptr;
-    if (deriv) {
-        cudaMemPool_t pool;
-        KCIG_TRY(eik_pool(&pool));
-        cudaError_t e = cudaMallocFromPoolAsync((void **)&dl1, (size_t)npos * nz * nx * sizeof(float), pool,
-                                                (cudaStream_t)stream);
-        if (e != cudaSuccess) return cuda_error(e, "cudaMallocFromPoolAsync(tdl1)");
-    }
-    const int rc = kcig_eikods(vel, nz, nx, z0, x0, dz, dx, 0.0f, 1.0f, shots.data(), npos, &o, time, dl1, deriv,
-                               nullptr, nullptr, nullptr, stream);
-    if (dl1) cudaFreeAsync(dl1, (cudaStream_t)stream);
-    return rc;
+    cudaMemPool_t pool;
+    KCIG_TRY(eik_pool(&pool));
+    PoolSettle settle{pool, (cudaStream_t)stream};
+    DevBuf dl1;
+    dl1.st = (cudaStream_t)stream;
+    size_t fr = 0;
+    if (deriv && (size_t)npos * nz * nx * sizeof(float) > kEikKeep) KCIG_TRY(eik_device_full(pool, &fr, &settle.full));
+    if (deriv)
+        KCIG_CUDA(cudaMallocFromPoolAsync(&dl1.p, (size_t)npos * nz * nx * sizeof(float), pool, (cudaStream_t)stream));
+    return kcig_eikods(vel, nz, nx, z0, x0, dz, dx, 0.0f, 1.0f, shots.data(), npos, &o, time, (float *)dl1.p, deriv,
+                       nullptr, nullptr, nullptr, stream);
 }

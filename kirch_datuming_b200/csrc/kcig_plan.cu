@@ -32,6 +32,10 @@ struct DevBuf {
         n = 0;
         if (bytes == 0) return KCIG_OK;
         cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation && eik_release_pool() == KCIG_OK) {  // what the table calls keep
+            cudaGetLastError();
+            e = cudaMalloc(&p, bytes);
+        }
         if (e != cudaSuccess) {
             p = nullptr;
             return cuda_error(e, "cudaMalloc(scratch)");
