@@ -190,11 +190,12 @@ struct SumArgs {
     Fold fold;             // pairs of skipped reciprocal traces are left out
     int shot0, rcv0;       // first shot and receiver of the batch in the call
     double uk, ub, utop, uhi, top;  // set by launch_sum: u = theta uk + ub, ng - 1 (+ 1e-5), nt - 1
+    int lists;             // walk lists of the pairs that may reach a tile, else every receiver
     void *cull;            // scratch of sum_cull_bytes
     const unsigned char *need_r, *need_s;  // [legs][leg_tiles] blocks whose fields exist, or null (all)
     int nrl;               // receiver legs (RTP, RXW)
     int unit_all;          // every trace weight is 1, none is 0 (unit_tw: every one that is not 0)
-    int parts;             // set by launch_sum: parts of a block's list (rows of CTAs beyond the blocks)
+    int parts;             // set by launch_sum: parts of a block's walk (rows of CTAs beyond the blocks)
     int nblk;              // set by launch_sum: blocks of shots, and per tile and block the
     const int *cnt;        // [tiles][nblk] number of receivers with a pair that may reach the tile
     const unsigned *list;  // [tiles][nblk][nh] and those receivers: r << 4 | shots of the block
@@ -202,6 +203,12 @@ struct SumArgs {
 // launches: k_sum launches added; aux: the launches that prepare them added
 int launch_sum(const SumArgs &a, cudaStream_t st, int *launches, int *aux = nullptr);
 size_t sum_cull_bytes(int nz, int nx, int nsb, int nh, int nrl, int ng, int tile, bool shared_r);
+// Whether the sum has to walk lists whatever they cost.
+bool sum_needs_lists(const SumArgs &a);
+// A sample of the batch: out[kReachPairs] (pinned host memory), the points (of
+// kReachPoints) that each of some pairs misses.
+constexpr int kReachPairs = 64, kReachPoints = 256;
+int launch_reach(const SumArgs &a, int *out, cudaStream_t st);
 // Tile variants the summation can be launched with (the autotuner's choices):
 // {TZ, TX, shots per block on the receiver-shared path}.
 // Forward modelling (adj=0): the picks of k_sum run backwards, each image
@@ -236,7 +243,7 @@ int eik_release_pool();
 
 // How many rows of CTAs (partial images) a summation over nsb shots of nh
 // receivers on an nz x nx image is split into to fill the GPU (1: none).
-int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r);
+int sum_nsplit(int nz, int nx, int nsb, int nh, int ng, bool shared_r);
 constexpr int kSumTiles = 5;
 extern const int kSumTileShape[kSumTiles][3];
 

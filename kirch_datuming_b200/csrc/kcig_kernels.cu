@@ -1149,9 +1149,14 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 #define KCIG_SUM_MINB_UNSHARED KCIG_SUM_MINB
 #endif
 
-// PLAIN: every trace weight of the launch is 1 and it holds all angle bins
-// (one chunk), so neither a weight nor a bin's range is tested per pair.
-template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool PLAIN, bool PARTS>
+// The receivers a block of shots walks: all of them or those on its list (pairs
+// that may reach the tile, k_cull); the whole walk, or a part of it.
+enum Walk { kWalkAll, kWalkAllParts, kWalkList, kWalkListParts };
+
+// PLAIN: every trace weight of the launch is 1 (or, with lists, 0) and it holds
+// all angle bins (one chunk), so neither a weight nor a bin's range is tested
+// per pair.
+template <int TZ, int TX, int KB, bool SHARED_R, int MODE, bool PLAIN, Walk WALK>
 __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_MINB_UNSHARED) * 128 / (TZ * TX))
     k_sum(const __grid_constant__ SumArgs a)
 {
@@ -1193,20 +1198,35 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
     // shot (receivers not shared), so that KB independent (shot, receiver)
     // gather chains are in flight per thread either way
     constexpr int KR = SHARED_R ? 1 : KB;
-    // (rows beyond the blocks: each block's list in as many parts, PARTS)
+    // (rows beyond the blocks: each block's walk in as many parts)
+    constexpr bool LIST = WALK >= kWalkList, PARTS = WALK == kWalkAllParts || WALK == kWalkListParts;
     for (int blk = PARTS ? blockIdx.y / a.parts : blockIdx.y; blk < a.nblk; blk += PARTS ? a.nblk : gridDim.y) {
+        const int sb = blk * KB;
         // the block's receivers with a pair that may reach this tile, in
         // order, each with the shots it may do so with (k_cull)
         const size_t lb = (size_t)blockIdx.x * a.nblk + blk;
-        int cnt = __ldg(a.cnt + lb);
-        const unsigned *lst = a.list + lb * a.nh;
-        if (PARTS) {
-            const int part = blockIdx.y % a.parts, lo = cnt * part / a.parts;
-            cnt = cnt * (part + 1) / a.parts - lo;
-            lst += lo;
+        int cnt = LIST ? __ldg(a.cnt + lb) : a.nh;
+        // without a list: every receiver, with the block's shots or, with
+        // receivers of their own, those shots that have as many
+        int nrk[KR];
+        if (!LIST && !SHARED_R) {
+            cnt = 0;
+#pragma unroll
+            for (int j = 0; j < KR; j++) {
+                nrk[j] = sb + j >= a.nsb ? 0 : a.snh ? __ldg(a.snh + sb + j) : a.nh;
+                cnt = max(cnt, nrk[j]);
+            }
         }
+        int lo = 0;  // first step of the part
+        if (PARTS) {
+            const int part = blockIdx.y % a.parts;
+            lo = cnt * part / a.parts;
+            cnt = cnt * (part + 1) / a.parts - lo;
+        }
+        const unsigned *lst = LIST ? a.list + lb * a.nh + lo : nullptr;
         if (cnt == 0) continue;
-        const int sb = blk * KB;
+        // the list's q-th entry, 0 past its end
+        auto entry = [&](int q) -> unsigned { return LIST && q < cnt ? __ldg(lst + q) : 0u; };
         double2 sTP[KB];
         float2 sXW[KB];
 #pragma unroll
@@ -1231,26 +1251,29 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
         int fnext[KR];
         double2 nTP[KR];
         float2 nXW[KR];
-        unsigned e1 = __ldg(lst), e2 = cnt > 1 ? __ldg(lst + 1) : 0u, e3 = !SHARED_R && cnt > 2 ? __ldg(lst + 2) : 0u;
+        unsigned e1 = entry(0), e2 = entry(1), e3 = LIST && !SHARED_R ? entry(2) : 0u;
+        // whether stream j's shot takes the step of receiver r (entry e)
+        auto takes = [&](unsigned e, int r, int j) { return LIST ? (e >> j & 1u) != 0u : r < nrk[j]; };
 #pragma unroll
         for (int j = 0; j < KR; j++) {
             topk[j] = (!SHARED_R && a.stop && sb + j < a.nsb) ? (double)__ldg(a.stop + sb + j) : a.top;
             fnext[j] = 0;
             nTP[j] = make_double2(0.0, 0.0);
             nXW[j] = make_float2(0.f, 0.f);
-            if (SHARED_R || (e1 >> j & 1u)) {
-                const size_t f0 = SHARED_R ? (size_t)(e1 >> 4) : (size_t)__ldg(a.rfi + (size_t)(sb + j) * a.nh + (e1 >> 4));
+            const int r0 = LIST ? (int)(e1 >> 4) : lo, r1 = LIST ? (int)(e2 >> 4) : lo + 1;
+            if (SHARED_R || takes(e1, r0, j)) {
+                const size_t f0 = SHARED_R ? (size_t)r0 : (size_t)__ldg(a.rfi + (size_t)(sb + j) * a.nh + r0);
                 nTP[j] = __ldg(a.RTP + f0 * nzx + i);
                 nXW[j] = __ldg(a.RXW + f0 * nzx + i);
             }
-            if (!SHARED_R && (e2 >> j & 1u)) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + (e2 >> 4));
+            if (!SHARED_R && takes(e2, r1, j)) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + r1);
         }
         for (int q = 0; q < cnt; q++) {
             const unsigned e0 = e1;
-            const int r = (int)(e0 >> 4);
+            const int r = LIST ? (int)(e0 >> 4) : lo + q;
             e1 = e2;  // 0 past the end
-            e2 = SHARED_R ? (q + 2 < cnt ? __ldg(lst + q + 2) : 0u) : e3;
-            if (!SHARED_R) e3 = q + 3 < cnt ? __ldg(lst + q + 3) : 0u;
+            e2 = LIST && !SHARED_R ? e3 : entry(q + 2);
+            if (LIST && !SHARED_R) e3 = entry(q + 3);
             double2 rTP[KR];
             float2 rXW[KR];
 #pragma unroll
@@ -1260,22 +1283,26 @@ __global__ void __launch_bounds__(TZ *TX, (SHARED_R ? KCIG_SUM_MINB : KCIG_SUM_M
                 // the receiver's share, once per receiver for the stream's shots
                 rTP[j].x *= a.inv_dt;
                 rXW[j].x = fabsf(rXW[j].x) * aal_abs * inv_dt_f;
-                if (SHARED_R ? e1 != 0u : (e1 >> j & 1u) != 0u) {
-                    const size_t f1 = SHARED_R ? (size_t)(e1 >> 4) : (size_t)fnext[j];
+                if (SHARED_R ? (LIST ? e1 != 0u : q + 1 < cnt) : takes(e1, r + 1, j)) {
+                    const size_t f1 = !SHARED_R ? (size_t)fnext[j] : LIST ? (size_t)(e1 >> 4) : (size_t)(r + 1);
                     nTP[j] = __ldg(a.RTP + f1 * nzx + i);
                     nXW[j] = __ldg(a.RXW + f1 * nzx + i);
                 }
-                if (!SHARED_R && (e2 >> j & 1u)) fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + (e2 >> 4));
+                if (!SHARED_R && takes(e2, r + 2, j))
+                    fnext[j] = __ldg(a.rfi + (size_t)(sb + j) * a.nh + (LIST ? (int)(e2 >> 4) : r + 2));
             }
 #pragma unroll
             for (int k = 0; k < KB; k++) {
-                if (!(e0 >> k & 1u)) continue;
                 const int j = SHARED_R ? 0 : k;  // this shot's receiver stream
+                if (!LIST && SHARED_R && sb + k >= a.nsb) break;
+                if ((LIST || !SHARED_R) && !takes(e0, r, k)) continue;
                 const double2 rTPk = rTP[j];
                 const float2 rXWk = rXW[j];
                 const double topj = SHARED_R ? a.top : topk[j];
                 const int trc = (sb + k) * a.nh + r;
-                const float tw = PLAIN || a.unit_tw ? 1.0f : __ldg(a.trw + trc);  // not 0: k_cull
+                // a weight of 0 (trace aperture, offset bin) is on no list
+                const float tw = PLAIN || (LIST ? a.unit_tw : a.unit_all) ? 1.0f : __ldg(a.trw + trc);
+                if (!LIST && !PLAIN && tw == 0.0f) continue;
                 const float apw = sXW[k].y * rXWk.y;
                 if (!(apw > 0.0f)) continue;
                 int b0 = 0;
@@ -1526,9 +1553,19 @@ static int launch_sum_t(const SumArgs &a, int nb, cudaStream_t st)
 {
     constexpr int P = TZ * TX;
     const size_t sm = (size_t)nb * P * sizeof(float);
-    const bool plain = MODE <= 1 && a.unit_tw && nb == a.ng;
-    auto kern = plain ? k_sum<TZ, TX, KB, SR, MODE, MODE <= 1, false> : k_sum<TZ, TX, KB, SR, MODE, false, false>;
-    if (a.parts > 1) kern = plain ? k_sum<TZ, TX, KB, SR, MODE, MODE <= 1, true> : k_sum<TZ, TX, KB, SR, MODE, false, true>;
+    const bool plain = MODE <= 1 && (a.lists ? a.unit_tw : a.unit_all) && nb == a.ng;
+    constexpr bool PL = MODE <= 1;
+    const int walk = (a.lists ? kWalkList : kWalkAll) + (a.parts > 1);
+    auto kern = k_sum<TZ, TX, KB, SR, MODE, false, kWalkAll>;
+    if (plain)
+        kern = walk == kWalkAll        ? k_sum<TZ, TX, KB, SR, MODE, PL, kWalkAll>
+               : walk == kWalkAllParts ? k_sum<TZ, TX, KB, SR, MODE, PL, kWalkAllParts>
+               : walk == kWalkList     ? k_sum<TZ, TX, KB, SR, MODE, PL, kWalkList>
+                                       : k_sum<TZ, TX, KB, SR, MODE, PL, kWalkListParts>;
+    else if (walk != kWalkAll)
+        kern = walk == kWalkAllParts ? k_sum<TZ, TX, KB, SR, MODE, false, kWalkAllParts>
+               : walk == kWalkList   ? k_sum<TZ, TX, KB, SR, MODE, false, kWalkList>
+                                     : k_sum<TZ, TX, KB, SR, MODE, false, kWalkListParts>;
     // all of the unified L1/shared memory as shared: the accumulators of as
     // many CTAs as the registers allow (the driver's own choice held 8x8
     // tiles to 10 CTAs per SM)
@@ -1618,6 +1655,42 @@ static int launch_bounds_t(const SumArgs &a, int nlegs, float4 *out, int tiles, 
     return KCIG_OK;
 }
 
+// Sums that cannot go without lists: reciprocal traces left out, legs without
+// their fields everywhere.
+bool sum_needs_lists(const SumArgs &a) { return a.fold.on || a.need_r || a.need_s; }
+
+// How many of kReachPoints points of the image each of kReachPairs pairs of
+// the batch misses: no weight, out of the record or past the angle axis.
+__global__ void __launch_bounds__(kReachPoints) k_reach(const __grid_constant__ SumArgs a, int *out)
+{
+    const int p = blockIdx.x, k = (int)((long long)p * a.nsb / kReachPairs);
+    const int nh = a.snh ? a.snh[k] : a.nh;
+    const int r = (int)(((unsigned)p * 2654435769u >> 16) * (unsigned long long)nh >> 16);  // golden-ratio steps
+    const size_t t = (size_t)k * a.nh + r, nzx = (size_t)a.nz * a.nx;
+    // 8 depths x 32 positions, in the middle of as many cells
+    const int iz = (2 * (int)(threadIdx.x & 7) + 1) * (long long)a.nz / 16, ix = (2 * (int)(threadIdx.x >> 3) + 1) * (long long)a.nx / 64;
+    const size_t i = (size_t)ix * a.nz + iz, rl = a.shared_r ? r : a.rfi[t];
+    const double2 s = a.STP[k * nzx + i], q = a.RTP[rl * nzx + i];
+    bool in = a.trw[t] != 0.0f && a.SXW[k * nzx + i].y * a.RXW[rl * nzx + i].y > 0.0f;
+    const double f = (s.x + q.x + a.tau - a.t0) * a.inv_dt;
+    in = in && f >= 0.0 && f < (a.stop ? (double)a.stop[k] : (double)(a.nt - 1));
+    if (a.mode < 2) {
+        double th = fabs(s.y - q.y);
+        th = th > 3.14159265358979 ? 6.28318530717959 - th : th;
+        const double u = (th * a.deg - a.ug0) * a.uinv;
+        in = in && u >= -0.5 && u <= (double)a.ng - 0.5;
+    }
+    const int missed = __syncthreads_count(!in);
+    if (threadIdx.x == 0) out[p] = missed;
+}
+
+int launch_reach(const SumArgs &a, int *out, cudaStream_t st)
+{
+    k_reach<<<kReachPairs, kReachPoints, 0, st>>>(a, out);
+    KCIG_CUDA(cudaGetLastError());
+    return KCIG_OK;
+}
+
 int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
 {
     static_assert((KCIG_KB == 4 || KCIG_KB == 2) && (KCIG_KB_UNSHARED == 2 || KCIG_KB_UNSHARED == 4), "k_cull's block sizes");
@@ -1635,6 +1708,8 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         int tz, tx, kb;
         sum_shape(a.tile, nb, a.shared_r != 0, &tz, &tx, &kb);
         a.nblk = (a.nsb + kb - 1) / kb;
+        a.parts = a.nsplit > a.nblk ? a.nsplit / a.nblk : 1;
+        a.lists = a.lists || sum_needs_lists(a);
         // the lists of this tile shape: legs' bounds, then the receivers per
         // tile and block.  Shots whose fields are a receiver's take its bounds.
         const int tiles = ((a.nz + tz - 1) / tz) * ((a.nx + tx - 1) / tx);
@@ -1645,16 +1720,17 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         float4 *br = reinterpret_cast<float4 *>(a.cull), *bs = br + (alias ? off : a.nrl);
         int *cnt = reinterpret_cast<int *>(br + (size_t)tiles * nlegs);
         unsigned *list = reinterpret_cast<unsigned *>(cnt) + (size_t)tiles * a.nblk;
-        if (tz == 16) KCIG_TRY((launch_bounds_t<16, 8>(a, nlegs, br, tiles, st)));
-        else if (tx == 16) KCIG_TRY((launch_bounds_t<8, 16>(a, nlegs, br, tiles, st)));
-        else KCIG_TRY((launch_bounds_t<8, 8>(a, nlegs, br, tiles, st)));
-        const unsigned grid = (unsigned)(((long long)tiles * a.nblk + 7) / 8);
-        if (kb == 4) k_cull<4><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
-        else k_cull<2><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
-        KCIG_CUDA(cudaGetLastError());
-        a.cnt = cnt;
-        a.list = list;
-        a.parts = a.nsplit > a.nblk ? a.nsplit / a.nblk : 1;
+        if (a.lists) {
+            if (tz == 16) KCIG_TRY((launch_bounds_t<16, 8>(a, nlegs, br, tiles, st)));
+            else if (tx == 16) KCIG_TRY((launch_bounds_t<8, 16>(a, nlegs, br, tiles, st)));
+            else KCIG_TRY((launch_bounds_t<8, 8>(a, nlegs, br, tiles, st)));
+            const unsigned grid = (unsigned)(((long long)tiles * a.nblk + 7) / 8);
+            if (kb == 4) k_cull<4><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
+            else k_cull<2><<<grid, 256, 0, st>>>(a, bs, br, nlegs, tiles, list, cnt);
+            KCIG_CUDA(cudaGetLastError());
+            a.cnt = cnt;
+            a.list = list;
+        }
         int rc;
         const bool fits128 = (size_t)nb * 128 * 4 <= 200 * 1024;
         if (a.tile == 1 && fits128) rc = launch_sum_mode<16, 8, 4>(a, nb, st);
@@ -1665,7 +1741,7 @@ int launch_sum(const SumArgs &args, cudaStream_t st, int *launches, int *aux)
         else rc = launch_sum_mode<8, 8, KCIG_KB>(a, nb, st);
         if (rc) return rc;
         if (launches) (*launches)++;
-        if (aux) *aux += 2;
+        if (aux && a.lists) *aux += 2;
     }
     if (a0.nsplit > 1) {
         const size_t n = (size_t)a0.ng * a0.nz * a0.nx;
@@ -1841,7 +1917,7 @@ size_t spray_scratch_bytes(int nz, int nx, int nsb, int nrl)
 #define KCIG_SPLIT_WAVES 8
 #endif
 
-int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
+int sum_nsplit(int nz, int nx, int nsb, int nh, int ng, bool shared_r)
 {
     static int sms = 0;
     if (!sms) {
@@ -1852,6 +1928,19 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
     const long long tiles = (long long)((nz + 15) / 16) * ((nx + 7) / 8);
     const long long slots = (long long)sms * KCIG_SUM_MINB;  // resident CTAs of one wave
     const int blocks = shared_r ? (nsb + KCIG_KB - 1) / KCIG_KB : (nsb + KCIG_KB_UNSHARED - 1) / KCIG_KB_UNSHARED;
+    // Time of rows of CTAs, each `length` blocks long, in `waves` waves: a wave
+    // takes ~0.65 us a pair of a block (less where the bins' shared memory holds
+    // fewer CTAs), the rows' partial images 8 bytes a bin and point, their
+    // reduction 5 us.
+    const int kb = shared_r ? KCIG_KB : KCIG_KB_UNSHARED;
+    const int per_sm = std::max(1, std::min(KCIG_SUM_MINB, 232448 / (std::min(ng, kMaxBins) * 512 + 1024)));
+    const double held = (double)sms * per_sm;
+    const double block_us = (double)std::min(kb, nsb) * nh * 0.65 * std::max(0.5, (double)per_sm / KCIG_SUM_MINB);
+    auto time = [&](double waves, double length, int rows) {
+        return waves * length * block_us + (rows > 1 ? 5.0 + (double)rows * ng * nz * nx * 1.6e-6 : 0.0);
+    };
+    // blocks one a row may go on in parts of their walks, of four receivers or more
+    const int most = std::min(std::min(8, nh / 4), 64 / std::max(1, blocks));
     if (tiles >= (long long)KCIG_SPLIT_BELOW * slots) {
         // fill(n): the waves of n parts over whole waves
         auto fill = [&](int n) {
@@ -1870,33 +1959,44 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, bool shared_r)
         // v(z) 201 x 401 survey (663 tiles, 16 blocks): 16 parts of one block
         // each, 11 units, against 13 parts (the 8-wave aim) at 9 x 2 = 18 --
         // measured 4.80 -> 4.42 ms
-        // Blocks one a row may go on in parts of their receiver lists, of four
-        // receivers or more: a row then lasts 1 / parts of a block (41 x 81
-        // points, 2 blocks of 21 receivers: the stage 62 -> 36 us in five parts;
-        // 43 x 172 points, 9 blocks of 202: 0.74 -> 0.39 ms); from three waves
-        // on the set-up of more rows costs more than the last wave gains (the
-        // v(z) survey with parts: 2.64 -> 3.02 ms)
-        long long best = 1;
-        double cost = -1.0;
-        auto offer = [&](long long rows, double length) {
-            const double c = (double)((rows * tiles + slots - 1) / slots) * length;
-            if (cost < 0.0 || 20.0 * c < 19.0 * cost) {
+        long long best = 1, cost = -1;
+        for (long long n = 1; n <= std::min(blocks, 64); n++) {
+            const long long c = ((n * tiles + slots - 1) / slots) * ((blocks + n - 1) / n);
+            if (cost < 0 || 20 * c < 19 * cost) {
                 cost = c;
-                best = rows;
+                best = n;
             }
-        };
-        for (long long n = 1; n <= std::min(blocks, 64); n++) offer(n, (double)((blocks + n - 1) / n));
-        if (blocks * tiles < 3 * slots)
-            for (int p = 2; p <= std::min(8, nh / 4) && (long long)p * blocks <= 64; p++)
-                offer((long long)p * blocks, 1.0 / p);
+        }
+        // In parts where that lowers the time (41 x 81 points, 2 blocks of 21
+        // receivers, 61 bins: the stage 62 -> 36 us in five; 118 x 262 points, 4
+        // blocks of 223: 0.80 -> 0.39 ms); from three waves on the set-up of more
+        // rows costs more than the last wave gains (the v(z) survey in parts:
+        // 2.64 -> 3.02 ms)
+        if (blocks * tiles < 3 * slots) {
+            auto whole = [&](int rows, double length) { return time(ceil((double)rows * tiles / held), length, rows); };
+            double t = whole((int)best, (double)((blocks + best - 1) / best));
+            for (int p = 2; p <= most; p++)
+                if (whole(p * blocks, 1.0 / p) < 0.92 * t) {
+                    best = (long long)p * blocks;
+                    t = whole((int)best, 1.0 / p);
+                }
+        }
         return (int)best;
     }
     const long long want = (long long)KCIG_SPLIT_WAVES * slots;
     long long ns = (want + tiles - 1) / tiles;
-    if (ns >= 2LL * blocks && nh >= 8)  // too few blocks: their lists in parts
-        return blocks * (int)std::max<long long>(1, std::min<long long>(std::min(8, nh / 4), std::min<long long>(ns, 64) / blocks));
-    ns = std::min<long long>(ns, std::min(blocks, 64));
-    return (int)std::max<long long>(1, ns);
+    const int parts = (int)std::min<long long>(most, ns / std::max(1, blocks));
+    ns = std::max<long long>(1, std::min<long long>(ns, std::min(blocks, 64)));
+    if (ns < blocks) return (int)ns;
+    // too few blocks for that: their walks in parts, half a wave of idle CTAs at
+    // the end (45 shots of 167 receivers on 41 x 455 points: 2.8% faster in two
+    // parts; one shot of 16 on 301 x 801 points, 61 bins: 328 us a call, 490 in
+    // four)
+    int best = 1;
+    auto part = [&](int p) { return time((double)p * blocks * tiles / held + 0.5, 1.0 / p, p * blocks); };
+    for (int p = 2; p <= parts; p++)
+        if (part(p) < 0.98 * part(best)) best = p;
+    return best * blocks;
 }
 
 }  // namespace kcig

@@ -69,6 +69,10 @@ struct kcig_plan {
     NeedArgs need_args = {0, 0, 0, 0.0};  // of the legs computed next (nr = 0: all needed)
     const unsigned char *need = nullptr;  // the last legs' flags (null: all their fields exist)
     DevBuf d_cull;  // the summation's lists of pairs that may reach a tile
+    // the sample by which a sum's lists are judged (lists_begin): written to
+    // pinned memory (reach_take) by the device, and its arrival
+    int *h_reach = nullptr;
+    cudaEvent_t reach_ev = nullptr;
     DevBuf d_status;  // flag of the leg-field kernels' bounded waits (k_leg_tile)
     // tables left in host memory (KCIG_MEM_HOST_STREAM): the slices of each
     // leg batch are copied into d_stage
@@ -102,7 +106,9 @@ struct ShotBatch {
     int ns = 0, nhb = 0, nrl = 0;  // shots, padded receivers per shot, receiver legs
     size_t sleg0 = 0, rleg0 = 0;   // first source / receiver leg in `legs`
     size_t tr0 = 0, shot0 = 0;     // first padded trace, first shot
-    int unit_tw = 0;
+    int unit_tw = 0, unit_all = 0; // every trace weight is 1 or 0; every one is 1
+    double pairs = 0;              // traces that are no padding
+    int lists = 1;                 // the walk of its sum, as judged by the last run outside a capture
 };
 struct ShotsPrepared {
     std::vector<ShotBatch> batches;
@@ -454,6 +460,83 @@ int compute_fields(kcig_plan *P, int is_source, const std::vector<LegInterp> &le
     return KCIG_OK;
 }
 
+// Pinned memory for the plans' samples: a page of slots, allocated once and
+// kept (pinning memory takes milliseconds); a plan beyond them pins its own.
+constexpr int kReachSlots = 64;
+std::mutex g_reach_mu;
+int *g_reach = nullptr;
+unsigned long long g_reach_used = 0;  // one bit a slot
+
+int reach_take(int **slot)
+{
+    std::lock_guard<std::mutex> lock(g_reach_mu);
+    if (!g_reach)
+        KCIG_CUDA(cudaHostAlloc((void **)&g_reach, kReachSlots * kReachPairs * sizeof(int), cudaHostAllocPortable));
+    for (int i = 0; i < kReachSlots; i++)
+        if (!(g_reach_used >> i & 1ull)) {
+            g_reach_used |= 1ull << i;
+            *slot = g_reach + i * kReachPairs;
+            return KCIG_OK;
+        }
+    KCIG_CUDA(cudaHostAlloc((void **)slot, kReachPairs * sizeof(int), cudaHostAllocPortable));
+    return KCIG_OK;
+}
+
+void reach_give(int *slot)
+{
+    if (!slot) return;
+    std::lock_guard<std::mutex> lock(g_reach_mu);
+    const ptrdiff_t i = (slot - g_reach) / kReachPairs;
+    if (slot >= g_reach && i < kReachSlots) g_reach_used &= ~(1ull << i);
+    else cudaFreeHost(slot);
+}
+
+// Whether a batch's sum walks lists of the pairs that may reach a tile, or
+// every receiver.  The lists cost a pass over the legs' fields for their bounds
+// (a cost per leg), and walking one costs more a pair than counting receivers
+// up: they pay where more of the pairs than that miss the tiles, the part that
+// lists_cost returns.  How many do is sampled from the fields (64 pairs at 256
+// points); the sample is queued before the traces' prelude and read while that
+// runs.  Sums below kListsLeast pairs x points are not worth its ~9 us.
+// The parts were fitted to migrations of 201 x 401 .. 601 x 1601 points, 1 x 16
+// .. 64 x 201 traces, records of 0.8 to 12 s, walked either way (stack, 16 x 64
+// traces on 601 x 1601: 6.8 ms by lists and 5.9 by all where no pair misses,
+// 1.4 and 3.3 where nearly all do; angle gathers, 64 x 201 on 201 x 401: 6.8
+// and 6.6, 1.8 and 4.0).  With receivers of their own every pair has a leg.
+constexpr double kListsLeast = 24e6;
+double lists_cost(const SumArgs &a, double pairs, double legs)
+{
+    const double x = legs / pairs;
+    if (!a.shared_r) return 0.15 + 0.57 * x;
+    return a.mode < 2 ? 0.25 + 2.2 * x : a.mode == 2 ? 0.45 + x : 0.05 + 0.9 * x;
+}
+
+// *lists: 1 or 0 where that needs no sample, -1: sampled, lists_end tells
+int lists_begin(kcig_plan *P, const SumArgs &a, double pairs, double legs, cudaStream_t st, int *lists)
+{
+    *lists = 1;
+    if (sum_needs_lists(a)) return KCIG_OK;
+    *lists = 0;
+    if (pairs * a.nz * a.nx < kListsLeast || lists_cost(a, pairs, legs) >= 1.0) return KCIG_OK;
+    if (!P->h_reach) KCIG_TRY(reach_take(&P->h_reach));
+    if (!P->reach_ev) KCIG_CUDA(cudaEventCreateWithFlags(&P->reach_ev, cudaEventDisableTiming));
+    KCIG_TRY(launch_reach(a, P->h_reach, st));
+    P->all_launches++;
+    KCIG_CUDA(cudaEventRecord(P->reach_ev, st));
+    *lists = -1;
+    return KCIG_OK;
+}
+
+int lists_end(kcig_plan *P, const SumArgs &a, double pairs, double legs, int *lists)
+{
+    if (*lists >= 0) return KCIG_OK;
+    KCIG_CUDA(cudaEventSynchronize(P->reach_ev));
+    long long missed = 0;
+    for (int i = 0; i < kReachPairs; i++) missed += P->h_reach[i];
+    *lists = (double)missed > lists_cost(a, pairs, legs) * kReachPairs * kReachPoints;
+    return KCIG_OK;
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ C ABI --
@@ -504,6 +587,8 @@ extern "C" int kcig_plan_destroy(kcig_plan *P)
                       &P->d_part,   &P->d_stage, &P->d_cull, &P->d_need};
     for (DevBuf *b : bufs) b->release();
     release_shots(P);
+    reach_give(P->h_reach);
+    if (P->reach_ev) cudaEventDestroy(P->reach_ev);
     if (P->own_st) cudaStreamDestroy(P->own_st);
     if (P->copy_st) cudaStreamDestroy(P->copy_st);
     if (P->copy_ev) cudaEventDestroy(P->copy_ev);
@@ -962,18 +1047,6 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             pa.intercept = p.direct_mute_intercept;
             pa.taper = p.direct_mute_taper;
             pa.fold = fold;
-            if (data_pending) {  // the traces have landed before their first use
-                cudaError_t e = cudaStreamWaitEvent(st, P->copy_ev, 0);
-                if (e != cudaSuccess) {
-                    rc = cuda_error(e, "cudaStreamWaitEvent(traces)");
-                    break;
-                }
-                data_pending = false;
-            }
-            rc = launch_prelude(pa, st);
-            if (rc) break;
-            P->all_launches++;
-
             SumArgs sa;
             memset(&sa, 0, sizeof sa);
             sa.STP = sT;
@@ -1007,7 +1080,7 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.unit_tw = sa.unit_all ||
                          std::all_of(h_trw.begin(), h_trw.begin() + nb, [](float v) { return v == 1.0f || v == 0.0f; });
             sa.tile = P->tile;
-            sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, nhb, shared_r);
+            sa.nsplit = sum_nsplit(g.nz, g.nx, nsh, nhb, P->ng, shared_r);
             if (sa.nsplit > 1) {
                 rc = P->scratch(P->d_part, (size_t)sa.nsplit * P->ng * nzx * sizeof(float));
                 if (rc) break;
@@ -1031,6 +1104,22 @@ extern "C" int kcig_migrate(kcig_plan *P, const float *data, float *image, int m
             sa.oaztaper = p.oaztaper;
             sa.ats = p.angle_taper_start;
             sa.ate = p.angle_taper_end;
+            const double nlegs = sa.nrl + (alias_src ? 0 : nsh);
+            rc = lists_begin(P, sa, (double)nb, nlegs, st, &sa.lists);
+            if (rc) break;
+            if (data_pending) {  // the traces have landed before their first use
+                cudaError_t e = cudaStreamWaitEvent(st, P->copy_ev, 0);
+                if (e != cudaSuccess) {
+                    rc = cuda_error(e, "cudaStreamWaitEvent(traces)");
+                    break;
+                }
+                data_pending = false;
+            }
+            rc = launch_prelude(pa, st);
+            if (rc) break;
+            P->all_launches++;
+            rc = lists_end(P, sa, (double)nb, nlegs, &sa.lists);
+            if (rc) break;
             cudaEvent_t e0, e1;
             cudaEventCreate(&e0);
             cudaEventCreate(&e1);
@@ -1423,7 +1512,7 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.stop = S->stop.as<float>() + B.shot0;
     sa.snh = S->snh.as<int>() + B.shot0;
     sa.tile = P->tile;
-    sa.nsplit = sum_nsplit(g.nz, g.nx, B.ns, B.nhb, false);
+    sa.nsplit = sum_nsplit(g.nz, g.nx, B.ns, B.nhb, P->ng, false);
     if (sa.nsplit > 1) sa.partial = P->d_part.as<float>();  // sized by kcig_shots_prepare
     sa.image = d_img;
     sa.zero_init = b == 0 ? 1 : 0;
@@ -1437,6 +1526,8 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     sa.ng = P->ng;
     sa.mode = angle ? (p.angle_interp ? 0 : 1) : 2;
     sa.unit_tw = B.unit_tw;
+    sa.unit_all = B.unit_all;
+    sa.lists = B.lists;
     sa.shared_r = 0;
     sa.half = p.half_angle;
     sa.t0 = g.t0;
@@ -1458,23 +1549,30 @@ SumArgs batch_sum_args(const kcig_plan *P, size_t b, float *d_img)
     return sa;
 }
 
-int batch_inputs(kcig_plan *P, size_t b, cudaStream_t st)
+// leg fields and integrated traces of batch b, and the walk of its sum (judged
+// from the fields; a capture keeps what the run before it found)
+int batch_inputs(kcig_plan *P, size_t b, cudaStream_t st, bool capturing, cudaEvent_t *ev = nullptr)
 {
+    if (ev) cudaEventRecord(ev[0], st);
     KCIG_TRY(batch_fields(P, b, st));
-    return batch_prelude(P, b, st);
+    if (ev) cudaEventRecord(ev[1], st);
+    if (capturing) return batch_prelude(P, b, st);
+    ShotBatch &B = P->shots->batches[b];
+    const SumArgs sa = batch_sum_args(P, b, nullptr);
+    const double legs = B.nrl + B.ns;
+    KCIG_TRY(lists_begin(P, sa, B.pairs, legs, st, &B.lists));
+    KCIG_TRY(batch_prelude(P, b, st));
+    return lists_end(P, sa, B.pairs, legs, &B.lists);
 }
 
 // `ev` (4 events per batch, or null): before the fields, after the fields,
 // after the prelude, after the summation -- for the stage times of a direct
 // (uncaptured) run
-int run_prepared(kcig_plan *P, float *d_img, cudaStream_t st, cudaEvent_t *ev = nullptr)
+int run_prepared(kcig_plan *P, float *d_img, cudaStream_t st, bool capturing, cudaEvent_t *ev = nullptr)
 {
     ShotsPrepared *S = P->shots;
     for (size_t b = 0; b < S->batches.size(); b++) {
-        if (ev) cudaEventRecord(ev[4 * b], st);
-        KCIG_TRY(batch_fields(P, b, st));
-        if (ev) cudaEventRecord(ev[4 * b + 1], st);
-        KCIG_TRY(batch_prelude(P, b, st));
+        KCIG_TRY(batch_inputs(P, b, st, capturing, ev ? ev + 4 * b : nullptr));
         if (ev) cudaEventRecord(ev[4 * b + 2], st);
         const SumArgs sa = batch_sum_args(P, b, d_img);
         int nl = 0;
@@ -1588,7 +1686,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
         }
         B.rleg0 = hlegs.size();
         std::map<std::tuple<double, float, float>, int> index;
-        bool unit = true;
+        bool unit = true, all = true;
         for (int k = 0; k < B.ns; k++) {
             const kcig_shot &sh = shots[i0 + k];
             const float dhf = sh.nh == 1 ? 0.0f : sh.dh;
@@ -1643,6 +1741,8 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
                     ig = b < 0 ? 0 : b;
                 }
                 if (w != 1.0 && w != 0.0) unit = false;
+                if (w != 1.0) all = false;
+                B.pairs += 1.0;
                 h_msx.push_back((double)sh.sx);
                 h_mrx.push_back(rpos);
                 h_toff.push_back((long long)(base[i0 + k] + (size_t)r * sh.nt));
@@ -1655,6 +1755,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
         }
         B.nrl = (int)index.size();
         B.unit_tw = unit ? 1 : 0;
+        B.unit_all = all ? 1 : 0;
         max_s = std::max<size_t>(max_s, B.ns);
         max_r = std::max<size_t>(max_r, B.nrl);
         max_d = std::max<size_t>(max_d, (size_t)B.ns * B.nhb);
@@ -1675,7 +1776,7 @@ extern "C" int kcig_shots_prepare(kcig_plan *P, int nshots, const kcig_shot *sho
     if (!rc && angle && !(P->sg_src && P->sg_rcv))
         rc = P->scratch(P->d_work, (size_t)field_batch(P, std::max(max_s, max_r)) * 4 * nzx * sizeof(double));
     int max_split = 1;
-    for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, B.nhb, false));
+    for (const ShotBatch &B : S->batches) max_split = std::max(max_split, sum_nsplit(g.nz, g.nx, B.ns, B.nhb, P->ng, false));
     if (!rc && max_split > 1) rc = P->scratch(P->d_part, (size_t)max_split * P->ng * nzx * sizeof(float));
     size_t cull = 0;
     for (const ShotBatch &B : S->batches) cull = std::max(cull, batch_cull_bytes(P, B.ns, B.nhb, B.nrl));
@@ -1749,7 +1850,7 @@ extern "C" int kcig_migrate_prepared(kcig_plan *P, float *image, int memory)
         } else {
             // one direct run (it also raises every kernel's shared-memory
             // limit), then capture the same sequence for the next calls
-            rc = run_prepared(P, d_img, st);
+            rc = run_prepared(P, d_img, st, false);
             if (!rc) {
                 if (S->exec) {
                     cudaGraphExecDestroy(S->exec);
@@ -1762,7 +1863,7 @@ extern "C" int kcig_migrate_prepared(kcig_plan *P, float *image, int memory)
                 if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamBeginCapture");
                 if (!rc) {
                     S->captured = true;
-                    const int rc2 = run_prepared(P, d_img, st);
+                    const int rc2 = run_prepared(P, d_img, st, true);
                     cudaGraph_t gr = nullptr;
                     e = cudaStreamEndCapture(st, &gr);
                     if (rc2) rc = rc2;
@@ -1787,7 +1888,7 @@ extern "C" int kcig_migrate_prepared(kcig_plan *P, float *image, int memory)
     } else {
         std::vector<cudaEvent_t> ev(4 * S->batches.size());
         for (auto &x : ev) cudaEventCreate(&x);
-        rc = run_prepared(P, d_img, st, ev.data());
+        rc = run_prepared(P, d_img, st, false, ev.data());
         if (!rc) {
             cudaError_t e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamSynchronize(prepared)");
@@ -1823,7 +1924,7 @@ extern "C" int kcig_plan_autotune(kcig_plan *P, int *choice, float *ms)
     const size_t nzx = (size_t)P->g.nz * P->g.nx;
     KCIG_TRY(P->d_image.ensure((size_t)P->ng * nzx * sizeof(float)));
     cudaStream_t st = P->st;
-    KCIG_TRY(batch_inputs(P, 0, st));
+    KCIG_TRY(batch_inputs(P, 0, st, false));
     SumArgs sa = batch_sum_args(P, 0, P->d_image.as<float>());
     cudaEvent_t e0, e1;
     KCIG_CUDA(cudaEventCreate(&e0));
@@ -1878,7 +1979,7 @@ extern "C" int kcig_graph_create(int n, kcig_plan *const *plans, float *const *i
     KCIG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     int rc = KCIG_OK;
     // one direct pass first: kernels' shared-memory limits are raised outside the capture
-    for (int i = 0; i < n && rc == KCIG_OK; i++) rc = run_prepared(plans[i], images[i], st);
+    for (int i = 0; i < n && rc == KCIG_OK; i++) rc = run_prepared(plans[i], images[i], st, false);
     cudaError_t e = cudaStreamSynchronize(st);
     if (!rc && e != cudaSuccess) rc = cuda_error(e, "cudaStreamSynchronize(graph warm-up)");
     kcig_graph *G = new kcig_graph();
@@ -1889,7 +1990,7 @@ extern "C" int kcig_graph_create(int n, kcig_plan *const *plans, float *const *i
             int rc2 = KCIG_OK;
             for (int i = 0; i < n && rc2 == KCIG_OK; i++) {
                 plans[i]->shots->captured = true;
-                rc2 = run_prepared(plans[i], images[i], st);
+                rc2 = run_prepared(plans[i], images[i], st, true);
             }
             e = cudaStreamEndCapture(st, &G->graph);
             if (rc2) rc = rc2;
