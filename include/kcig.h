@@ -229,7 +229,9 @@ typedef struct kcig_eikods_opts {
  * took.  nz in 3..1400, nx >= 3.  Scratch comes from a memory pool
  * of the library: the working values of the sources in flight (32 MB each on
  * 601 x 1601; fewer at a time where memory is short), of which the pool keeps
- * up to a sixteenth of the device until kcig_datum_release.  The same local problem as the marching code, solved by
+ * up to a sixteenth of the device until kcig_datum_release (256 MB at most
+ * after a call on a device with less than a 32nd free; the library's other
+ * calls take it back before they fail).  The same local problem as the marching code, solved by
  * sweeps to the fixed point: identical results for order 1, within ~2.5e-4 s
  * for order 2 (whose marching result depends on the heap's acceptance
  * order).  KCIG_ERR_DEVICE if a source has no fixed point within max_iter. */
@@ -310,7 +312,10 @@ int kcig_plan_autotune(kcig_plan *plan, int *choice, float *ms);
  * the recursive workflow, each with its own tables, mute and image): create
  * runs every plan once directly, then captures the same sequence; launch
  * replays it asynchronously on `stream` (the caller synchronises).  The
- * plans, their prepared shots and the images must outlive the graph. */
+ * plans, their prepared shots and the images must outlive the graph.  Other
+ * calls on the plans between replays (kcig_plan_autotune, kcig_migrate,
+ * kcig_model) leave the graph valid: scratch that it holds is kept until the
+ * shots are prepared anew, also where such a call needs more. */
 typedef struct kcig_graph kcig_graph;
 int kcig_graph_create(int nplans, kcig_plan *const *plans, float *const *images, kcig_graph **out);
 int kcig_graph_launch(kcig_graph *graph, void *stream);

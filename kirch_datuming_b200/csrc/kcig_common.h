@@ -131,7 +131,8 @@ int sg_check_status(kcig_surrogate *s, cudaStream_t st);
 // their shots on receivers.  Of two traces whose shots' groups differ the one
 // of the smaller group is kept; traces inside a group stay apart.  Half the
 // pairs and half the leg fields of such a survey are left (601 x 1601, 400
-// shots on 400 receivers: summation 385 -> 190 ms, leg fields 32 -> 16 ms).
+// shots on 400 receivers, before pairs were listed and blocks of fields left
+// out: summation 385 -> 190 ms, leg fields 32 -> 16 ms).
 constexpr int kFoldGroup = 4;
 struct Fold {
     int on, off, ga, gb;

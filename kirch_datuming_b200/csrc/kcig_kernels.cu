@@ -1134,11 +1134,10 @@ __device__ __forceinline__ double floor_shift(double x) { return __dadd_rd(x, kF
 // Resident CTAs of 128 threads per SM the register allocation must allow
 // (scaled for other tile sizes, so every tile gets 28 warps and at most 72
 // registers): 7 CTAs of 128 threads is the most the 61-bin accumulators'
-// shared memory admits (7 x 31 KB); occupancy is what this latency- and
-// issue-bound loop needs (measured on the benchmark: 6 CTAs/SM at 80
-// registers 500 ms per launch, 7 CTAs/SM 482 ms; earlier 16x16 tiles at 2
-// CTAs/SM were slower still; 8x8 tiles of ragged shots at 82 registers held
-// 10 CTAs, 20 warps, and waited on their gathers).
+// shared memory admits (7 x 31 KB).  The production survey's listed pairs take
+// 21.2 ms with 7 CTAs and 21.4 with 6 at 80 registers; walking every receiver
+// (issue-bound) 482 and 500, and 8x8 tiles of ragged shots at 82 registers
+// held 10 CTAs, 20 warps, and waited on their gathers.
 #ifndef KCIG_SUM_MINB
 #define KCIG_SUM_MINB 7
 #endif
@@ -1866,6 +1865,7 @@ int launch_spray(const SprayArgs &a0, cudaStream_t st)
     if (a0.nsb <= 0 || a0.nh <= 0) return KCIG_OK;
     SprayArgs a = a0;
     const size_t sm = a.nt * sizeof(double);
+    // (the longest record accepted; a CTA's one trace then takes 50 KB)
     if (4 * sm > 200 * 1024) return set_error(KCIG_ERR_UNSUPPORTED, "nt=%d too long for forward modelling", a.nt);
     // what the pair bounds read, and the legs' ranges over the tiles
     memset(&a.cull, 0, sizeof a.cull);
@@ -1909,7 +1909,9 @@ size_t spray_scratch_bytes(int nz, int nx, int nsb, int nrl)
 // waves there are; each split adds a partial image).  A grid of more waves is split into
 // up to 4 parts only when that fills its last wave clearly better: the
 // 601 x 1601 grid's 7638 tiles are 7.37 waves of 1036 slots (the last one 37%
-// full), as two parts 14.75 waves (75% full), measured 1.7% faster.
+// full), as two parts 14.75 waves (75% full): the production survey's
+// summation 29.2 -> 27.7 ms, partial images and their reduction included
+// (tiles' lists differ in length, which more and shorter rows even out too).
 #ifndef KCIG_SPLIT_BELOW
 #define KCIG_SPLIT_BELOW 2
 #endif
@@ -1953,12 +1955,12 @@ int sum_nsplit(int nz, int nx, int nsb, int nh, int ng, bool shared_r)
         return best;
     }
     if (shared_r) {
-        // shots shared by every tile: a CTA row's duration is its number of
-        // shot blocks, so take the split with the fewest waves x blocks per
-        // row (whole waves, the longest row); more parts only for 5% less.  The
-        // v(z) 201 x 401 survey (663 tiles, 16 blocks): 16 parts of one block
-        // each, 11 units, against 13 parts (the 8-wave aim) at 9 x 2 = 18 --
-        // measured 4.80 -> 4.42 ms
+        // shots shared by every tile: a CTA row's duration is about its number
+        // of shot blocks (lists shorten all of them), so take the split with the
+        // fewest waves x blocks per row (whole waves, the longest row); more
+        // parts only for 5% less.  The v(z) 201 x 401 survey (663 tiles, 16
+        // blocks): 16 parts of one block each, 11 units, against 13 parts (the
+        // 8-wave aim) at 9 x 2 = 18 -- walking every receiver 4.80 -> 4.42 ms
         long long best = 1, cost = -1;
         for (long long n = 1; n <= std::min(blocks, 64); n++) {
             const long long c = ((n * tiles + slots - 1) / slots) * ((blocks + n - 1) / n);
